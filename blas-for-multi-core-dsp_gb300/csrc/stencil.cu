@@ -4,13 +4,16 @@
 // (stencil_2d_V1.2/device_code/kernel_stencil.c:1042, :14): one sweep
 // B = 0.2 * (N + S + E + W + C) over an (M+2) x (N+2) padded grid with a
 // fixed halo.  The reference streams 128x128 (+1 halo) tiles through AM;
-// here a CTA loads an output tile plus a halo of `t` cells into shared
-// memory, runs `t` sweeps there (each sweep's valid region shrinks by one
-// cell), and writes the final tile: HBM traffic per sweep drops to about
-// (1 + halo overhead) / t of a read plus a write.  Every interior point is
-// computed from the same neighbours in the same add order as the
-// unblocked recurrence, so results are bit-identical for any t.
+// here FP32 grids are streamed through registers several sweeps a pass
+// (temporal blocking: HBM traffic per sweep drops to about (1 + halo
+// overhead) / t of a read plus a write), FP64 grids one sweep a pass through
+// shared-memory tiles.  Every interior point is computed from the same
+// neighbours in the same add order as the unblocked recurrence, so results
+// are bit-identical for any number of sweeps a pass.
+#include <math.h>
+
 #include "gb_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace gb {
 namespace {
@@ -23,13 +26,6 @@ struct SOps<double> {
     __device__ static double mul(double a, double b) { return __dmul_rn(a, b); }
     __device__ static double fifth() { return 0.2; }
 };
-template <>
-struct SOps<float> {
-    __device__ static float add(float a, float b) { return __fadd_rn(a, b); }
-    __device__ static float mul(float a, float b) { return __fmul_rn(a, b); }
-    __device__ static float fifth() { return 0.2f; }
-};
-
 // The three reference add orders (see gbblas.h, gb_stencil_order).
 template <typename T, int ORDER>
 __device__ __forceinline__ T update(T top, T left, T right, T down, T mid, int64_t row) {
@@ -113,95 +109,183 @@ __global__ void __launch_bounds__(NT) stencil_tb_kernel(const T *__restrict__ sr
 }
 
 // FP32 form, no shared memory: register-streamed temporal blocking.  A warp
-// owns a strip of 128 columns (lane l: columns 4l .. 4l+3) and walks a
-// segment of rows top to bottom, one input row per step.  Sweep level
-// l = 1..T keeps the last two rows of level l-1 in registers; when level l-1
-// produces row rho+1, level l computes row rho from (rho-1, rho, rho+1)
-// with the left / right neighbours of the middle row from the adjacent
-// lanes (two shuffles per four points).  The level-T rows are written out.
-// Each level loses one column at each strip edge and one row at each
-// segment end, so a strip writes 128 - 2T columns and a segment reads T
-// rows of halo above and below.  Every point gets the same neighbours in the
-// same add order as one sweep at a time, so results are bit-identical.
-constexpr int RS_W = 128, RS_SEG = 256, RS_NT = 256;
+// owns a strip of 128 columns and walks a segment of rows top to bottom, one
+// input row per step.  Sweep level l = 1..T keeps the last two rows of level
+// l-1 in registers; when level l-1 produces row rho+1, level l computes row
+// rho from (rho-1, rho, rho+1).  The level-T rows are written out.  Each
+// level loses one column at each strip edge and one row at each segment end,
+// so a strip writes 128 - 2T columns and a segment of `seg` rows reads T rows
+// of halo above and below.  Every point gets the same neighbours in the same
+// add order as one sweep at a time, so results are bit-identical.
+//
+// Bound by FP32 issue.  Lane l holds columns 2l, 2l+1 and 64+2l, 65+2l as the
+// two packed FP32x2 values (2l, 64+2l) and (2l+1, 65+2l): every add and multiply serves two
+// points, the neighbours of a pair are again pairs (the other pair of the
+// lane, or the adjacent lane's, rotated once around the strip), and the ring
+// of two rows per level is indexed by the unrolled row, so no value is moved
+// from register to register.  Rows are loaded four steps before they are used
+// (a warp alone on a scheduler would otherwise wait for L2 at every row).
+// Only warps whose window touches the grid's boundary (EDGE) test for fixed
+// cells.
+constexpr int RS_W = 128, RS_T = 6, RS_U = 4, RS_WARPS = 16;   // strip, most sweeps a pass, rows unrolled, warps an SM holds
 
-template <typename E, int T, int ORDER>
-__global__ void __launch_bounds__(RS_NT) stencil_rs_kernel(const E *__restrict__ src, E *__restrict__ dst,
-                                                           int64_t M, int64_t N, int strips, int segs) {
+template <int ORDER, int PAR>
+__device__ __forceinline__ uint64_t update2(uint64_t top, uint64_t left, uint64_t right, uint64_t down, uint64_t mid,
+                                            uint64_t fifth) {
+    using ptx::f2_add;
+    if (ORDER == GB_STENCIL_HOST)
+        return ptx::f2_mul(f2_add(f2_add(f2_add(f2_add(top, left), right), down), mid), fifth);
+    if (ORDER == GB_STENCIL_SCALAR)
+        return ptx::f2_mul(fifth, f2_add(f2_add(f2_add(f2_add(top, mid), down), left), right));
+    if (PAR == 0) return ptx::f2_mul(f2_add(right, f2_add(f2_add(left, top), f2_add(mid, down))), fifth);
+    return ptx::f2_mul(f2_add(right, f2_add(f2_add(left, down), f2_add(top, mid))), fifth);
+}
+
+template <int T, int ORDER, bool EDGE>
+__device__ __forceinline__ void rs_walk(const float *__restrict__ src, float *__restrict__ dst, int64_t M, int64_t N,
+                                        int64_t c0, int64_t out_r0, int64_t out_r1) {
     const int lane = threadIdx.x % 32;
-    const int64_t wid = (int64_t)blockIdx.x * (RS_NT / 32) + threadIdx.x / 32;
-    if (wid >= (int64_t)strips * segs) return;   // whole warp
-    const int sx = (int)(wid % strips), sy = (int)(wid / strips);
     const int64_t ld = N + 2;
-    const int64_t c0 = 1 + (int64_t)sx * (RS_W - 2 * T) - T;   // padded column of lane 0, q = 0
-    const int64_t out_r0 = 1 + (int64_t)sy * RS_SEG;            // padded rows written: [out_r0, out_r1)
-    const int64_t out_r1 = out_r0 + RS_SEG < M + 1 ? out_r0 + RS_SEG : M + 1;
-    const int64_t cl = c0 + 4 * lane;                            // this lane's first column
-
-    bool cfix[4], cload[4], cstore[4];
+    const int64_t cl = c0 + 2 * lane;   // this lane's columns: cl, cl + 1, cl + 64, cl + 65
+    const int lprev = (lane + 31) & 31, lnext = (lane + 1) & 31;
+    // bit q + 2h: column cl + q + 64h is inside the padded grid / fixed / written
+    unsigned cload = 0, cfix = 0, cstore = 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int64_t gc = cl + q;
-        const int lc = 4 * lane + q;
-        cfix[q] = gc <= 0 || gc >= N + 1;
-        cload[q] = gc >= 0 && gc <= N + 1;
-        cstore[q] = lc >= T && lc < RS_W - T && gc >= 1 && gc <= N;
+    for (int b = 0; b < 4; b++) {
+        const int d = (b & 1) + 64 * (b >> 1);
+        const int64_t gc = cl + d;
+        if (gc >= 0 && gc <= N + 1) cload |= 1u << b;
+        if (gc <= 0 || gc >= N + 1) cfix |= 1u << b;
+        if (2 * lane + d >= T && 2 * lane + d < RS_W - T && gc >= 1 && gc <= N) cstore |= 1u << b;
     }
+    const uint64_t fifth = ptx::f2_pack(0.2f, 0.2f);
 
-    E p2[T][4], p1[T][4];   // level l-1 rows rho-1 and rho of level l's window
+    uint64_t R[2][T][2];   // [ring slot][level][pair]
 #pragma unroll
     for (int l = 0; l < T; l++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) p2[l][q] = p1[l][q] = E(0);
+        for (int q = 0; q < 2; q++) R[0][l][q] = R[1][l][q] = 0ull;
 
-    for (int64_t i = out_r0 - T - 1; i < out_r1 + T; i++) {   // input row i (level 0)
-        E x[4] = {E(0), E(0), E(0), E(0)};
-        if (i >= 0 && i <= M + 1) {
-            const E *row = src + i * ld + cl;
+    // input rows i0 + k, k = 0 .. kn - 1, up to row out_r1 + T - 1; i0 even so that a row's parity is
+    // known when unrolled
+    const int64_t i0 = (out_r0 - T) & ~(int64_t)1;
+    const int kn = (int)(out_r1 + T - i0), ks = (int)(out_r0 + T - i0);   // row k - T is written from k = ks
+    const int klo = (int)(-i0 > -(1 << 30) ? -i0 : -(1 << 30));                                           // rows k < klo lie above the grid
+    const int khi = (int)(M + 2 - i0 < kn ? M + 2 - i0 : kn);              // rows k >= khi below it, or unused
+    const int kend = (int)(M + 1 - i0 < (1 << 30) ? M + 1 - i0 : 1 << 30); // row M + 1, fixed like row 0
+    const float *pin = src + i0 * ld + cl;
+    float *pout = dst + (i0 - T) * ld + cl;
+    float f[RS_U][4];
+    auto load = [&](float (&x)[4], int k) {   // row k, at pin
+        if (EDGE) {
+            const unsigned m = k >= klo && k < khi ? cload : 0u;
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (cload[q]) x[q] = __ldg(row + q);
+            for (int b = 0; b < 4; b++) x[b] = (m >> b) & 1u ? __ldg(pin + (b & 1) + 64 * (b >> 1)) : 0.f;
+        } else if (k < kn) {
+#pragma unroll
+            for (int b = 0; b < 4; b++) x[b] = __ldg(pin + (b & 1) + 64 * (b >> 1));
         }
+        pin += ld;
+    };
 #pragma unroll
-        for (int l = 0; l < T; l++) {
-            // level l+1, row rho = i - l - 1: top p2[l], middle p1[l], down x
-            const int64_t gr = i - l - 1;
-            const E left0 = __shfl_up_sync(0xffffffffu, p1[l][3], 1);
-            const E right3 = __shfl_down_sync(0xffffffffu, p1[l][0], 1);
-            const bool rfix = gr <= 0 || gr >= M + 1;
-            E v[4];
+    for (int u = 0; u < RS_U; u++) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const E lft = q == 0 ? left0 : p1[l][q - 1];
-                const E rgt = q == 3 ? right3 : p1[l][q + 1];
-                v[q] = (rfix || cfix[q]) ? p1[l][q] : update<E, ORDER>(p2[l][q], lft, rgt, x[q], p1[l][q], gr - 1);
+        for (int b = 0; b < 4; b++) f[u][b] = 0.f;
+        load(f[u], u);
+    }
+
+    for (int kb = 0; kb < kn; kb += RS_U) {
+#pragma unroll
+        for (int u = 0; u < RS_U; u++) {
+            const int k = kb + u;
+            uint64_t x[2] = {ptx::f2_pack(f[u][0], f[u][2]), ptx::f2_pack(f[u][1], f[u][3])};
+            load(f[u], k + RS_U);
+#pragma unroll
+            for (int l = 0; l < T; l++) {
+                // level l+1, row k - l - 1: top R[slot], middle R[slot ^ 1], down x
+                uint64_t(&top)[2] = R[u & 1][l];
+                const uint64_t(&mid)[2] = R[(u & 1) ^ 1][l];
+                float m0l, m0h, m1l, m1h;
+                ptx::f2_unpack(mid[0], m0l, m0h);
+                ptx::f2_unpack(mid[1], m1l, m1h);
+                // column 2l - 1 from the previous lane's second pair; the high half of lane 0 follows
+                // the low half of lane 31
+                const float al = __shfl_sync(0xffffffffu, m1l, lprev), ah = __shfl_sync(0xffffffffu, m1h, lprev);
+                const uint64_t left0 = ptx::f2_pack(al, lane == 0 ? al : ah);
+                const float bl = __shfl_sync(0xffffffffu, m0l, lnext), bh = __shfl_sync(0xffffffffu, m0h, lnext);
+                const uint64_t right1 = ptx::f2_pack(lane == 31 ? bh : bl, bh);
+                uint64_t v[2];
+                if ((u + l) & 1) {   // (row - 1) is odd
+                    v[0] = update2<ORDER, 1>(top[0], left0, mid[1], x[0], mid[0], fifth);
+                    v[1] = update2<ORDER, 1>(top[1], mid[0], right1, x[1], mid[1], fifth);
+                } else {
+                    v[0] = update2<ORDER, 0>(top[0], left0, mid[1], x[0], mid[0], fifth);
+                    v[1] = update2<ORDER, 0>(top[1], mid[0], right1, x[1], mid[1], fifth);
+                }
+                if (EDGE) {
+                    const int kr = k - l - 1;
+                    const unsigned m = kr <= klo || kr >= kend ? 15u : cfix;
+                    float w0l, w0h, w1l, w1h;
+                    ptx::f2_unpack(v[0], w0l, w0h);
+                    ptx::f2_unpack(v[1], w1l, w1h);
+                    v[0] = ptx::f2_pack(m & 1u ? m0l : w0l, m & 4u ? m0h : w0h);
+                    v[1] = ptx::f2_pack(m & 2u ? m1l : w1l, m & 8u ? m1h : w1h);
+                }
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    top[q] = x[q];
+                    x[q] = v[q];
+                }
             }
+            if (k >= ks && k < kn) {   // x: level T, row k - T
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                p2[l][q] = p1[l][q];
-                p1[l][q] = x[q];
-                x[q] = v[q];
+                for (int q = 0; q < 2; q++) {
+                    float lo, hi;
+                    ptx::f2_unpack(x[q], lo, hi);
+                    if ((cstore >> q) & 1u) pout[q] = lo;
+                    if ((cstore >> (q + 2)) & 1u) pout[q + 64] = hi;
+                }
             }
-        }
-        // x: level T, row i - T
-        const int64_t ro = i - T;
-        if (ro >= out_r0 && ro < out_r1) {
-            E *row = dst + ro * ld + cl;
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (cstore[q]) row[q] = x[q];
+            pout += ld;
         }
     }
 }
 
-template <typename E, int T>
-void launch_rs(const E *src, E *dst, int64_t M, int64_t N, int order, cudaStream_t st) {
-    const int strips = (int)ceil_div(N, RS_W - 2 * T);
-    const int segs = (int)ceil_div(M, RS_SEG);
-    const unsigned blocks = (unsigned)ceil_div((int64_t)strips * segs, RS_NT / 32);
-    if (order == 0) stencil_rs_kernel<E, T, 0><<<blocks, RS_NT, 0, st>>>(src, dst, M, N, strips, segs);
-    else if (order == 1) stencil_rs_kernel<E, T, 1><<<blocks, RS_NT, 0, st>>>(src, dst, M, N, strips, segs);
-    else stencil_rs_kernel<E, T, 2><<<blocks, RS_NT, 0, st>>>(src, dst, M, N, strips, segs);
+// One warp per CTA, 16 of them resident per SM (128 registers), so that a
+// grid that does not fill the GPU spreads evenly.  A pass after the first is
+// launched as a programmatic dependent: its launch overlaps the pass before,
+// whose rows it waits for here.
+template <int T, int ORDER>
+__global__ void __launch_bounds__(32, RS_WARPS) stencil_rs_kernel(const float *__restrict__ src,
+                                                                  float *__restrict__ dst, int64_t M, int64_t N,
+                                                                  int strips, int seg) {
+    ptx::pdl_wait();   // returns at once when not launched as a dependent
+    const int64_t sx = blockIdx.x % (unsigned)strips, sy = blockIdx.x / (unsigned)strips;
+    const int64_t c0 = 1 + sx * (RS_W - 2 * T) - T;   // padded column of the strip's first
+    const int64_t r0 = 1 + sy * seg;                   // padded rows written: [r0, r1)
+    const int64_t r1 = r0 + seg < M + 1 ? r0 + seg : M + 1;
+    // no fixed cell in the window and every load inside the grid
+    const bool inside = c0 >= 0 && c0 + RS_W <= N + 2 && r0 - T - 1 >= 0 && r1 + T <= M + 2;
+    if (inside) rs_walk<T, ORDER, false>(src, dst, M, N, c0, r0, r1);
+    else rs_walk<T, ORDER, true>(src, dst, M, N, c0, r0, r1);
+}
+
+template <int T>
+cudaError_t launch_rs(const float *src, float *dst, int64_t M, int64_t N, int seg, int order, bool dependent,
+                      cudaStream_t st) {
+    const int64_t strips = ceil_div(N, RS_W - 2 * T);
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(strips * ceil_div(M, seg)));
+    cfg.blockDim = dim3(32);
+    cfg.stream = st;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = dependent ? 1 : 0;
+    auto kernel = order == GB_STENCIL_HOST ? stencil_rs_kernel<T, 0>
+                  : order == GB_STENCIL_SCALAR ? stencil_rs_kernel<T, 1> : stencil_rs_kernel<T, 2>;
+    return cudaLaunchKernelEx(&cfg, kernel, src, dst, M, N, (int)strips, seg);
 }
 
 // 9-point stencil with a 3x3 weight window (w[0..2] the row above, w[3..5]
@@ -234,17 +318,19 @@ __device__ __forceinline__ float mul_rn<float>(float a, float b) { return __fmul
 template <>
 __device__ __forceinline__ double mul_rn<double>(double a, double b) { return __dmul_rn(a, b); }
 
+constexpr int R9_SEG = 256, R9_NT = 256;
+
 template <typename E, int T>
-__global__ void __launch_bounds__(RS_NT) stencil9_rs_kernel(const E *__restrict__ src, E *__restrict__ dst,
+__global__ void __launch_bounds__(R9_NT) stencil9_rs_kernel(const E *__restrict__ src, E *__restrict__ dst,
                                                             int64_t M, int64_t N, int strips, int segs, W9<E> w) {
     const int lane = threadIdx.x % 32;
-    const int64_t wid = (int64_t)blockIdx.x * (RS_NT / 32) + threadIdx.x / 32;
+    const int64_t wid = (int64_t)blockIdx.x * (R9_NT / 32) + threadIdx.x / 32;
     if (wid >= (int64_t)strips * segs) return;   // whole warp
     const int sx = (int)(wid % strips), sy = (int)(wid / strips);
     const int64_t ld = N + 2;
     const int64_t c0 = 1 + (int64_t)sx * (RS_W - 2 * T) - T;
-    const int64_t out_r0 = 1 + (int64_t)sy * RS_SEG;
-    const int64_t out_r1 = out_r0 + RS_SEG < M + 1 ? out_r0 + RS_SEG : M + 1;
+    const int64_t out_r0 = 1 + (int64_t)sy * R9_SEG;
+    const int64_t out_r1 = out_r0 + R9_SEG < M + 1 ? out_r0 + R9_SEG : M + 1;
     const int64_t cl = c0 + 4 * lane;
 
     bool cfix[4], cload[4], cstore[4];
@@ -316,9 +402,9 @@ __global__ void __launch_bounds__(RS_NT) stencil9_rs_kernel(const E *__restrict_
 template <typename E, int T>
 void launch_rs9(const E *src, E *dst, int64_t M, int64_t N, const W9<E> &w, cudaStream_t st) {
     const int strips = (int)ceil_div(N, RS_W - 2 * T);
-    const int segs = (int)ceil_div(M, RS_SEG);
-    const unsigned blocks = (unsigned)ceil_div((int64_t)strips * segs, RS_NT / 32);
-    stencil9_rs_kernel<E, T><<<blocks, RS_NT, 0, st>>>(src, dst, M, N, strips, segs, w);
+    const int segs = (int)ceil_div(M, R9_SEG);
+    const unsigned blocks = (unsigned)ceil_div((int64_t)strips * segs, R9_NT / 32);
+    stencil9_rs_kernel<E, T><<<blocks, R9_NT, 0, st>>>(src, dst, M, N, strips, segs, w);
 }
 
 template <typename E>
@@ -328,7 +414,7 @@ gb_status stencil9(int64_t M, int64_t N, E *A, E *B, int iters, const E *w_host,
     if (M == 0 || N == 0 || iters == 0) return ok();
     GB_CHECK_ARG(A && B && A != B, "stencil9: A and B must be distinct device buffers");
     GB_CHECK_ARG(w_host != nullptr, "stencil9: null weight window");
-    GB_CHECK_ARG((M + RS_SEG - 1) / RS_SEG < (1 << 30), "stencil9: M too large");
+    GB_CHECK_ARG((M + R9_SEG - 1) / R9_SEG < (1 << 30), "stencil9: M too large");
     W9<E> w;
     for (int i = 0; i < 9; i++) w.w[i] = w_host[i];
     // FP32: 4 sweeps per pass (the window rows of 4 levels fill the register
@@ -355,6 +441,43 @@ gb_status stencil9(int64_t M, int64_t N, E *A, E *B, int iters, const E *w_host,
     return ok();
 }
 
+// Sweeps per pass and rows per segment of the FP32 form: the plan of least
+// estimated time.  A warp's row of t sweeps costs about (t + 1.2) (46 + 28 k)
+// cycles with k warps on its scheduler (measured, t = 6: 89 / 120 / 153 / 191 a sweep at
+// k = 1 / 2 / 3 / 4; 146 in waves of four that other waves follow; the 1.2
+// are the row's loads and stores), a pass about 6000 cycles besides (launch,
+// first rows).  Long segments waste few halo rows, short ones fill the GPU:
+// 1000 x 1500, 60 sweeps, measures 105 us in segments of 12 rows, 116 in 24,
+// 120 in 16; 8192 x 8192, 48 sweeps, 1115 us in segments of 84, 1136 in 112,
+// 1153 in 64 (segments of 256 whatever the grid: 2311 and 2620 us).
+struct RsPlan {
+    int launches, seg;
+};
+RsPlan rs_plan(int64_t M, int64_t N, int iters) {
+    RsPlan best{1, 8};
+    double best_cost = 1e300;
+    const double sched = 4.0 * sm_count(), wave = (double)RS_WARPS * sm_count();
+    for (int t = RS_T < iters ? RS_T : iters; t >= 1; t--) {
+        int launches = (int)ceil_div(iters, t);
+        if ((launches & 1) != (iters & 1)) launches++;   // the result lands in B for odd iters, in A for even
+        const int tt = (int)ceil_div(iters, launches);
+        const double strips = (double)ceil_div(N, RS_W - 2 * tt);
+        for (int seg = 8; seg <= 256; seg += seg < 64 ? 4 : 8) {
+            const double warps = strips * (double)ceil_div(M, seg);
+            if (warps > 2147483647.0) continue;
+            const double full = floor(warps / wave), rest = ceil((warps - full * wave) / sched);
+            const double level = full * 122.0 + (rest > 0 ? 46.0 + 28.0 * rest : 0.0);
+            const double cost = launches * (6000.0 + level * (tt + 1.2) * (seg + 2 * tt));
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = RsPlan{launches, seg};
+            }
+        }
+        if (t <= RS_T - 2) break;   // fewer sweeps a pass only add passes (and, on large grids, HBM traffic)
+    }
+    return best;
+}
+
 template <typename T>
 gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *stream) {
     GB_CHECK_ARG(M >= 0 && N >= 0, "stencil2d: negative size");
@@ -362,64 +485,50 @@ gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *
     GB_CHECK_ARG(order >= 0 && order <= 2, "stencil2d: order %d not in 0..2", order);
     if (M == 0 || N == 0 || iters == 0) return ok();
     GB_CHECK_ARG(A && B && A != B, "stencil2d: A and B must be distinct device buffers");
-    // tile and temporal depth: FP32 is HBM-bound (block 8 sweeps); FP64 is
-    // bound by the FP64 pipe, where recomputing halos only costs, so t = 1.
-    const char *rsenv = getenv("GB_STENCIL_RS");   // "0": the shared-memory kernel (measurement)
-    // FP64 keeps the shared-memory kernel with t = 1: it is bound by the FP64
-    // pipe, and the streaming form measured slower there (1.38 vs 1.64 TB/s)
-    const bool rs = sizeof(T) == 4 && !(rsenv && rsenv[0] == '0');
-    const int tmax = sizeof(T) == 4 ? 8 : 1;
-    const int TH = sizeof(T) == 4 ? 64 : 32, TW = sizeof(T) == 4 ? 128 : 64;
-    // launches L with L == iters (mod 2) so the result lands in B for odd
-    // iters and in A for even iters, as with one sweep per launch
-    int L = (int)ceil_div(iters, tmax);
-    if ((L & 1) != (iters & 1)) L += 1;
-    dim3 grid((unsigned)ceil_div(N, TW), (unsigned)ceil_div(M, TH));
-    GB_CHECK_ARG(grid.y <= 65535u, "stencil2d: M too large");
     cudaStream_t st = as_stream(stream);
-    int done = 0;
-    for (int l = 0; l < L; l++) {
-        int t = (iters - done) / (L - l);      // spread evenly
-        int rem = (iters - done) % (L - l);
-        if (rem) t += 1;
-        const T *src = (l % 2 == 0) ? A : B;
-        T *dst = (l % 2 == 0) ? B : A;
-        if (rs) {
-            {
-                const float *s4 = (const float *)src;
-                float *d4 = (float *)dst;
-                switch (t) {
-                    case 1: launch_rs<float, 1>(s4, d4, M, N, order, st); break;
-                    case 2: launch_rs<float, 2>(s4, d4, M, N, order, st); break;
-                    case 3: launch_rs<float, 3>(s4, d4, M, N, order, st); break;
-                    case 4: launch_rs<float, 4>(s4, d4, M, N, order, st); break;
-                    case 5: launch_rs<float, 5>(s4, d4, M, N, order, st); break;
-                    case 6: launch_rs<float, 6>(s4, d4, M, N, order, st); break;
-                    case 7: launch_rs<float, 7>(s4, d4, M, N, order, st); break;
-                    default: launch_rs<float, 8>(s4, d4, M, N, order, st); break;
-                }
+    if (sizeof(T) == 4) {
+        GB_CHECK_ARG(ceil_div(M, 64) <= 65535, "stencil2d: M too large");
+        const RsPlan pl = rs_plan(M, N, iters);
+        // captured launches keep plain stream order
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        GB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+        int done = 0;
+        for (int l = 0; l < pl.launches; l++) {
+            const int t = (int)ceil_div(iters - done, pl.launches - l);   // spread evenly
+            const float *src = (const float *)(l % 2 == 0 ? A : B);
+            float *dst = (float *)(l % 2 == 0 ? B : A);
+            const bool dep = l > 0 && cap == cudaStreamCaptureStatusNone;
+            cudaError_t e;
+            switch (t) {
+                case 1: e = launch_rs<1>(src, dst, M, N, pl.seg, order, dep, st); break;
+                case 2: e = launch_rs<2>(src, dst, M, N, pl.seg, order, dep, st); break;
+                case 3: e = launch_rs<3>(src, dst, M, N, pl.seg, order, dep, st); break;
+                case 4: e = launch_rs<4>(src, dst, M, N, pl.seg, order, dep, st); break;
+                case 5: e = launch_rs<5>(src, dst, M, N, pl.seg, order, dep, st); break;
+                default: e = launch_rs<RS_T>(src, dst, M, N, pl.seg, order, dep, st); break;
             }
+            GB_CUDA_TRY(e);
             GB_LAUNCH_CHECK("stencil_rs_kernel");
             done += t;
-            continue;
         }
-        size_t smem = 2 * (size_t)(TH + 2 * t) * (TW + 2 * t) * sizeof(T);
+        return ok();
+    }
+    // FP64 is bound by the FP64 pipe, where recomputing halos only costs: one
+    // sweep per launch from shared-memory tiles (the streaming form measured
+    // slower there, 1.38 against 1.64 TB/s)
+    constexpr int TH = 32, TW = 64;
+    dim3 grid((unsigned)ceil_div(N, TW), (unsigned)ceil_div(M, TH));
+    GB_CHECK_ARG(grid.y <= 65535u, "stencil2d: M too large");
+    const size_t smem = 2 * (size_t)(TH + 2) * (TW + 2) * sizeof(double);
+    for (int l = 0; l < iters; l++) {
+        const double *src = (const double *)(l % 2 == 0 ? A : B);
+        double *dst = (double *)(l % 2 == 0 ? B : A);
         switch (order) {
-            case 0:
-                cudaFuncSetAttribute(stencil_tb_kernel<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                stencil_tb_kernel<T, 0><<<grid, NT, smem, st>>>(src, dst, M, N, t, TH, TW);
-                break;
-            case 1:
-                cudaFuncSetAttribute(stencil_tb_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                stencil_tb_kernel<T, 1><<<grid, NT, smem, st>>>(src, dst, M, N, t, TH, TW);
-                break;
-            default:
-                cudaFuncSetAttribute(stencil_tb_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                stencil_tb_kernel<T, 2><<<grid, NT, smem, st>>>(src, dst, M, N, t, TH, TW);
-                break;
+            case 0: stencil_tb_kernel<double, 0><<<grid, NT, smem, st>>>(src, dst, M, N, 1, TH, TW); break;
+            case 1: stencil_tb_kernel<double, 1><<<grid, NT, smem, st>>>(src, dst, M, N, 1, TH, TW); break;
+            default: stencil_tb_kernel<double, 2><<<grid, NT, smem, st>>>(src, dst, M, N, 1, TH, TW); break;
         }
         GB_LAUNCH_CHECK("stencil_tb_kernel");
-        done += t;
     }
     return ok();
 }
