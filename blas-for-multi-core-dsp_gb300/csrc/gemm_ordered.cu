@@ -13,16 +13,24 @@
 // FP32 products use the double-precision fma() on float operands rounded
 // back to float, as those C loops do (fma() is the double libm function).
 //
-// Tiling: 64x64 C tile per CTA, 256 threads, 4x4 elements per thread,
-// K staged through shared memory 16 at a time.  The tiling does not change
-// the per-element order.  FP64 throughput on GB300 is ~1.2 TFLOP/s, so this
-// kernel is FP64-pipe bound; it is also the library's plain DGEMM.
+// Tiling: a CTA owns a TM x TN tile of C, a thread RM x RN neighbouring
+// elements, K is staged through double-buffered shared memory 16 at a time
+// with the next step's loads in flight.  The tiling does not change the
+// per-element order.
+//
+// FP64 is bound by the FP64 pipe (2 DFMA per clock and SM, ~1.1 TFLOP/s); it
+// is also the library's plain DGEMM.  FP32 would be too, and by the
+// conversions around each double fma; it runs on the FP32 pipe instead (see
+// fmac_step below).
+#include <math.h>
+
 #include "gb_common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace gb {
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
+constexpr int BK = 16;
 
 template <typename T>
 struct Ord;
@@ -32,6 +40,7 @@ struct Ord<double> {
     __device__ static double fmac(double a, double b, double t) { return __fma_rn(a, b, t); }
     __device__ static double add(double a, double b) { return __dadd_rn(a, b); }
     __device__ static double mul(double a, double b) { return __dmul_rn(a, b); }
+    __device__ static bool plain(double) { return true; }
 };
 
 template <>
@@ -42,7 +51,111 @@ struct Ord<float> {
     }
     __device__ static float add(float a, float b) { return __fadd_rn(a, b); }
     __device__ static float mul(float a, float b) { return __fmul_rn(a, b); }
+    // zero, or a magnitude in [2^-40, 2^45] (see fmac_step)
+    __device__ static bool plain(float v) {
+        const unsigned u = __float_as_uint(v) & 0x7fffffffu;
+        return u == 0u || u - 0x2B800000u <= 0x56000000u - 0x2B800000u;
+    }
 };
+
+// One k of a thread's RM x RN products: t = fmac(a, b, t).
+template <typename T, int RM, int RN>
+struct Micro {
+    T a[RM], b[RN];
+    __device__ __forceinline__ void load(const T *As, const T *Bs) {
+#pragma unroll
+        for (int i = 0; i < RM; i++) a[i] = As[i];
+#pragma unroll
+        for (int j = 0; j < RN; j++) b[j] = Bs[j];
+    }
+    __device__ __forceinline__ void exact(T (&t)[RM][RN]) const {
+#pragma unroll
+        for (int i = 0; i < RM; i++)
+#pragma unroll
+            for (int j = 0; j < RN; j++) t[i][j] = Ord<T>::fmac(a[i], b[j], t[i][j]);
+    }
+};
+
+// FP32 without the FP64 pipe.  The wanted value is x = a b + t rounded to 53
+// bits and then to 24.  r = fmaf(a, b, t) rounds x once; the two differ only
+// if the first rounding lands on the midpoint of two floats and x does not.
+// With p + q = a b exactly (q by an fma):
+//  - 2^-22 |p| <= |t| < 16 |p|: x has at most 53 significant bits, the first
+//    rounding changes nothing and r is the result;
+//  - |t| >= 16 |p|: the distance e = x - r = (p - (r - t)) + q is formed in
+//    FP32 (r - t and p - (r - t) are exact, the sum rounds once).  If the two
+//    differ, x lies within 2^-28 of half a spacing of the midpoint, and r + (1 + 2^-21) e
+//    rounds away from r;
+//  - |t| < 2^-22 |p|: not decided here.
+// A thread that finds a product undecided or near a midpoint (5.6e-7 of random
+// products; every tie) redoes its products of that k with the double fma.
+// All this holds while nothing nears the ends of FP32's range: operands are
+// checked as they are staged to be zero or in [2^-40, 2^45], so that products
+// and sums are multiples of 2^-126 below 2^122; a chain with any other operand
+// (Inf and NaN too) runs on the double fma from that slice on.
+// Nine FP32 operations (packed in pairs) and four compares a product in place
+// of a DFMA and its conversions (the FP64 pipe serves 2 lanes a clock and SM,
+// the FP32 pipe 128): 768 x 1000 x 1536
+// takes 0.70 ms, with the double fma 12.0.
+template <int RM, int RN>
+__device__ __forceinline__ void fmac_step(const Micro<float, RM, RN> &m, float (&t)[RM][RN]) {
+    static_assert(RN % 2 == 0, "packed pairs of columns");
+    const uint64_t minus1 = ptx::f2_pack(-1.f, -1.f), grow = ptx::f2_pack(1.f + 0x1p-21f, 1.f + 0x1p-21f);
+    const uint64_t p16 = ptx::f2_pack(16.f, 16.f), ptiny = ptx::f2_pack(0x1p-22f, 0x1p-22f);
+    float r[RM][RN];
+    bool redo = false;
+#pragma unroll
+    for (int j = 0; j < RN; j += 2) {
+        const uint64_t b2 = ptx::f2_pack(m.b[j], m.b[j + 1]), nb2 = ptx::f2_pack(-m.b[j], -m.b[j + 1]);
+#pragma unroll
+        for (int i = 0; i < RM; i++) {
+            const uint64_t a2 = ptx::f2_pack(m.a[i], m.a[i]), t2 = ptx::f2_pack(t[i][j], t[i][j + 1]);
+            const uint64_t p2 = ptx::f2_mul(a2, b2);
+            const uint64_t nq2 = ptx::f2_fma_rn(a2, nb2, p2);       // -q
+            const uint64_t r2 = ptx::f2_fma_rn(a2, b2, t2);
+            const uint64_t z2 = ptx::f2_fma_rn(t2, minus1, r2);     // r - t
+            const uint64_t w2 = ptx::f2_fma_rn(z2, minus1, p2);     // p - (r - t)
+            const uint64_t e2 = ptx::f2_fma_rn(nq2, minus1, w2);    // + q
+            const uint64_t s2 = ptx::f2_fma_rn(e2, grow, r2);
+            float s[2], big[2], tiny[2];
+            ptx::f2_unpack(s2, s[0], s[1]);
+            ptx::f2_unpack(r2, r[i][j], r[i][j + 1]);
+            ptx::f2_unpack(ptx::f2_mul(p2, p16), big[0], big[1]);
+            ptx::f2_unpack(ptx::f2_mul(p2, ptiny), tiny[0], tiny[1]);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float at = fabsf(t[i][j + h]);
+                redo = redo || (at >= fabsf(big[h]) && s[h] != r[i][j + h]) || at < fabsf(tiny[h]);
+            }
+        }
+    }
+    if (redo) {
+        m.exact(t);
+    } else {
+#pragma unroll
+        for (int i = 0; i < RM; i++)
+#pragma unroll
+            for (int j = 0; j < RN; j++) t[i][j] = r[i][j];
+    }
+}
+
+// The first k of a chain: a b rounded to 53 bits (exact) and to 24.
+template <int RM, int RN>
+__device__ __forceinline__ void first_step(const Micro<float, RM, RN> &m, float (&t)[RM][RN]) {
+#pragma unroll
+    for (int i = 0; i < RM; i++)
+#pragma unroll
+        for (int j = 0; j < RN; j++) t[i][j] = __fmaf_rn(m.a[i], m.b[j], 0.f);
+}
+template <int RM, int RN>
+__device__ __forceinline__ void first_step(const Micro<double, RM, RN> &m, double (&t)[RM][RN]) {
+    m.exact(t);
+}
+
+template <int RM, int RN>
+__device__ __forceinline__ void fmac_step(const Micro<double, RM, RN> &m, double (&t)[RM][RN]) {
+    m.exact(t);
+}
 
 struct OrdParams {
     int64_t M, N, K, lda, ldb, ldc;
@@ -54,139 +167,187 @@ struct OrdParams {
     int blas_general;     // C = alpha*c + beta*C_in after the sum
 };
 
-template <typename T>
-__device__ __forceinline__ void load_tiles(const T *__restrict__ A, const T *__restrict__ B, T (*As)[BM + 1],
-                                           T (*Bs)[BN + 1], const OrdParams &p, int64_t m0, int64_t n0,
-                                           int64_t k0, int64_t kend, T alpha) {
-    const int tid = threadIdx.x;
-#pragma unroll
-    for (int r = 0; r < (BM * BK) / NT; r++) {
-        int l = tid + r * NT;
-        int mm, kk;
-        if (p.ta) { mm = l % BM; kk = l / BM; } else { mm = l / BK; kk = l % BK; }
-        int64_t m = m0 + mm, k = k0 + kk;
-        T v = T(0);
-        if (m < p.M && k < kend) v = p.ta ? A[k * p.lda + m] : A[m * p.lda + k];
-        if (p.scale_a) v = Ord<T>::mul(alpha, v);
-        As[kk][mm] = v;
-    }
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / NT; r++) {
-        int l = tid + r * NT;
-        int nn, kk;
-        if (p.tb) { nn = l / BK; kk = l % BK; } else { nn = l % BN; kk = l / BN; }
-        int64_t n = n0 + nn, k = k0 + kk;
-        T v = T(0);
-        if (n < p.N && k < kend) v = p.tb ? B[n * p.ldb + k] : B[k * p.ldb + n];
-        if (p.scale_b) v = Ord<T>::mul(alpha, v);
-        Bs[kk][nn] = v;
-    }
-}
+// Shared memory of a CTA: two buffers of a 16-step slice of op(A) and op(B),
+// k-major; rows padded by 16 bytes (aligned vector reads, spread banks).
+template <typename T, int TM, int TN>
+struct Stage {
+    static constexpr int PAD = 16 / (int)sizeof(T);
+    T A[2][BK][TM + PAD], B[2][BK][TN + PAD];
+};
 
-// Sum op(A)op(B) over k in [ks, ke) into t (a fresh chain, t starts at 0).
-template <typename T>
-__device__ __forceinline__ void chain(const T *__restrict__ A, const T *__restrict__ B, T (*As)[BM + 1],
-                                      T (*Bs)[BN + 1], const OrdParams &p, int64_t m0, int64_t n0, int64_t ks,
-                                      int64_t ke, T alpha, T (&t)[4][4]) {
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+template <typename T, int TM, int TN, int NT>
+struct Loader {
+    static constexpr int NA = TM * BK / NT, NB = TN * BK / NT;
+    static_assert(TM * BK % NT == 0 && TN * BK % NT == 0, "whole elements a thread");
+    T a[NA], b[NB];
+
+    // rows past M (columns past N) repeat the last one: their products are never stored
+    __device__ __forceinline__ void fetch(const T *__restrict__ A, const T *__restrict__ B, const OrdParams &p,
+                                          int64_t m0, int64_t n0, int64_t k0, int64_t kend) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+        for (int r = 0; r < NA; r++) {
+            const int l = (int)threadIdx.x + r * NT;
+            const int mm = p.ta ? l % TM : l / BK, kk = p.ta ? l / TM : l % BK;
+            const int64_t m = m0 + mm < p.M ? m0 + mm : p.M - 1, k = k0 + kk;
+            a[r] = k < kend ? (p.ta ? A[k * p.lda + m] : A[m * p.lda + k]) : T(0);
+        }
 #pragma unroll
-        for (int j = 0; j < 4; j++) t[i][j] = T(0);
-    for (int64_t k0 = ks; k0 < ke; k0 += BK) {
-        __syncthreads();
-        load_tiles<T>(A, B, As, Bs, p, m0, n0, k0, ke, alpha);
-        __syncthreads();
-        int kn = (int)((ke - k0) < BK ? (ke - k0) : BK);
-        for (int kk = 0; kk < kn; kk++) {
-            T a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) t[i][j] = Ord<T>::fmac(a[i], b[j], t[i][j]);
+        for (int r = 0; r < NB; r++) {
+            const int l = (int)threadIdx.x + r * NT;
+            const int nn = p.tb ? l / BK : l % TN, kk = p.tb ? l % BK : l / TN;
+            const int64_t n = n0 + nn < p.N ? n0 + nn : p.N - 1, k = k0 + kk;
+            b[r] = k < kend ? (p.tb ? B[n * p.ldb + k] : B[k * p.ldb + n]) : T(0);
         }
     }
+
+    // into buffer `buf`, scaled; whether an operand is outside the FP32 path's range
+    __device__ __forceinline__ bool store(Stage<T, TM, TN> &s, int buf, const OrdParams &p, T alpha) const {
+        bool odd = false;
+#pragma unroll
+        for (int r = 0; r < NA; r++) {
+            const int l = (int)threadIdx.x + r * NT;
+            const T v = p.scale_a ? Ord<T>::mul(alpha, a[r]) : a[r];
+            odd = odd || !Ord<T>::plain(v);
+            s.A[buf][p.ta ? l / TM : l % BK][p.ta ? l % TM : l / BK] = v;
+        }
+#pragma unroll
+        for (int r = 0; r < NB; r++) {
+            const int l = (int)threadIdx.x + r * NT;
+            const T v = p.scale_b ? Ord<T>::mul(alpha, b[r]) : b[r];
+            odd = odd || !Ord<T>::plain(v);
+            s.B[buf][p.tb ? l % BK : l / TN][p.tb ? l / BK : l % TN] = v;
+        }
+        return odd;
+    }
+};
+
+// Sum op(A)op(B) over k in [ks, ke) into t (a fresh chain, t starts at 0).
+template <typename T, int TM, int TN, int RM, int RN>
+__device__ __forceinline__ void chain(const T *__restrict__ A, const T *__restrict__ B, Stage<T, TM, TN> &s,
+                                      const OrdParams &p, int64_t m0, int64_t n0, int64_t ks, int64_t ke, T alpha,
+                                      T (&t)[RM][RN]) {
+    constexpr int NT = TM / RM * (TN / RN);
+    constexpr int KU = sizeof(T) == 4 ? 2 : 4;   // unrolled steps
+    const int tx = threadIdx.x % (TN / RN), ty = threadIdx.x / (TN / RN);
+#pragma unroll
+    for (int i = 0; i < RM; i++)
+#pragma unroll
+        for (int j = 0; j < RN; j++) t[i][j] = T(0);
+    if (ks >= ke) return;
+    Loader<T, TM, TN, NT> ld;
+    ld.fetch(A, B, p, m0, n0, ks, ke);
+    int buf = 0;
+    // a chain's first buffer was last read before the previous chain's last barrier
+    bool odd = __syncthreads_or(ld.store(s, 0, p, alpha));
+    for (int64_t k0 = ks; k0 < ke; k0 += BK, buf ^= 1) {
+        const bool more = k0 + BK < ke;
+        if (more) ld.fetch(A, B, p, m0, n0, k0 + BK, ke);
+        const int kn = (int)(ke - k0 < BK ? ke - k0 : BK);
+        Micro<T, RM, RN> m;
+        int kk = 0;
+        if (odd) {
+            for (; kk < kn; kk++) {
+                m.load(&s.A[buf][kk][ty * RM], &s.B[buf][kk][tx * RN]);
+                m.exact(t);
+            }
+        } else if (k0 == ks) {
+            m.load(&s.A[buf][0][ty * RM], &s.B[buf][0][tx * RN]);
+            first_step(m, t);
+            kk = 1;
+        }
+        if (kk == 0 && kn == BK) {
+#pragma unroll KU
+            for (int k = 0; k < BK; k++) {
+                m.load(&s.A[buf][k][ty * RM], &s.B[buf][k][tx * RN]);
+                fmac_step(m, t);
+            }
+        } else {
+#pragma unroll 1
+            for (; kk < kn; kk++) {
+                m.load(&s.A[buf][kk][ty * RM], &s.B[buf][kk][tx * RN]);
+                fmac_step(m, t);
+            }
+        }
+        const bool next_odd = more && ld.store(s, buf ^ 1, p, alpha);
+        odd = __syncthreads_or(next_odd) || odd;
+    }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT) gemm_ordered_kernel(const T *__restrict__ A, const T *__restrict__ B,
-                                                          T *__restrict__ C, OrdParams p, T alpha, T beta) {
-    __shared__ T As[BK][BM + 1];
-    __shared__ T Bs[BK][BN + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
+// (FP32: two CTAs of 64 x 64 an SM, 128 registers a thread: 4.5 TFLOP/s at 2048 x 2048 x 1024, 3.8
+// with one)
+template <typename T, int TM, int TN, int RM, int RN, bool SLABS>
+__global__ void __launch_bounds__(TM / RM * (TN / RN), sizeof(T) == 4 && !SLABS ? 512 * RM * RN / (TM * TN) : 1)
+    gemm_ordered_kernel(const T *__restrict__ A, const T *__restrict__ B, T *__restrict__ C, OrdParams p, T alpha,
+                        T beta, unsigned tiles_n) {
+    __shared__ __align__(16) Stage<T, TM, TN> s;
+    const int tx = threadIdx.x % (TN / RN), ty = threadIdx.x / (TN / RN);
+    const int64_t m0 = (int64_t)(blockIdx.x / tiles_n) * TM, n0 = (int64_t)(blockIdx.x % tiles_n) * TN;
 
-    T c[4][4], t[4][4];
+    T c[RM][RN], t[RM][RN];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < RM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int64_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+        for (int j = 0; j < RN; j++) {
+            const int64_t m = m0 + ty * RM + i, n = n0 + tx * RN + j;
             c[i][j] = (p.start_from_c && m < p.M && n < p.N) ? C[m * p.ldc + n] : T(0);
         }
 
-    if (p.ka == 0) {
+    if (!SLABS) {
         // two-level: full K blocks, then the (possibly empty) tail block
         const int64_t kfull = p.K - p.K % p.kg;
-        for (int64_t kb = 0; kb < kfull; kb += p.kg) {
-            chain<T>(A, B, As, Bs, p, m0, n0, kb, kb + p.kg, alpha, t);
+        for (int64_t kb = 0; kb <= kfull; kb += p.kg) {
+            chain<T, TM, TN, RM, RN>(A, B, s, p, m0, n0, kb, kb < kfull ? kb + p.kg : p.K, alpha, t);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < RM; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) c[i][j] = Ord<T>::add(c[i][j], t[i][j]);
+                for (int j = 0; j < RN; j++) c[i][j] = Ord<T>::add(c[i][j], t[i][j]);
         }
-        chain<T>(A, B, As, Bs, p, m0, n0, kfull, p.K, alpha, t);
+        if (p.scalar_beta) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+            for (int i = 0; i < RM; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                c[i][j] = Ord<T>::add(c[i][j], t[i][j]);
-                if (p.scalar_beta) c[i][j] = Ord<T>::add(c[i][j], beta);
-            }
+                for (int j = 0; j < RN; j++) c[i][j] = Ord<T>::add(c[i][j], beta);
+        }
     } else {
         // three-level: slabs of ka inside blocks of kg (min-sized at the end)
-        T to[4][4], ti[4][4];
+        T to[RM][RN], ti[RM][RN];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < RM; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) to[i][j] = T(0);
+            for (int j = 0; j < RN; j++) to[i][j] = T(0);
         for (int64_t ko = 0; ko < p.K; ko += p.kg) {
             int64_t kgc = p.kg < p.K - ko ? p.kg : p.K - ko;
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < RM; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) ti[i][j] = T(0);
+                for (int j = 0; j < RN; j++) ti[i][j] = T(0);
             for (int64_t ki = 0; ki < kgc; ki += p.ka) {
                 int64_t kac = p.ka < kgc - ki ? p.ka : kgc - ki;
-                chain<T>(A, B, As, Bs, p, m0, n0, ko + ki, ko + ki + kac, alpha, t);
+                chain<T, TM, TN, RM, RN>(A, B, s, p, m0, n0, ko + ki, ko + ki + kac, alpha, t);
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+                for (int i = 0; i < RM; i++)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) ti[i][j] = Ord<T>::add(ti[i][j], t[i][j]);
+                    for (int j = 0; j < RN; j++) ti[i][j] = Ord<T>::add(ti[i][j], t[i][j]);
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < RM; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) to[i][j] = Ord<T>::add(to[i][j], ti[i][j]);
+                for (int j = 0; j < RN; j++) to[i][j] = Ord<T>::add(to[i][j], ti[i][j]);
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < RM; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                T s = p.scalar_beta ? Ord<T>::add(to[i][j], beta) : to[i][j];
-                c[i][j] = Ord<T>::add(c[i][j], s);
+            for (int j = 0; j < RN; j++) {
+                const T v = p.scalar_beta ? Ord<T>::add(to[i][j], beta) : to[i][j];
+                c[i][j] = Ord<T>::add(c[i][j], v);
             }
     }
 
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < RM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int64_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+        for (int j = 0; j < RN; j++) {
+            const int64_t m = m0 + ty * RM + i, n = n0 + tx * RN + j;
             if (m < p.M && n < p.N) {
                 T v = c[i][j];
                 if (p.blas_general) {
@@ -196,6 +357,27 @@ __global__ void __launch_bounds__(NT) gemm_ordered_kernel(const T *__restrict__ 
                 C[m * p.ldc + n] = v;
             }
         }
+}
+
+template <typename T, int TM, int TN, int RM, int RN>
+gb_status launch_tile(const GemmArgs &g, const OrdParams &p) {
+    const int64_t tn = ceil_div(g.N, TN), tiles = ceil_div(g.M, TM) * tn;
+    if (tiles > 0x7fffffff) return set_status(GB_ERR_UNSUPPORTED, "ordered gemm: C too large");
+    const int nt = TM / RM * (TN / RN);
+    auto kernel = p.ka > 0 ? gemm_ordered_kernel<T, TM, TN, RM, RN, true> : gemm_ordered_kernel<T, TM, TN, RM, RN, false>;
+    kernel<<<(unsigned)tiles, nt, 0, g.stream>>>((const T *)g.A, (const T *)g.B, (T *)g.C, p, (T)g.alpha, (T)g.beta,
+                                                 (unsigned)tn);
+    GB_LAUNCH_CHECK("gemm_ordered_kernel");
+    return ok();
+}
+
+// Estimated time (ns) of one k with this tiling: the SM with the most tiles
+// decides, each tile costs `tile`, and an SM with few of them still waits out
+// a step's latency, `least`.
+inline double step_ns(const GemmArgs &g, int tm, int tn, double least, double tile, double once = 0.0) {
+    const double tiles = (double)ceil_div(g.M, tm) * (double)ceil_div(g.N, tn);
+    const double t = ceil(tiles / sm_count()) * tile + once;
+    return t > least ? t : least;
 }
 
 template <typename T>
@@ -219,12 +401,25 @@ gb_status launch(const GemmArgs &g) {
         if (g.alpha_on_b) p.scale_b = 1; else p.scale_a = 1;
     }
     if (g.M == 0 || g.N == 0) return ok();
-    dim3 grid((unsigned)ceil_div(g.N, BN), (unsigned)ceil_div(g.M, BM));
-    if (grid.y > 65535u) return set_status(GB_ERR_UNSUPPORTED, "ordered gemm: M too large (%lld)", (long long)g.M);
-    gemm_ordered_kernel<T><<<grid, NT, 0, g.stream>>>((const T *)g.A, (const T *)g.B, (T *)g.C, p, (T)g.alpha,
-                                                     (T)g.beta);
-    GB_LAUNCH_CHECK("gemm_ordered_kernel");
-    return ok();
+    if (ceil_div(g.M, 64) > 65535)
+        return set_status(GB_ERR_UNSUPPORTED, "ordered gemm: M too large (%lld)", (long long)g.M);
+    // The tiling of least estimated time; the constants are measured (a k of
+    // FP32 64 x 64 / 32 x 64 / 32 x 32: 340 / 280 / 165 ns alone on an SM, 268 /
+    // 140 / 87 a tile when there are many; FP64 32 x 32 / 16 x 16: 310 / 190 and 268 /
+    // 72).  FP32 768 x 1000 x 1536: 703 us in 32 x 64, 796 in 32 x 32, 839 in
+    // 64 x 64; 256^3: 75 / 43 / 92; 2048 x 2048 x 512: 1004 / 1182 / 961.  FP64 256^3:
+    // 81 us in 32 x 32, 55 in 16 x 16; 512^3: 287 / 310 (64 x 64: 283 and 554).
+    if constexpr (sizeof(T) == 8) {
+        const double t32 = step_ns(g, 32, 32, 310, 268), t16 = step_ns(g, 16, 16, 190, 72, 60);
+        if (t16 < t32) return launch_tile<T, 16, 16, 2, 2>(g, p);
+        return launch_tile<T, 32, 32, 2, 2>(g, p);
+    } else {
+        const double t64 = step_ns(g, 64, 64, 340, 268), t48 = step_ns(g, 32, 64, 280, 140, 40),
+                     t32 = step_ns(g, 32, 32, 165, 87);
+        if (t32 < t48 && t32 < t64) return launch_tile<T, 32, 32, 2, 2>(g, p);
+        if (t48 < t64) return launch_tile<T, 32, 64, 4, 4>(g, p);
+        return launch_tile<T, 64, 64, 4, 4>(g, p);
+    }
 }
 
 }  // namespace
