@@ -164,6 +164,13 @@ struct GemmArgs {
 gb_status launch_gemm_ordered_f64(const GemmArgs &g);
 gb_status launch_gemm_ordered_f32(const GemmArgs &g);
 gb_status launch_sgemm_simt(const GemmArgs &g);
+// sgemm_small.cu: tile side (32 or 64) and CTAs along K of a product too small for 128 x 128 tiles;
+// tile 0: it is not.
+struct SmallPlan {
+    int tile, split;
+};
+SmallPlan sgemm_small_plan(const GemmArgs &g);
+gb_status launch_sgemm_small(const GemmArgs &g, SmallPlan plan);
 gb_status launch_dgemm_dmma(const GemmArgs &g);
 gb_status launch_sgemm_bf16x3(const GemmArgs &g);
 gb_status launch_sgemm_bf16x6(const GemmArgs &g);

@@ -11,7 +11,8 @@
 // 128x128 C tile per CTA, K step 8, 256 threads with an 8x8 register tile
 // each, shared memory double-buffered with the next tile prefetched into
 // registers while the current one is consumed.  alpha/beta are applied in
-// the epilogue (BLAS, scalar-beta or accumulate semantics).
+// the epilogue (BLAS, scalar-beta or accumulate semantics).  Products whose
+// tiles would leave SMs idle go to sgemm_small.cu.
 #include "gb_common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -205,6 +206,8 @@ gb_status launch_mode(const GemmArgs &g, const SimtParams &p, bool vec) {
 gb_status launch_sgemm_simt(const GemmArgs &g) {
     if (g.M == 0 || g.N == 0) return ok();
     if (ceil_div(g.M, BM) > 65535) return set_status(GB_ERR_UNSUPPORTED, "simt sgemm: M too large");
+    const SmallPlan plan = sgemm_small_plan(g);
+    if (plan.tile) return launch_sgemm_small(g, plan);
     SimtParams p{g.M, g.N, g.K, g.lda, g.ldb, g.ldc, (float)g.alpha, (float)g.beta, g.semantics};
     bool vec = (g.lda % 4 == 0) && (g.ldb % 4 == 0) && ((uintptr_t)g.A % 16 == 0) && ((uintptr_t)g.B % 16 == 0);
     if (!g.ta && !g.tb) return launch_mode<false, false>(g, p, vec);
