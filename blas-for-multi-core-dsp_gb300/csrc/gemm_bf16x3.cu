@@ -23,8 +23,9 @@
 //     K-major), Kp = K rounded up to 64 with zeros.  The transpose modes are
 //     absorbed here (a row-major or a transposed read, always a K-major
 //     write), so the GEMM kernel has one operand layout.
-//  3. gemm: persistent, one CTA per SM over 128 x 256 C tiles, K in blocks of
-//     32 (one 64-byte swizzle atom), a 4-stage TMA -> shared memory pipeline
+//  3. gemm: persistent, one CTA per SM over 128 x 256 C tiles (128 x 128 or
+//     128 x 64 where those would leave SMs idle), K in blocks of 32 (one
+//     64-byte swizzle atom), a 4- to 8-stage TMA -> shared memory pipeline
 //     with mbarriers; warp 0 issues TMA, warp 1 issues tcgen05.mma (M=128,
 //     N=256, K=16, three products per K step into a TMEM accumulator of 256
 //     columns, two accumulators alternating), the epilogue warps read the
@@ -34,6 +35,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -200,6 +202,13 @@ __device__ __forceinline__ void split_entry_guard(const unsigned long long *done
     if (must_wait) ptx::pdl_wait();   // returns at once when not launched as a dependent
 }
 
+// The end of a scan or split grid that may overlap the previous call's GEMM:
+// one thread keeps the grid from completing before that GEMM has, so the
+// stream order of what follows is unchanged.
+__device__ __forceinline__ void split_exit() {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ptx::pdl_wait();
+}
+
 // ------------------------------------------------------------------ scan
 // Largest |x| bit pattern of every row of op(X) (rows x K) -- non-negative
 // floats order as their bit patterns -- by atomicMax from 64 x 256 tiles.
@@ -305,8 +314,7 @@ __global__ void __launch_bounds__(256) maxbits_kernel(const __grid_constant__ Sc
         if (a.scan_done) atomicAdd(a.scan_done, 1ull);
         ptx::pdl_launch_dependents();
     }
-    // as split_kernel: the grid does not complete before the previous grid has
-    if (blockIdx.x == 0 && threadIdx.x == 0) ptx::pdl_wait();
+    split_exit();
 }
 
 // The split pass of the FP16 form waits for every CTA of its scan: `expect`
@@ -363,62 +371,14 @@ struct Pieces<true> {
     static __device__ __forceinline__ uint16_t bits(T v) { return __half_as_ushort(v); }
 };
 
-// out_hi/out_lo(/out_lo2): rows x kp (K-major).  Source element (r, k):
-// trans ? X[k*ldx + r] : X[r*ldx + k].  32x32 tiles through shared memory
-// so both the read and the write are coalesced in either layout.  With
-// out_lo2 the value is cut in three BF16 pieces (hi, mid, lo: 24 bits).
-// mbits (FP16 form): the largest |x| bit pattern of each row (low 32 bits).
-template <bool F16>
-__global__ void __launch_bounds__(256) split_kernel(const float *__restrict__ X, int64_t ldx, int trans, int64_t rows,
-                                                    int64_t K, int64_t kp, uint16_t *__restrict__ out_hi,
-                                                    uint16_t *__restrict__ out_lo, uint16_t *__restrict__ out_lo2,
-                                                    const unsigned long long *__restrict__ mbits,
-                                                    const unsigned long long *done, unsigned long long expect,
-                                                    const unsigned long long *scan_done,
-                                                    unsigned long long scan_expect, int *err) {
-    using P = Pieces<F16>;
-    __shared__ float tile[32][33];
-    if (scan_done) scan_entry_wait(scan_done, scan_expect, err);
-    else split_entry_guard(done, expect);
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;   // 32 x 8
-    const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
-#pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-        float v = 0.f;
-        if (trans) {   // coalesced along r: tile[k][r]
-            int64_t k = k0 + ty + i, r = r0 + tx;
-            if (k < K && r < rows) v = X[k * ldx + r];
-            tile[ty + i][tx] = v;
-        } else {       // coalesced along k: tile[k][r] via transposed store
-            int64_t r = r0 + ty + i, k = k0 + tx;
-            if (k < K && r < rows) v = X[r * ldx + k];
-            tile[tx][ty + i] = v;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-        int64_t r = r0 + ty + i, k = k0 + tx;
-        if (r < rows && k < kp) {
-            typename P::T h, l, l2;
-            P::cut(tile[tx][ty + i], F16 ? f16_line_scale((unsigned)mbits[r]) : 0, h, l, l2);
-            out_hi[r * kp + k] = P::bits(h);
-            out_lo[r * kp + k] = P::bits(l);
-            if (out_lo2) out_lo2[r * kp + k] = P::bits(l2);
-        }
-    }
-    // possibly launched to overlap the previous call's GEMM: one thread keeps the grid from
-    // completing before that grid has, so the stream order of the GEMM that follows is unchanged
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ptx::pdl_wait();
-}
-
-// Vectorised split of both operands in one launch (16-byte aligned sources
-// with leading dimensions a multiple of 4).  A CTA converts a 64 x 64 block
+// Split of both operands in one launch.  Pieces: rows x kp, K-major, zeros
+// past K.  Source element (r, k): trans ? X[k*ldx + r] : X[r*ldx + k], read
+// 16 bytes at a time (VEC: aligned bases, leading dimensions a multiple of 4)
+// or value by value.  A CTA converts a 64 x 64 block
 // of (row, k): a K-contiguous source is read and written 4 values at a time
 // straight from registers; a row-contiguous source is read 4 rows at a time
 // into shared memory and written 4 k at a time, in two halves of 32 k (a
-// small tile, so that a split CTA fits on an SM beside a GEMM CTA).  Same values as
-// split_kernel, about two-thirds of its time at the 4096^2 operands.
+// small tile, so that a split CTA fits on an SM beside a GEMM CTA).
 struct SplitOp {
     const float *X;
     int64_t ldx, rows, tiles_k, tiles;
@@ -458,8 +418,20 @@ __device__ __forceinline__ void split_store4(const SplitArgs &a, const SplitOp &
     if (a.np == 3) *reinterpret_cast<uint2 *>(o.out[2] + off) = make_uint2(l2[0], l2[1]);
 }
 
-template <bool F16>
-__global__ void __launch_bounds__(256) split_vec_kernel(const __grid_constant__ SplitArgs a) {
+// four consecutive values at src, those from `left` on zero
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float *src, int64_t left) {
+    if (VEC && left >= 4) return __ldg(reinterpret_cast<const float4 *>(src));
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (left > 0) x.x = __ldg(src);
+    if (left > 1) x.y = __ldg(src + 1);
+    if (left > 2) x.z = __ldg(src + 2);
+    if (left > 3) x.w = __ldg(src + 3);
+    return x;
+}
+
+template <bool F16, bool VEC>
+__global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ SplitArgs a) {
     __shared__ float tile[32][65];   // 8.3 KB: fits beside a GEMM CTA on its SM
     if (a.scan_done) scan_entry_wait(a.scan_done, a.scan_expect, a.err);
     else split_entry_guard(a.done, a.expect);
@@ -474,19 +446,11 @@ __global__ void __launch_bounds__(256) split_vec_kernel(const __grid_constant__ 
         for (int i = 0; i < 4; i++) {
             const int64_t r = r0 + rl + 16 * i, k = k0 + c4;
             if (r >= o.rows) continue;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            const float *src = o.X + r * o.ldx + k;
-            if (k + 3 < a.K) {
-                const float4 x = __ldg(reinterpret_cast<const float4 *>(src));
-                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (k + q < a.K) v[q] = src[q];
-            }
+            const float4 x = load4<VEC>(o.X + r * o.ldx + k, a.K - k);
+            const float v[4] = {x.x, x.y, x.z, x.w};
             split_store4<F16>(a, o, r, k, v);
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) ptx::pdl_wait();   // as split_kernel
+        split_exit();
         return;
     }
     // row-contiguous source: the 64 x 64 block in two halves of 32 k through tile[k][r]
@@ -498,17 +462,7 @@ __global__ void __launch_bounds__(256) split_vec_kernel(const __grid_constant__ 
         for (int i = 0; i < 2; i++) {   // tile[k][r], 4 consecutive r per load
             const int kl = rl + 16 * i;
             const int64_t k = k0 + 32 * h + kl, r = r0 + c4;
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < a.K) {
-                const float *src = o.X + k * o.ldx + r;
-                if (r + 3 < o.rows) {
-                    x = __ldg(reinterpret_cast<const float4 *>(src));
-                } else {
-                    if (r < o.rows) x.x = src[0];
-                    if (r + 1 < o.rows) x.y = src[1];
-                    if (r + 2 < o.rows) x.z = src[2];
-                }
-            }
+            const float4 x = load4<VEC>(o.X + k * o.ldx + r, k < a.K ? o.rows - r : 0);
             tile[kl][c4] = x.x; tile[kl][c4 + 1] = x.y; tile[kl][c4 + 2] = x.z; tile[kl][c4 + 3] = x.w;
         }
         __syncthreads();
@@ -521,7 +475,7 @@ __global__ void __launch_bounds__(256) split_vec_kernel(const __grid_constant__ 
             split_store4<F16>(a, o, r, k0 + 32 * h + kw, v);
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) ptx::pdl_wait();   // as split_kernel
+    split_exit();
 }
 
 // ------------------------------------------------------------------- gemm
@@ -531,7 +485,7 @@ __global__ void __launch_bounds__(256) split_vec_kernel(const __grid_constant__ 
 // holding NP 16-bit pieces of the A and B tiles (NP = 2: hi, lo with BN =
 // 256; NP = 3: hi, mid, lo with BN = 128).  Two TMEM accumulators: the
 // epilogue of tile (or accumulator chunk) i overlaps the MMAs of i+1.
-constexpr int BM = 128, BK = 32, STAGES = 4, GROUP_M = 8;
+constexpr int BM = 128, BK = 32, GROUP_M = 8;
 constexpr int A_TILE = BM * BK * 2;            // 8 KB
 constexpr int EPI_BYTES = 4 * 32 * 33 * 4;     // four warps' 32 x 32 staging, padded
 
@@ -542,6 +496,7 @@ template <int NP, int BN, int EW>
 struct TwoPass {
     static constexpr int B_TILE = BN * BK * 2;
     static constexpr int STAGE_BYTES = NP * A_TILE + NP * B_TILE;
+    static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;   // 4 (48 KB: two pieces, BN = 256; three, 128), 6, 8
     static constexpr int NT = 64 + 32 * EW;
     // C staging: 4 warps x 32 x 32 (padded 33), or 8 warps x 32 x 16 (padded 17)
     static constexpr int EPI = EW == 4 ? EPI_BYTES : 8 * 32 * 17 * 4;
@@ -674,7 +629,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
     static_assert(!SEP || BN == 128, "the separated folding form keeps a 128-column total per thread");
     static_assert(EW == 4 || (FOLD && BN == 256), "eight epilogue warps: the wide folding form");
     static_assert(!F16 || EW == 8, "FP16 pieces: the wide folding form");
-    constexpr int B_TILE = CF::B_TILE, STAGE_BYTES = CF::STAGE_BYTES;
+    constexpr int B_TILE = CF::B_TILE, STAGE_BYTES = CF::STAGE_BYTES, STAGES = CF::STAGES;
     constexpr uint32_t ACC_COLS = SEP ? 256 : BN, TMEM_COLS = 2 * ACC_COLS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -711,6 +666,9 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    // launched as a dependent of the split pass: the set-up above overlaps it, its pieces are waited
+    // for here (and, through its last thread, everything before it on the stream)
+    ptx::pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {   // TMA producer
@@ -1495,26 +1453,29 @@ static void span(const void *p, bool trans, int64_t rows, int64_t cols, int64_t 
     hi = lo + (uintptr_t)(((sr - 1) * ld + sc) * elem);
 }
 
+// bn: tile width; 128 with the 256-wide folding kernel runs every tile as two halves
 template <int NP, int BN, bool FOLD, bool F16, int EW>
-static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64_t kp, const EpiParams &base,
-                                 int *grid_out) {
+static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64_t kp, const EpiParams &base, int bn,
+                                 bool dependent, int *grid_out) {
     using CF = TwoPass<NP, BN, EW>;
+    auto kernel = bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW>;
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
-        GB_CUDA_TRY(cudaFuncSetAttribute(bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM_BYTES));
+        GB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM_BYTES));
         device_setup_done(attr);
     }
     const int tiles_m = (int)ceil_div(g.M, BM), tiles_n = (int)ceil_div(g.N, BN);
     const int tiles = tiles_m * tiles_n;
-    const int grid = tiles < sm_count() ? tiles : sm_count();
+    const bool halves = bn < BN;
+    const int64_t items = halves ? 2 * (int64_t)tiles : tiles;
+    const int grid = items < sm_count() ? (int)items : sm_count();
     // half-tile tail when the last wave is at most half full (whole tiles
     // would leave most of the GPU idle for a tile time); GB_BF16X3_HALF=0 off.
     // The folding form keeps whole tiles unless GB_BF16X3_HALF=1: its halves
     // fold and store as often as whole tiles for half the MMA work, and the
     // FP16X3 call at 4096^3 measured 0.383 ms with them against 0.368 without.
-    int half_start = tiles;
-    {
+    int half_start = halves ? 0 : tiles;
+    if (!halves) {
         const char *e = getenv("GB_BF16X3_HALF");
         const int rem = tiles % grid;
         const bool on = FOLD ? (EW == 8 && e && e[0] == '1') : !(e && e[0] == '0');
@@ -1526,7 +1487,17 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
     p.tiles_n = tiles_n;
     p.chunk_kb = FOLD ? (p.chunk_kb > 0 ? p.chunk_kb : p.num_kb) : 1;
     p.half_start = half_start;
-    bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW><<<grid, CF::NT, CF::SMEM_BYTES, g.stream>>>(maps, p);
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(CF::NT);
+    cfg.dynamicSmemBytes = CF::SMEM_BYTES;
+    cfg.stream = g.stream;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = dependent ? 1 : 0;
+    GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p));
     GB_LAUNCH_CHECK("bf16x3_gemm_kernel");
     *grid_out = grid;
     return ok();
@@ -1534,18 +1505,49 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
 
 template <bool F16>
 static gb_status gemm_launch(const GemmArgs &g, int np, int fold_kb, const PieceMaps &maps, int64_t kp,
-                             const EpiParams &p, int *grid) {
+                             const EpiParams &p, int bn, bool dependent, int *grid) {
     if constexpr (!F16) {   // three pieces are BF16 only
         if (np == 3)
-            return fold_kb > 0 ? two_pass_launch<3, 128, true, false, 4>(g, maps, kp, p, grid)
-                               : two_pass_launch<3, 128, false, false, 4>(g, maps, kp, p, grid);
+            return fold_kb > 0 ? two_pass_launch<3, 128, true, false, 4>(g, maps, kp, p, bn, dependent, grid)
+                               : two_pass_launch<3, 128, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
     }
     if constexpr (F16) {   // always the wide folding form (fold_kb 0: one chunk over all of K)
-        return two_pass_launch<2, 256, true, true, 8>(g, maps, kp, p, grid);
+        return two_pass_launch<2, 256, true, true, 8>(g, maps, kp, p, bn, dependent, grid);
     } else {
-        return fold_kb > 0 ? two_pass_launch<2, 256, true, false, 8>(g, maps, kp, p, grid)
-                           : two_pass_launch<2, 256, false, false, 4>(g, maps, kp, p, grid);
+        if (fold_kb > 0) return two_pass_launch<2, 256, true, false, 8>(g, maps, kp, p, bn, dependent, grid);
+        switch (bn) {
+            case 64: return two_pass_launch<2, 64, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
+            case 128: return two_pass_launch<2, 128, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
+            default: return two_pass_launch<2, 256, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
+        }
     }
+}
+
+// Width of the C tiles.  256 columns need the least operand traffic per
+// product (48 KB a k-block of 32 in at least 0.66 us, against 0.40 for 128
+// and 0.34 for 64, which the L2 -> SM path bounds), narrow ones fill more SMs:
+// the width of least estimated time (waves of tiles x k-blocks, a tail wave
+// of 256 at most half full counted half, plus launch and epilogue).  Measured, us:
+//
+//                     64      128     256
+//   513^3             13.5    17.4    27.4
+//   1111x937x1500     24.5    27.9    39.5
+//   1280^3            34.7    24.4    35.5
+//   2048^3            95.9    58.7    60.8
+//   3000^3            265     149     121
+//
+// The folding form has 256-wide tiles only; as halves (128) they pay while
+// all of them run at once with SMs to spare: 1024^3 26.0 against 32.0 us,
+// 1280^3 30.0 / 37.9, but 1500^3 (144 halves on 152 SMs) 49.6 / 47.0.
+static int tile_width(const GemmArgs &g, int np, bool fold) {
+    if (np == 3) return 128;
+    const double sms = sm_count(), kb = (double)ceil_div(g.K, BK);
+    auto waves = [&](int bn) { return (double)ceil_div(g.M, BM) * (double)ceil_div(g.N, bn) / sms; };
+    if (fold) return 2.0 * waves(256) <= 0.8 ? 128 : 256;
+    const double whole = floor(waves(256)), rest = waves(256) - whole;
+    const double t64 = 7.0 + ceil(waves(64)) * kb * 0.34, t128 = 8.0 + ceil(waves(128)) * kb * 0.40,
+                 t256 = 12.0 + (whole + (rest == 0.0 ? 0.0 : whole > 0.0 && rest <= 0.5 ? 0.5 : 1.0)) * kb * 0.66;
+    return t64 < t128 && t64 < t256 ? 64 : t128 < t256 ? 128 : 256;
 }
 
 // Split pass (NP 16-bit pieces per operand, K-major) + MMA kernel; fold_kb >
@@ -1584,10 +1586,9 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     GB_CUDA_TRY(cudaGetDevice(&dev));
     static std::atomic<uint64_t> carve{0};
     if (device_setup_needed(carve)) {   // the GEMM's shared-memory configuration, so a split fits beside it
-        GB_CUDA_TRY(cudaFuncSetAttribute(split_vec_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        GB_CUDA_TRY(cudaFuncSetAttribute(split_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        GB_CUDA_TRY(cudaFuncSetAttribute(split_vec_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        GB_CUDA_TRY(cudaFuncSetAttribute(split_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        for (auto kernel : {split_kernel<true, true>, split_kernel<true, false>, split_kernel<false, true>,
+                            split_kernel<false, false>})
+            GB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         GB_CUDA_TRY(cudaFuncSetAttribute(maxbits_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         device_setup_done(carve);
     }
@@ -1666,7 +1667,9 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
 
     // split: op(A)(m, k) = ta ? A[k*lda + m] : A[m*lda + k]
     //        op(B)^T(n, k) = op(B)(k, n) = tb ? B[n*ldb + k] : B[k*ldb + n]
-    if (vec) {
+    {
+        if (!vec && (ceil_div(g.M, 32) > 65535 || ceil_div(g.N, 32) > 65535))
+            return set_status(GB_ERR_UNSUPPORTED, "bf16x3: M or N too large");
         SplitArgs sa;
         memset(&sa, 0, sizeof(sa));
         sa.K = g.K; sa.kp = kp; sa.np = np; sa.done = gdone; sa.expect = expect;
@@ -1683,49 +1686,21 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
         cfg.stream = g.stream;
         cfg.attrs = pdl_attr;
         cfg.numAttrs = pdl ? 1 : 0;
-        if (f16) GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_vec_kernel<true>, sa));
-        else GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_vec_kernel<false>, sa));
+        auto kernel = f16 ? (vec ? split_kernel<true, true> : split_kernel<true, false>)
+                          : (vec ? split_kernel<false, true> : split_kernel<false, false>);
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, sa));
         GB_LAUNCH_CHECK("bf16x3 split");
-    } else {
-        dim3 sgA((unsigned)ceil_div(kp, 32), (unsigned)ceil_div(g.M, 32));
-        dim3 sgB((unsigned)ceil_div(kp, 32), (unsigned)ceil_div(g.N, 32));
-        if (sgA.y > 65535u || sgB.y > 65535u) return set_status(GB_ERR_UNSUPPORTED, "bf16x3: M or N too large");
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = sgA;
-        cfg.blockDim = dim3(256);
-        cfg.stream = g.stream;
-        cfg.attrs = pdl_attr;
-        cfg.numAttrs = pdl ? 1 : 0;
-        const unsigned long long *mb = bits;
-        const unsigned long long *no_scan = nullptr;
-        if (f16)
-            GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kernel<true>, (const float *)g.A, g.lda, g.ta ? 1 : 0, g.M, g.K,
-                                           kp, ap[0], ap[1], (uint16_t *)nullptr, mb, gdone, expect,
-                                           (const unsigned long long *)scan_done, scan_expect, err));
-        else
-            GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, split_kernel<false>, (const float *)g.A, g.lda, g.ta ? 1 : 0, g.M,
-                                           g.K, kp, ap[0], ap[1], np == 3 ? ap[2] : (uint16_t *)nullptr, mb, gdone,
-                                           expect, no_scan, 0ull, err));
-        GB_LAUNCH_CHECK("bf16x3 split A");
-        const unsigned long long *mbB = f16 ? bits + g.M : nullptr;
-        if (f16)
-            split_kernel<true><<<sgB, 256, 0, g.stream>>>((const float *)g.B, g.ldb, g.tb ? 0 : 1, g.N, g.K, kp, bp[0],
-                                                          bp[1], nullptr, mbB, nullptr, 0ull, nullptr, 0ull, err);
-        else
-            split_kernel<false><<<sgB, 256, 0, g.stream>>>((const float *)g.B, g.ldb, g.tb ? 0 : 1, g.N, g.K, kp,
-                                                           bp[0], bp[1], np == 3 ? bp[2] : nullptr, nullptr, nullptr,
-                                                           0ull, nullptr, 0ull, err);
-        GB_LAUNCH_CHECK("bf16x3 split B");
     }
 
-    const int bn = np == 3 ? 128 : 256;
+    const int bn = tile_width(g, np, fold_kb > 0 || f16);
+    const int box = np == 2 && (fold_kb > 0 || f16) ? 256 : bn;   // rows of a B box (the halves have half boxes)
     PieceMaps maps;
     memset(&maps, 0, sizeof(maps));
     bool okm = true;
     for (int i = 0; i < np; i++) {   // 2-byte elements, copied as they are (BF16 or FP16)
         okm = okm && make_tmap_bf16(&maps.a[i], ap[i], kp, g.M, kp * 2, BK, BM, 64);
-        okm = okm && make_tmap_bf16(&maps.b[i], bp[i], kp, g.N, kp * 2, BK, bn, 64);
-        okm = okm && make_tmap_bf16(&maps.bh[i], bp[i], kp, g.N, kp * 2, BK, bn / 2, 64);
+        okm = okm && make_tmap_bf16(&maps.b[i], bp[i], kp, g.N, kp * 2, BK, box, 64);
+        okm = okm && make_tmap_bf16(&maps.bh[i], bp[i], kp, g.N, kp * 2, BK, box / 2, 64);
     }
     if (!okm) return set_status(GB_ERR_CUDA, "bf16x3: cuTensorMapEncodeTiled failed");
     EpiParams p;
@@ -1742,8 +1717,9 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
         p.ta = g.ta ? 1 : 0; p.tb = g.tb ? 1 : 0;
     }
     int grid = 0;
-    gb_status s = f16 ? gemm_launch<true>(g, np, fold_kb, maps, kp, p, &grid)
-                      : gemm_launch<false>(g, np, fold_kb, maps, kp, p, &grid);
+    const bool dependent = pdl_env && !capturing;
+    gb_status s = f16 ? gemm_launch<true>(g, np, fold_kb, maps, kp, p, bn, dependent, &grid)
+                      : gemm_launch<false>(g, np, fold_kb, maps, kp, p, bn, dependent, &grid);
     if (s != GB_OK) return s;
     if (done) st.launched += (unsigned long long)grid;
     st.valid = done != nullptr;
