@@ -26,11 +26,12 @@
 
 #include "gb_common.cuh"
 #include "sm100_ptx.cuh"
+#include "tile_stage.cuh"
 
 namespace gb {
 namespace {
 
-constexpr int BK = 16;
+constexpr int BK = STAGE_K;
 
 template <typename T>
 struct Ord;
@@ -167,59 +168,19 @@ struct OrdParams {
     int blas_general;     // C = alpha*c + beta*C_in after the sum
 };
 
-// Shared memory of a CTA: two buffers of a 16-step slice of op(A) and op(B),
-// k-major; rows padded by 16 bytes (aligned vector reads, spread banks).
-template <typename T, int TM, int TN>
-struct Stage {
-    static constexpr int PAD = 16 / (int)sizeof(T);
-    T A[2][BK][TM + PAD], B[2][BK][TN + PAD];
-};
-
+// Stage a slice, scaled; whether an operand is outside the FP32 path's range.
 template <typename T, int TM, int TN, int NT>
-struct Loader {
-    static constexpr int NA = TM * BK / NT, NB = TN * BK / NT;
-    static_assert(TM * BK % NT == 0 && TN * BK % NT == 0, "whole elements a thread");
-    T a[NA], b[NB];
-
-    // rows past M (columns past N) repeat the last one: their products are never stored
-    __device__ __forceinline__ void fetch(const T *__restrict__ A, const T *__restrict__ B, const OrdParams &p,
-                                          int64_t m0, int64_t n0, int64_t k0, int64_t kend) {
-#pragma unroll
-        for (int r = 0; r < NA; r++) {
-            const int l = (int)threadIdx.x + r * NT;
-            const int mm = p.ta ? l % TM : l / BK, kk = p.ta ? l / TM : l % BK;
-            const int64_t m = m0 + mm < p.M ? m0 + mm : p.M - 1, k = k0 + kk;
-            a[r] = k < kend ? (p.ta ? A[k * p.lda + m] : A[m * p.lda + k]) : T(0);
-        }
-#pragma unroll
-        for (int r = 0; r < NB; r++) {
-            const int l = (int)threadIdx.x + r * NT;
-            const int nn = p.tb ? l / BK : l % TN, kk = p.tb ? l % BK : l / TN;
-            const int64_t n = n0 + nn < p.N ? n0 + nn : p.N - 1, k = k0 + kk;
-            b[r] = k < kend ? (p.tb ? B[n * p.ldb + k] : B[k * p.ldb + n]) : T(0);
-        }
-    }
-
-    // into buffer `buf`, scaled; whether an operand is outside the FP32 path's range
-    __device__ __forceinline__ bool store(Stage<T, TM, TN> &s, int buf, const OrdParams &p, T alpha) const {
-        bool odd = false;
-#pragma unroll
-        for (int r = 0; r < NA; r++) {
-            const int l = (int)threadIdx.x + r * NT;
-            const T v = p.scale_a ? Ord<T>::mul(alpha, a[r]) : a[r];
-            odd = odd || !Ord<T>::plain(v);
-            s.A[buf][p.ta ? l / TM : l % BK][p.ta ? l % TM : l / BK] = v;
-        }
-#pragma unroll
-        for (int r = 0; r < NB; r++) {
-            const int l = (int)threadIdx.x + r * NT;
-            const T v = p.scale_b ? Ord<T>::mul(alpha, b[r]) : b[r];
-            odd = odd || !Ord<T>::plain(v);
-            s.B[buf][p.tb ? l % BK : l / TN][p.tb ? l / BK : l % TN] = v;
-        }
-        return odd;
-    }
-};
+__device__ __forceinline__ bool stage(const StageLoader<T, TM, TN, NT> &ld, Stage<T, TM, TN> &s, int buf,
+                                      const OrdParams &p, T alpha) {
+    bool odd = false;
+    auto put = [&](T v, int scale) {
+        if (scale) v = Ord<T>::mul(alpha, v);
+        odd = odd || !Ord<T>::plain(v);
+        return v;
+    };
+    ld.store(s, buf, p, [&](T v) { return put(v, p.scale_a); }, [&](T v) { return put(v, p.scale_b); });
+    return odd;
+}
 
 // Sum op(A)op(B) over k in [ks, ke) into t (a fresh chain, t starts at 0).
 template <typename T, int TM, int TN, int RM, int RN>
@@ -234,11 +195,11 @@ __device__ __forceinline__ void chain(const T *__restrict__ A, const T *__restri
 #pragma unroll
         for (int j = 0; j < RN; j++) t[i][j] = T(0);
     if (ks >= ke) return;
-    Loader<T, TM, TN, NT> ld;
+    StageLoader<T, TM, TN, NT> ld;
     ld.fetch(A, B, p, m0, n0, ks, ke);
     int buf = 0;
     // a chain's first buffer was last read before the previous chain's last barrier
-    bool odd = __syncthreads_or(ld.store(s, 0, p, alpha));
+    bool odd = __syncthreads_or(stage(ld, s, 0, p, alpha));
     for (int64_t k0 = ks; k0 < ke; k0 += BK, buf ^= 1) {
         const bool more = k0 + BK < ke;
         if (more) ld.fetch(A, B, p, m0, n0, k0 + BK, ke);
@@ -268,7 +229,7 @@ __device__ __forceinline__ void chain(const T *__restrict__ A, const T *__restri
                 fmac_step(m, t);
             }
         }
-        const bool next_odd = more && ld.store(s, buf ^ 1, p, alpha);
+        const bool next_odd = more && stage(ld, s, buf ^ 1, p, alpha);
         odd = __syncthreads_or(next_odd) || odd;
     }
 }

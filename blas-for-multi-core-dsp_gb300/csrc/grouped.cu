@@ -2,8 +2,11 @@
 //
 // A batch of GEMMs of uneven shapes, transpose modes, semantics and dtypes
 // (FP32 and FP64 mixed) is described by a device work list; a persistent
-// grid of CTAs pulls 64 x 64 C tiles from the whole list through one atomic
-// counter, so small problems that could not fill the GPU alone share it.
+// grid of CTAs pulls C tiles from the whole list through one atomic counter,
+// so small problems that could not fill the GPU alone share it.  FP64 tiles,
+// 16 x 16 or 32 x 32, come first, those of the longest K before the others:
+// the FP64 pipe (2 FMAs a clock and SM) bounds a mixed batch, and it is busy to
+// the end only if the last tiles are small.  FP32 tiles, 64 x 64, follow.
 // The reference runs one problem at a time per DSP cluster; this is the
 // GB300 batching layer of the serving path and has no reference counterpart.
 //
@@ -13,16 +16,19 @@
 // replayed for every batch that uses the slot.
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
 #include "gb_common.cuh"
 #include "gb_internal.h"
+#include "sm100_ptx.cuh"
+#include "tile_stage.cuh"
 
 namespace gb {
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16, NT = 256;
+constexpr int NT = 256, T32 = 64, PER_SM = 2;   // threads of a CTA; side of an FP32 tile; CTAs of an SM
 
 struct alignas(16) GItem {
     const void *A, *B;
@@ -30,61 +36,78 @@ struct alignas(16) GItem {
     int64_t M, N, K, lda, ldb, ldc;
     double alpha, beta;
     int32_t bits, ta, tb, semantics;
-    int32_t tiles_n, tile_base;
+    int32_t tiles_n, tile_base, tile;   // C tiles of side `tile`
 };
 
 struct alignas(16) GHeader {
     int32_t count, total_tiles, counter, pad;
 };
 
-template <typename T>
-__device__ void tile_gemm(const GItem &g, int tm, int tn, unsigned char *smem) {
-    T(*As)[TM + 1] = reinterpret_cast<T(*)[TM + 1]>(smem);
-    T(*Bs)[TN + 1] = reinterpret_cast<T(*)[TN + 1]>(smem + sizeof(T) * TK * (TM + 1));
+// One k of a thread's RM x RN outputs, FMAs in k order.
+template <int RM, int RN>
+__device__ __forceinline__ void fma_step(const double *As, const double *Bs, double (&acc)[RM][RN]) {
+    double a[RM], b[RN];
+#pragma unroll
+    for (int i = 0; i < RM; i++) a[i] = As[i];
+#pragma unroll
+    for (int j = 0; j < RN; j++) b[j] = Bs[j];
+#pragma unroll
+    for (int i = 0; i < RM; i++)
+#pragma unroll
+        for (int j = 0; j < RN; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+}
+// FP32: two outputs of a row in one packed FMA.
+__device__ __forceinline__ void fma_step(const float *As, const float *Bs, float (&acc)[4][4]) {
+    const float4 a = *reinterpret_cast<const float4 *>(As), b = *reinterpret_cast<const float4 *>(Bs);
+    const float av[4] = {a.x, a.y, a.z, a.w};
+    const uint64_t b01 = ptx::f2_pack(b.x, b.y), b23 = ptx::f2_pack(b.z, b.w);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint64_t a2 = ptx::f2_pack(av[i], av[i]);
+        ptx::f2_unpack(ptx::f2_fma_rn(a2, b01, ptx::f2_pack(acc[i][0], acc[i][1])), acc[i][0], acc[i][1]);
+        ptx::f2_unpack(ptx::f2_fma_rn(a2, b23, ptx::f2_pack(acc[i][2], acc[i][3])), acc[i][2], acc[i][3]);
+    }
+}
+
+template <typename T, int TILE>
+__device__ __forceinline__ void tile_gemm(const GItem &g, int tm, int tn, unsigned char *smem) {
+    constexpr int R = TILE / 16;   // 16 x 16 threads, R x R neighbouring outputs each
+    Stage<T, TILE, TILE> &s = *reinterpret_cast<Stage<T, TILE, TILE> *>(smem);
     const T *A = (const T *)g.A, *B = (const T *)g.B;
     T *C = (T *)g.C;
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    const int64_t m0 = (int64_t)tm * TM, n0 = (int64_t)tn * TN;
-    T acc[4][4];
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int64_t m0 = (int64_t)tm * TILE, n0 = (int64_t)tn * TILE;
+    T acc[R][R];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = T(0);
-    for (int64_t k0 = 0; k0 < g.K; k0 += TK) {
+        for (int j = 0; j < R; j++) acc[i][j] = T(0);
+    StageLoader<T, TILE, TILE, NT> ld;
+    const auto same = [](T v) { return v; };
+    if (g.K > 0) {
+        ld.fetch(A, B, g, m0, n0, 0, g.K);
+        ld.store(s, 0, g, same, same);
+    }
+    __syncthreads();
+    int buf = 0;
+    for (int64_t k0 = 0; k0 < g.K; k0 += STAGE_K, buf ^= 1) {
+        const bool more = k0 + STAGE_K < g.K;
+        if (more) ld.fetch(A, B, g, m0, n0, k0 + STAGE_K, g.K);
+        if (g.K - k0 >= STAGE_K) {
+#pragma unroll
+            for (int kk = 0; kk < STAGE_K; kk++) fma_step(&s.A[buf][kk][ty * R], &s.B[buf][kk][tx * R], acc);
+        } else {
+            for (int kk = 0; kk < (int)(g.K - k0); kk++)
+                fma_step(&s.A[buf][kk][ty * R], &s.B[buf][kk][tx * R], acc);
+        }
+        if (more) ld.store(s, buf ^ 1, g, same, same);
         __syncthreads();
-#pragma unroll
-        for (int r = 0; r < (TM * TK) / NT; r++) {
-            int l = tid + r * NT, mm, kk;
-            if (g.ta) { mm = l % TM; kk = l / TM; } else { mm = l / TK; kk = l % TK; }
-            int64_t m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < g.M && k < g.K) ? (g.ta ? A[k * g.lda + m] : A[m * g.lda + k]) : T(0);
-        }
-#pragma unroll
-        for (int r = 0; r < (TN * TK) / NT; r++) {
-            int l = tid + r * NT, nn, kk;
-            if (g.tb) { nn = l / TK; kk = l % TK; } else { nn = l % TN; kk = l / TN; }
-            int64_t n = n0 + nn, k = k0 + kk;
-            Bs[kk][nn] = (n < g.N && k < g.K) ? (g.tb ? B[n * g.ldb + k] : B[k * g.ldb + n]) : T(0);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; kk++) {
-            T a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int64_t m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+        for (int j = 0; j < R; j++) {
+            const int64_t m = m0 + ty * R + i, n = n0 + tx * R + j;
             if (m >= g.M || n >= g.N) continue;
             T *cp = C + m * g.ldc + n;
             T v = (T)g.alpha * acc[i][j];
@@ -99,8 +122,9 @@ __device__ void tile_gemm(const GItem &g, int tm, int tn, unsigned char *smem) {
         }
 }
 
-__global__ void __launch_bounds__(NT) grouped_gemm_kernel(GHeader *hdr, const GItem *items) {
-    __shared__ __align__(16) unsigned char smem[2 * sizeof(double) * TK * (TM + 1)];
+__global__ void __launch_bounds__(NT, PER_SM) grouped_gemm_kernel(GHeader *hdr, const GItem *items) {
+    __shared__ __align__(16) unsigned char smem[sizeof(Stage<double, 32, 32>)];
+    static_assert(sizeof(Stage<float, T32, T32>) <= sizeof(smem), "both tile types share the buffer");
     __shared__ int s_tile;
     const int count = hdr->count, total = hdr->total_tiles;
     for (;;) {
@@ -118,8 +142,9 @@ __global__ void __launch_bounds__(NT) grouped_gemm_kernel(GHeader *hdr, const GI
         const GItem g = items[lo];
         const int local = t - g.tile_base;
         const int tm = local / g.tiles_n, tn = local - tm * g.tiles_n;
-        if (g.bits == 64) tile_gemm<double>(g, tm, tn, smem);
-        else tile_gemm<float>(g, tm, tn, smem);
+        if (g.bits == 32) tile_gemm<float, T32>(g, tm, tn, smem);
+        else if (g.tile == 16) tile_gemm<double, 16>(g, tm, tn, smem);
+        else tile_gemm<double, 32>(g, tm, tn, smem);
     }
 }
 
@@ -179,27 +204,44 @@ struct GroupRunner {
         GB_CUDA_TRY(cudaEventSynchronize(s.done));   // previous batch in this slot finished reading it
         GHeader *h = reinterpret_cast<GHeader *>(s.host);
         GItem *it = reinterpret_cast<GItem *>(s.host + sizeof(GHeader));
-        int tiles = 0, count = 0;
+        // FP64 before FP32, long K first; FP64 in 16 x 16 tiles where 32 x 32 would leave an SM
+        // fewer than four.  Mixed batches, us (16 / 32): 1.6 tiles of 32 x 32 an SM 109 / 152, 2.0
+        // 104 / 116, 4.1 311 / 301, 5.6 281 / 265 (the FP64 pipe alone: 60, 36, 219, 201; 64 x 64
+        // tiles in the order given: 448, 367, 762, 615)
+        std::vector<int> order;
+        int64_t tiles32 = 0;
         for (int i = 0; i < n; i++) {
+            if (d[i].M == 0 || d[i].N == 0) continue;
+            order.push_back(i);
+            if (d[i].dtype_bits == 64) tiles32 += ceil_div(d[i].M, 32) * ceil_div(d[i].N, 32);
+        }
+        std::stable_sort(order.begin(), order.end(), [d](int x, int y) {
+            return d[x].dtype_bits != d[y].dtype_bits ? d[x].dtype_bits > d[y].dtype_bits : d[x].K > d[y].K;
+        });
+        const int side64 = tiles32 < 4 * (int64_t)sm_count() ? 16 : 32;
+        int64_t tiles = 0;
+        int count = 0;
+        for (int i : order) {
             const gb_gemm_desc &q = d[i];
-            if (q.M == 0 || q.N == 0) continue;
             GItem &g = it[count++];
             g.A = q.A; g.B = q.B; g.C = q.C;
             g.M = q.M; g.N = q.N; g.K = q.K; g.lda = q.lda; g.ldb = q.ldb; g.ldc = q.ldc;
             g.alpha = q.alpha; g.beta = q.beta;
             g.bits = q.dtype_bits; g.ta = is_trans(q.transA); g.tb = is_trans(q.transB); g.semantics = q.semantics;
-            g.tiles_n = (int)ceil_div(q.N, TN);
-            g.tile_base = tiles;
-            tiles += (int)(ceil_div(q.M, TM) * g.tiles_n);
+            g.tile = q.dtype_bits == 64 ? side64 : T32;
+            g.tiles_n = (int)ceil_div(q.N, g.tile);
+            g.tile_base = (int)tiles;
+            tiles += ceil_div(q.M, g.tile) * g.tiles_n;
+            if (tiles > 0x7fffffff) return set_status(GB_ERR_UNSUPPORTED, "gb_gemm_batch: too many tiles");
         }
         h->count = count;
-        h->total_tiles = tiles;
+        h->total_tiles = (int)tiles;
         h->counter = 0;
         h->pad = 0;
         if (count == 0) return ok();
-        const size_t bytes = sizeof(GHeader) + sizeof(GItem) * (size_t)max_items;
-        const int grid = 2 * sm_count();
-        if (use_graph) {
+        const int grid = PER_SM * sm_count();
+        if (use_graph) {   // the captured copy takes any batch: the whole list
+            const size_t bytes = sizeof(GHeader) + sizeof(GItem) * (size_t)max_items;
             if (!s.graph || s.graph_stream != stream) {
                 if (s.graph) cudaGraphExecDestroy(s.graph);
                 s.graph = nullptr;
@@ -222,7 +264,8 @@ struct GroupRunner {
             count_launch();
             GB_CUDA_TRY(cudaGraphLaunch(s.graph, stream));
         } else {
-            GB_CUDA_TRY(cudaMemcpyAsync(s.dev, s.host, bytes, cudaMemcpyHostToDevice, stream));
+            GB_CUDA_TRY(cudaMemcpyAsync(s.dev, s.host, sizeof(GHeader) + sizeof(GItem) * (size_t)count,
+                                        cudaMemcpyHostToDevice, stream));
             grouped_gemm_kernel<<<grid, NT, 0, stream>>>(reinterpret_cast<GHeader *>(s.dev),
                                                          reinterpret_cast<const GItem *>(s.dev + sizeof(GHeader)));
             GB_LAUNCH_CHECK("grouped_gemm_kernel");
@@ -250,7 +293,7 @@ gb_status check_desc(const gb_gemm_desc &q, int i) {
         GB_CHECK_ARG(q.C != nullptr, "gemm %d: C is null", i);
         if (q.K > 0) GB_CHECK_ARG(q.A && q.B, "gemm %d: A or B is null", i);
     }
-    GB_CHECK_ARG(ceil_div(q.M, TM) * ceil_div(q.N, TN) < (1ll << 30), "gemm %d: too many tiles", i);
+    GB_CHECK_ARG(ceil_div(q.M, 64) * ceil_div(q.N, 64) < (1ll << 30), "gemm %d: too many tiles", i);
     return ok();
 }
 

@@ -248,7 +248,7 @@ typedef struct gb_gemm_desc {
 
 /* Run n independent GEMMs of any shapes, modes, semantics and dtypes
  * (FP32 / FP64 mixed) in one launch of a persistent grouped kernel: the
- * descriptors become a device work list and every CTA pulls 64 x 64 C tiles
+ * descriptors become a device work list and every CTA pulls tiles of C
  * from the whole batch, so many small problems fill the GPU together.  No
  * reference counterpart (the reference runs one problem per DSP cluster);
  * it is the batching layer of the serving path.  n <= 4096.  Asynchronous
