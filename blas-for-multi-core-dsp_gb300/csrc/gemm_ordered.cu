@@ -41,6 +41,13 @@ struct Ord<double> {
     __device__ static double fmac(double a, double b, double t) { return __fma_rn(a, b, t); }
     __device__ static double add(double a, double b) { return __dadd_rn(a, b); }
     __device__ static double mul(double a, double b) { return __dmul_rn(a, b); }
+    // the same product, never computed ahead of the branch around it: an unused multiply of every
+    // staged value would take 4-6 % of the FP64 pipe
+    __device__ static double scaled(double a, double b) {
+        double v;
+        asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(v) : "d"(a), "d"(b));
+        return v;
+    }
     __device__ static bool plain(double) { return true; }
 };
 
@@ -52,6 +59,7 @@ struct Ord<float> {
     }
     __device__ static float add(float a, float b) { return __fadd_rn(a, b); }
     __device__ static float mul(float a, float b) { return __fmul_rn(a, b); }
+    __device__ static float scaled(float a, float b) { return mul(a, b); }
     // zero, or a magnitude in [2^-40, 2^45] (see fmac_step)
     __device__ static bool plain(float v) {
         const unsigned u = __float_as_uint(v) & 0x7fffffffu;
@@ -174,7 +182,7 @@ __device__ __forceinline__ bool stage(const StageLoader<T, TM, TN, NT> &ld, Stag
                                       const OrdParams &p, T alpha) {
     bool odd = false;
     auto put = [&](T v, int scale) {
-        if (scale) v = Ord<T>::mul(alpha, v);
+        if (scale) v = Ord<T>::scaled(alpha, v);
         odd = odd || !Ord<T>::plain(v);
         return v;
     };
@@ -366,13 +374,14 @@ gb_status launch(const GemmArgs &g) {
         return set_status(GB_ERR_UNSUPPORTED, "ordered gemm: M too large (%lld)", (long long)g.M);
     // The tiling of least estimated time; the constants are measured (a k of
     // FP32 64 x 64 / 32 x 64 / 32 x 32: 340 / 280 / 165 ns alone on an SM, 268 /
-    // 140 / 87 a tile when there are many; FP64 32 x 32 / 16 x 16: 310 / 190 and 268 /
-    // 72).  FP32 768 x 1000 x 1536: 703 us in 32 x 64, 796 in 32 x 32, 839 in
+    // 140 / 87 a tile when there are many; FP64 32 x 32 / 16 x 16: 310 / 120 and 256 /
+    // 78).  FP32 768 x 1000 x 1536: 703 us in 32 x 64, 796 in 32 x 32, 839 in
     // 64 x 64; 256^3: 75 / 43 / 92; 2048 x 2048 x 512: 1004 / 1182 / 961.  FP64 256^3:
-    // 81 us in 32 x 32, 55 in 16 x 16; 512^3: 287 / 310 (64 x 64: 283 and 554).
+    // 81 us in 32 x 32, 50 in 16 x 16; 128 x 200 x 300: 96 / 36; 512^3: 273 / 292 (64 x 64:
+    // 283, 328 and 554).
     if constexpr (sizeof(T) == 8) {
-        const double t32 = step_ns(g, 32, 32, 310, 268), t16 = step_ns(g, 16, 16, 190, 72, 60);
-        if (t16 < t32) return launch_tile<T, 16, 16, 2, 2>(g, p);
+        const double t32 = step_ns(g, 32, 32, 310, 256), t16 = step_ns(g, 16, 16, 120, 78, 40);
+        if (t16 < t32) return launch_tile<T, 16, 16, 1, 1>(g, p);
         return launch_tile<T, 32, 32, 2, 2>(g, p);
     } else {
         const double t64 = step_ns(g, 64, 64, 340, 268), t48 = step_ns(g, 32, 64, 280, 140, 40),
