@@ -481,22 +481,27 @@ __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ Spli
 // ------------------------------------------------------------------- gemm
 // Persistent: one CTA per SM walks the 128 x BN C tiles in a grouped order
 // (GROUP_M tile rows at a time, so neighbouring CTAs share A and B tiles in
-// L2).  K in blocks of 32 (one 64-byte swizzle atom), 4 shared-memory stages
-// holding NP 16-bit pieces of the A and B tiles (NP = 2: hi, lo with BN =
-// 256; NP = 3: hi, mid, lo with BN = 128).  Two TMEM accumulators: the
+// L2).  A shared-memory stage holds one k-block of the NP 16-bit pieces of
+// the A and B tiles (NP = 2: hi, lo with BN = 64, 128 or 256; NP = 3: hi, mid,
+// lo with BN = 128).  Two TMEM accumulators: the
 // epilogue of tile (or accumulator chunk) i overlaps the MMAs of i+1.
-constexpr int BM = 128, BK = 32, GROUP_M = 8;
-constexpr int A_TILE = BM * BK * 2;            // 8 KB
+// K-blocks are 32 (64-byte rows and swizzle) or 64 long (BK; 128 bytes): the
+// TMA unit takes a box row in about 1.5 clocks whether it has 64 or 128
+// bytes, so the longer rows load a narrow tile's operands faster (64 / 128
+// columns: 0.26 / 0.32 us per 32 k against 0.34 / 0.40), while 256 columns
+// have room for only two such stages (4096^3: 292 us against 270).
+constexpr int BM = 128, KB = 32, GROUP_M = 8;   // KB: the k-block that sizes and chunks are counted in
 constexpr int EPI_BYTES = 4 * 32 * 33 * 4;     // four warps' 32 x 32 staging, padded
 
 // EW epilogue warps: 4 (one per TMEM lane quarter, all BN columns) or 8 (two
 // per lane quarter, 128 columns each: the wide folding form); both stage C
 // through shared memory so that loads and stores of C are coalesced.
-template <int NP, int BN, int EW>
+template <int NP, int BN, int EW, int BK>
 struct TwoPass {
-    static constexpr int B_TILE = BN * BK * 2;
+    static_assert(BK == 32 || BK == 64, "64- or 128-byte swizzle atoms");
+    static constexpr int A_TILE = BM * BK * 2, B_TILE = BN * BK * 2;
     static constexpr int STAGE_BYTES = NP * A_TILE + NP * B_TILE;
-    static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;   // 4 (48 KB: two pieces, BN = 256; three, 128), 6, 8
+    static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;   // 2, 3 or 4
     static constexpr int NT = 64 + 32 * EW;
     // C staging: 4 warps x 32 x 32 (padded 33), or 8 warps x 32 x 16 (padded 17)
     static constexpr int EPI = EW == 4 ? EPI_BYTES : 8 * 32 * 17 * 4;
@@ -619,12 +624,13 @@ __device__ __forceinline__ void store_recomputed(const EpiParams &p, int64_t row
 //    16 columns at a time.
 // The MMAs of chunk c+1 overlap the fold of chunk c.
 // F16: FP16 pieces of scaled lines (FP16X3), the epilogue applies the scales.
-template <int NP, int BN, bool FOLD, bool F16, int EW>
+template <int NP, int BN, bool FOLD, bool F16, int EW, int BK>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
     bf16x3_gemm_kernel(const __grid_constant__ PieceMaps maps, EpiParams p) {
     // the next call's split pass may start beside this grid (it writes the other workspace half)
     if (threadIdx.x == 0) ptx::pdl_launch_dependents();
-    using CF = TwoPass<NP, BN, EW>;
+    using CF = TwoPass<NP, BN, EW, BK>;
+    constexpr int A_TILE = CF::A_TILE;
     constexpr bool SEP = FOLD && EW == 4;   // hi*hi apart from the cross products
     static_assert(!SEP || BN == 128, "the separated folding form keeps a 128-column total per thread");
     static_assert(EW == 4 || (FOLD && BN == 256), "eight epilogue warps: the wide folding form");
@@ -726,13 +732,14 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                         uint64_t ad[NP], bd[NP];
 #pragma unroll
                         for (int i = 0; i < NP; i++) {
-                            ad[i] = ptx::sdesc_kmajor_sw64(st + i * A_TILE);
-                            bd[i] = ptx::sdesc_kmajor_sw64(st + NP * A_TILE + i * B_TILE);
+                            const uint32_t a = st + i * A_TILE, b = st + NP * A_TILE + i * B_TILE;
+                            ad[i] = BK == 64 ? ptx::sdesc_kmajor_sw128(a) : ptx::sdesc_kmajor_sw64(a);
+                            bd[i] = BK == 64 ? ptx::sdesc_kmajor_sw128(b) : ptx::sdesc_kmajor_sw64(b);
                         }
                         const bool first = kb == kbc;
 #pragma unroll
                         for (int k = 0; k < BK / 16; k++) {
-                            // advance 16 values = 32 bytes along K inside the 64-byte swizzle atom
+                            // advance 16 values = 32 bytes along K inside the swizzle atom
                             const uint64_t dk = (uint64_t)((k * 32) >> 4);
                             // piece products (i, j) with i + j < NP, least significant first
 #pragma unroll
@@ -1454,11 +1461,11 @@ static void span(const void *p, bool trans, int64_t rows, int64_t cols, int64_t 
 }
 
 // bn: tile width; 128 with the 256-wide folding kernel runs every tile as two halves
-template <int NP, int BN, bool FOLD, bool F16, int EW>
+template <int NP, int BN, bool FOLD, bool F16, int EW, int BK>
 static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64_t kp, const EpiParams &base, int bn,
                                  bool dependent, int *grid_out) {
-    using CF = TwoPass<NP, BN, EW>;
-    auto kernel = bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW>;
+    using CF = TwoPass<NP, BN, EW, BK>;
+    auto kernel = bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW, BK>;
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
         GB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM_BYTES));
@@ -1485,7 +1492,7 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
     p.num_kb = (int)(kp / BK);
     p.tiles_m = tiles_m;
     p.tiles_n = tiles_n;
-    p.chunk_kb = FOLD ? (p.chunk_kb > 0 ? p.chunk_kb : p.num_kb) : 1;
+    p.chunk_kb = FOLD ? (p.chunk_kb > 0 ? p.chunk_kb * KB / BK : p.num_kb) : 1;
     p.half_start = half_start;
     cudaLaunchAttribute pdl;
     pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1503,50 +1510,62 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
     return ok();
 }
 
+// k of a pipeline stage: 64 for tiles (or halves) narrower than 256 columns,
+// where the accumulator chunk is whole in it.
+static int block_k(int np, bool fold, int fold_kb, int bn) {
+    return np == 2 && bn < 256 && (!fold || fold_kb % 2 == 0) ? 64 : 32;
+}
+
 template <bool F16>
 static gb_status gemm_launch(const GemmArgs &g, int np, int fold_kb, const PieceMaps &maps, int64_t kp,
                              const EpiParams &p, int bn, bool dependent, int *grid) {
     if constexpr (!F16) {   // three pieces are BF16 only
         if (np == 3)
-            return fold_kb > 0 ? two_pass_launch<3, 128, true, false, 4>(g, maps, kp, p, bn, dependent, grid)
-                               : two_pass_launch<3, 128, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
+            return fold_kb > 0 ? two_pass_launch<3, 128, true, false, 4, 32>(g, maps, kp, p, bn, dependent, grid)
+                               : two_pass_launch<3, 128, false, false, 4, 32>(g, maps, kp, p, bn, dependent, grid);
     }
+    const bool k64 = block_k(np, F16 || fold_kb > 0, fold_kb, bn) == 64;
     if constexpr (F16) {   // always the wide folding form (fold_kb 0: one chunk over all of K)
-        return two_pass_launch<2, 256, true, true, 8>(g, maps, kp, p, bn, dependent, grid);
+        return k64 ? two_pass_launch<2, 256, true, true, 8, 64>(g, maps, kp, p, bn, dependent, grid)
+                   : two_pass_launch<2, 256, true, true, 8, 32>(g, maps, kp, p, bn, dependent, grid);
     } else {
-        if (fold_kb > 0) return two_pass_launch<2, 256, true, false, 8>(g, maps, kp, p, bn, dependent, grid);
+        if (fold_kb > 0)
+            return k64 ? two_pass_launch<2, 256, true, false, 8, 64>(g, maps, kp, p, bn, dependent, grid)
+                       : two_pass_launch<2, 256, true, false, 8, 32>(g, maps, kp, p, bn, dependent, grid);
         switch (bn) {
-            case 64: return two_pass_launch<2, 64, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
-            case 128: return two_pass_launch<2, 128, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
-            default: return two_pass_launch<2, 256, false, false, 4>(g, maps, kp, p, bn, dependent, grid);
+            case 64: return two_pass_launch<2, 64, false, false, 4, 64>(g, maps, kp, p, bn, dependent, grid);
+            case 128: return two_pass_launch<2, 128, false, false, 4, 64>(g, maps, kp, p, bn, dependent, grid);
+            default: return two_pass_launch<2, 256, false, false, 4, 32>(g, maps, kp, p, bn, dependent, grid);
         }
     }
 }
 
 // Width of the C tiles.  256 columns need the least operand traffic per
-// product (48 KB a k-block of 32 in at least 0.66 us, against 0.40 for 128
-// and 0.34 for 64, which the L2 -> SM path bounds), narrow ones fill more SMs:
-// the width of least estimated time (waves of tiles x k-blocks, a tail wave
-// of 256 at most half full counted half, plus launch and epilogue).  Measured, us:
+// product, narrow ones fill more SMs: the width of least estimated time
+// (waves of tiles x k-blocks of 32 at 0.27 / 0.315 / 0.60 us for 64 / 128 /
+// 256 columns, a tail wave of 256 at most half full counted half, plus launch
+// and epilogue).  Measured, us:
 //
 //                     64      128     256
-//   513^3             13.5    17.4    27.4
-//   1111x937x1500     24.5    27.9    39.5
-//   1280^3            34.7    24.4    35.5
-//   2048^3            95.9    58.7    60.8
-//   3000^3            265     149     121
+//   513^3             12.0    15.9    27.1
+//   1111x937x1500     20.5    23.8    39.2
+//   1280^3            28.2    21.0    35.1
+//   2048^3            75.3    49.0    60.0
+//   2500^3            134     84.5    86.8
+//   4096^3            468     282     270
 //
 // The folding form has 256-wide tiles only; as halves (128) they pay while
-// all of them run at once with SMs to spare: 1024^3 26.0 against 32.0 us,
-// 1280^3 30.0 / 37.9, but 1500^3 (144 halves on 152 SMs) 49.6 / 47.0.
+// all of them run at once with SMs to spare: 1024^3 23.4 against 31.8 us,
+// 1280^3 26.6 / 37.7, 1500^3 (144 halves on 152 SMs) 45.2 / 46.4, 3000x700x1000
+// 38.8 / 37.9.
 static int tile_width(const GemmArgs &g, int np, bool fold) {
     if (np == 3) return 128;
-    const double sms = sm_count(), kb = (double)ceil_div(g.K, BK);
+    const double sms = sm_count(), kb = (double)ceil_div(g.K, KB);
     auto waves = [&](int bn) { return (double)ceil_div(g.M, BM) * (double)ceil_div(g.N, bn) / sms; };
-    if (fold) return 2.0 * waves(256) <= 0.8 ? 128 : 256;
+    if (fold) return 2.0 * waves(256) <= 0.9 ? 128 : 256;
     const double whole = floor(waves(256)), rest = waves(256) - whole;
-    const double t64 = 7.0 + ceil(waves(64)) * kb * 0.34, t128 = 8.0 + ceil(waves(128)) * kb * 0.40,
-                 t256 = 12.0 + (whole + (rest == 0.0 ? 0.0 : whole > 0.0 && rest <= 0.5 ? 0.5 : 1.0)) * kb * 0.66;
+    const double t64 = 7.0 + ceil(waves(64)) * kb * 0.27, t128 = 8.0 + ceil(waves(128)) * kb * 0.315,
+                 t256 = 12.0 + (whole + (rest == 0.0 ? 0.0 : whole > 0.0 && rest <= 0.5 ? 0.5 : 1.0)) * kb * 0.60;
     return t64 < t128 && t64 < t256 ? 64 : t128 < t256 ? 128 : 256;
 }
 
@@ -1555,7 +1574,7 @@ static int tile_width(const GemmArgs &g, int np, bool fold) {
 // f16: FP16 pieces of scaled lines (a max-exponent scan first).
 static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     if (f16 && np != 2) return set_status(GB_ERR_UNSUPPORTED, "fp16 pieces: two per value");
-    const int64_t kp = ceil_div(g.K, 64) * 64;   // multiple of BK, zero-padded
+    const int64_t kp = ceil_div(g.K, 64) * 64;   // a multiple of either k-block, zero-padded
     const size_t a_bytes = (size_t)g.M * kp * 2, b_bytes = (size_t)g.N * kp * 2;
     const size_t piece_bytes = (np * (a_bytes + b_bytes) + 255) / 256 * 256;
     const size_t pieces = piece_bytes;
@@ -1693,14 +1712,15 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     }
 
     const int bn = tile_width(g, np, fold_kb > 0 || f16);
+    const int bk = block_k(np, fold_kb > 0 || f16, fold_kb, bn);
     const int box = np == 2 && (fold_kb > 0 || f16) ? 256 : bn;   // rows of a B box (the halves have half boxes)
     PieceMaps maps;
     memset(&maps, 0, sizeof(maps));
     bool okm = true;
     for (int i = 0; i < np; i++) {   // 2-byte elements, copied as they are (BF16 or FP16)
-        okm = okm && make_tmap_bf16(&maps.a[i], ap[i], kp, g.M, kp * 2, BK, BM, 64);
-        okm = okm && make_tmap_bf16(&maps.b[i], bp[i], kp, g.N, kp * 2, BK, box, 64);
-        okm = okm && make_tmap_bf16(&maps.bh[i], bp[i], kp, g.N, kp * 2, BK, box / 2, 64);
+        okm = okm && make_tmap_bf16(&maps.a[i], ap[i], kp, g.M, kp * 2, bk, BM, 2 * bk);
+        okm = okm && make_tmap_bf16(&maps.b[i], bp[i], kp, g.N, kp * 2, bk, box, 2 * bk);
+        okm = okm && make_tmap_bf16(&maps.bh[i], bp[i], kp, g.N, kp * 2, bk, box / 2, 2 * bk);
     }
     if (!okm) return set_status(GB_ERR_CUDA, "bf16x3: cuTensorMapEncodeTiled failed");
     EpiParams p;
