@@ -109,6 +109,26 @@ __device__ __forceinline__ double mul_pow2(double x, int k) {
     return x * pow2_or_zero(a) * pow2_or_zero(b) * pow2_or_zero(c);
 }
 
+// The same product, by an addition to the exponent field where x and the
+// result are normal (the FP64 pipe serves 2 lanes a clock and SM; mul_pow2
+// takes three of its operations).
+__device__ __noinline__ inline double mul_pow2_cold(double x, int k) { return mul_pow2(x, k); }
+__device__ __forceinline__ double scale_pow2(double x, int k) {
+    const int hi = __double2hiint(x), E = (hi >> 20) & 0x7FF, F = E + k;
+    if (E > 0 && E < 0x7FF && F > 0 && F < 0x7FF) return __hiloint2double(hi + (k << 20), __double2loint(x));
+    return (hi & 0x7FFFFFFF) == 0 && __double2loint(x) == 0 ? x : mul_pow2_cold(x, k);
+}
+
+// n 2^k as a double (exact; |k| < 900), without the conversion instruction,
+// which takes the FP64 pipe like an addition.
+__device__ __forceinline__ double int_pow2(int n, int k) {
+    const unsigned a = n < 0 ? 0u - (unsigned)n : (unsigned)n;
+    const int z = __clz((int)a);
+    const unsigned m = (a << (z & 31)) << 1;   // the bits below the leading one, from the top
+    const int hi = (int)((((unsigned)(1023 + 31 - z + k)) << 20) | (m >> 12) | ((unsigned)n & 0x80000000u));
+    return a == 0 ? 0.0 : __hiloint2double(hi, (int)(m << 20));
+}
+
 // Plain FP64 dot product of row `row` of X (rows x K; tx: stored K x rows)
 // and column `col` of W (K x cols; tw: stored cols x K), in k order.  The
 // digit paths use it for the outputs whose row or column holds an Inf or a

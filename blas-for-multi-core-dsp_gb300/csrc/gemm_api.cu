@@ -179,14 +179,14 @@ size_t gemm_workspace_bound(int bits, int algo, bool ta, bool tb, int64_t M, int
             g.split_k = split_k;
             return skinny_workspace_bytes(g, bits);
         }
-        case GB_ALGO_OZAKI: {   // slices of both operands (K cut into chunks past 4 GiB) + exponents
+        case GB_ALGO_OZAKI: {   // slices of both operands (K cut into chunks past 4 GiB) + line maxima, exponents
             const int s = slices > 0 ? slices : ozaki_pick_slices(0.0, K);
             const int64_t kp = ceil_div(K, 64) * 64, mp = ceil_div(M, 128) * 128, np = ceil_div(N, 256) * 256;
             double v = (double)s * (double)(mp + np) * (double)kp * 2.0;
             const double cap = 4.0 * (1ull << 30) + (double)s * (mp + np) * 1024 * 2.0;
             if (v > cap) v = cap;
             // + the wide form's FP64 scratch: 256 KB per CTA
-            return (size_t)v + (size_t)(mp + np) * 4 + (size_t)sm_count() * (256 << 10) + 8192;
+            return (size_t)v + (size_t)(mp + np) * (4 + 8) + (size_t)sm_count() * (256 << 10) + 8192;
         }
         default:
             return 0;

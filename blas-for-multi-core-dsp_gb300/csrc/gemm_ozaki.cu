@@ -30,10 +30,13 @@
 // per SM over 128 x 128 C tiles, per tile a loop over slice pairs and K
 // chunks; warp 0 issues TMA (one digit tile of V_t and one of W_u per 64-wide
 // K block), warp 1 issues the MMAs into one of two FP32 accumulators
-// (alternating per chunk), warps 2-5 drain them into int32 registers and the
-// FP64 sum in TMEM, and write C.
+// (alternating per chunk), warps 2-9 drain them into int32 registers and the
+// FP64 sum in TMEM, and write C.  The FP64 pipe (2 lanes a clock and SM) gets one
+// addition an output and diagonal, and alpha and beta: conversions and
+// powers of two are made on the integer pipes.
 #include <cuda.h>
 #include <limits.h>
+#include <math.h>
 #include <cuda_bf16.h>
 
 #include "gb_common.cuh"
@@ -62,16 +65,15 @@ int ozaki_pick_slices(double target_err, int64_t K) {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 6, GROUP_M = 8;
+constexpr int BM = 128, BN = 128, BK = 64, STAGES = 7, GROUP_M = 8;
 constexpr int KCHUNK_BLOCKS = 16;              // 1024-long exact FP32 chunk
 constexpr int MAX_CHUNKS_INT32 = 127;          // chunk sums per int32 accumulator
 constexpr int MAXS = 9, MAXPAIRS = MAXS * (MAXS + 1) / 2;
 constexpr int TILE_BYTES = BM * BK * 2;        // 16 KB (BM == BN)
 constexpr int STAGE_BYTES = 2 * TILE_BYTES;
-constexpr int EPI_BYTES = 4 * 32 * 33 * 8;     // per-warp 32 x 32 FP64 staging
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 static_assert(SMEM_BYTES <= 232448, "shared memory");
-constexpr int NT = 192;
+constexpr int EWARPS = 8, NT = 64 + 32 * EWARPS;
 constexpr uint32_t TMEM_COLS = 512;            // [0,256): two FP32 accumulators, [256,512): FP64 sum
 
 // ------------------------------------------------------------- exponents
@@ -147,6 +149,72 @@ static void launch_maxexp_strided(const double *X, int64_t ld, int64_t cols, int
     exp_finish_kernel<<<nb, 256, 0, st>>>(e, cols);
 }
 
+// Largest |x| of every row of op(A) and column of op(B), as bits, by atomicMax
+// from blocks of 64 lines x 16 `steps` k, both operands in one launch (out
+// cleared before).  Element (r, k): trans ? X[k*ldx + r] : X[r*ldx + k].
+struct MaxOp {
+    const double *X;
+    int64_t ldx, rows, tiles_k, tiles;
+    int trans;
+    unsigned long long *out;
+};
+struct MaxArgs {
+    MaxOp op[2];
+    int64_t K;
+    int steps;
+};
+
+__global__ void __launch_bounds__(256) maxbits64_kernel(const __grid_constant__ MaxArgs a) {
+    __shared__ unsigned long long red[16][65];
+    int64_t b = blockIdx.x;
+    const int w = b < a.op[0].tiles ? 0 : 1;
+    if (w) b -= a.op[0].tiles;
+    const MaxOp &o = a.op[w];
+    const int64_t r0 = (b / o.tiles_k) * 64, kb0 = (b % o.tiles_k) * (16 * a.steps);
+    const int t = threadIdx.x, c4 = 4 * (t % 16), rl = t / 16;
+    const unsigned long long *X = reinterpret_cast<const unsigned long long *>(o.X);
+    auto top = [](unsigned long long m, unsigned long long v) {
+        v &= 0x7FFFFFFFFFFFFFFFull;
+        return v > m ? v : m;
+    };
+    unsigned long long m[4] = {0, 0, 0, 0};
+    if (!o.trans) {   // 16 threads (a half warp) per row, 16 rows apart
+#pragma unroll 4
+        for (int sb = 0; sb < a.steps; sb++) {
+            const int64_t k = kb0 + 16 * sb + t % 16;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int64_t r = r0 + rl + 16 * i;
+                if (r < o.rows && k < a.K) m[i] = top(m[i], __ldg(X + r * o.ldx + k));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+#pragma unroll
+            for (int s = 8; s >= 1; s >>= 1) m[i] = top(m[i], __shfl_xor_sync(0xffffffffu, m[i], s));
+            const int64_t r = r0 + rl + 16 * i;
+            if ((t & 15) == 0 && r < o.rows) atomicMax(o.out + r, m[i]);
+        }
+    } else {          // 4 consecutive rows, every 16th k
+#pragma unroll 4
+        for (int sb = 0; sb < a.steps; sb++) {
+            const int64_t k = kb0 + 16 * sb + rl, r = r0 + c4;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (k < a.K && r + q < o.rows) m[q] = top(m[q], __ldg(X + k * o.ldx + r + q));
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) red[rl][c4 + q] = m[q];
+        __syncthreads();
+        if (t < 64 && r0 + t < o.rows) {
+            unsigned long long mm = 0;
+#pragma unroll
+            for (int j = 0; j < 16; j++) mm = top(mm, red[j][t]);
+            atomicMax(o.out + r0 + t, mm);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- digits
 // s balanced base-256 digits of x (|x| < 2^e): N = +-round(|x| 2^(8s-1-e))
 // (to nearest: the representation error is half a unit of the last digit
@@ -185,33 +253,142 @@ __device__ __forceinline__ void digits(double x, int e, int s, unsigned short *o
     }
 }
 
-// out: s slices of rows_p x kp (K-major).  Source element (r, k):
-// trans ? X[k*ldx + r] : X[r*ldx + k]; padding rows / columns are zero.
-__global__ void __launch_bounds__(256) slice_kernel(const double *__restrict__ X, int64_t ldx, int trans, int64_t rows,
-                                                    int64_t K, int64_t rows_p, int64_t kp, const int *__restrict__ e,
-                                                    int s, unsigned short *__restrict__ out) {
-    __shared__ double tile[32][33];
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
-#pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-        double v = 0.0;
-        if (trans) {
-            int64_t k = k0 + ty + i, r = r0 + tx;
-            if (k < K && r < rows) v = X[k * ldx + r];
-            tile[ty + i][tx] = v;
-        } else {
-            int64_t r = r0 + ty + i, k = k0 + tx;
-            if (k < K && r < rows) v = X[r * ldx + k];
-            tile[tx][ty + i] = v;
-        }
+// The bytes of the digits of four values at once (s <= 8, the same digits as
+// above).  N' = N 2^(64-8s) has the digits of N above zeros; adding 128 to
+// every byte below the top one carries exactly as cutting the digits one by
+// one does, so byte i is digit i plus 128 and what is left above is the
+// leading digit.  |N'| <= 2^63: the sum is formed in two words.
+struct Digits8 {
+    uint32_t lo, hi;   // bytes 0-3, and 4-6: digit + 128
+    int top;           // [-128, 128]
+};
+
+__device__ __forceinline__ Digits8 digits8(double x, int e, int s) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int E = (int)((b >> 52) & 0x7FF);
+    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+    if (E) m |= 1ull << 52;
+    const int shift = (E ? E - 1075 : -1074) + 8 * s - 1 - e;
+    unsigned long long F = 0;
+    if (shift >= 0) F = m << (shift & 63);               // m 2^shift < 2^(8s-1); m == 0 whatever the shift
+    else if (shift > -64) F = (m + (1ull << (-shift - 1))) >> -shift;
+    F <<= 64 - 8 * s;
+    const bool neg = (long long)b < 0;
+    const unsigned long long U = neg ? 0ull - F : F;
+    const uint32_t lo = (uint32_t)U, hi = (uint32_t)(U >> 32);
+    Digits8 d;
+    d.lo = lo + 0x80808080u;
+    const long long h = (neg ? (long long)(int)hi : (long long)hi) + 0x00808080 + (d.lo < lo ? 1 : 0);
+    d.hi = (uint32_t)h;
+    d.top = (int)(h >> 24);
+    return d;
+}
+
+// byte `sel` of w, minus 128, as a float: 2^23 + byte, minus 2^23 + 128 (exact)
+__device__ __forceinline__ float digit_float(uint32_t w, int sel) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 | sel)) - 8388736.0f;
+}
+
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
+// s slices of an operand, rows_p x kp each (K-major, most significant first).
+// Source element (r, k): trans ? X[k*ldx + r] : X[r*ldx + k]; padding rows
+// and columns are zero.
+struct SliceOp {
+    const double *X;
+    int64_t ldx, rows, rows_p, tiles_k, tiles;
+    int trans;
+    const unsigned long long *maxbits;   // largest |x| of each line, as bits
+    int *e;                              // the lines' exponents, written here for the epilogue
+    unsigned short *out;
+};
+struct SliceArgs {
+    SliceOp op[2];
+    int64_t K, kp;
+    int s;
+};
+
+// four consecutive k of row r
+__device__ __forceinline__ void store_slices(const SliceArgs &a, const SliceOp &o, int64_t r, int64_t k,
+                                             const double (&v)[4]) {
+    const int e = r < o.rows ? exp_of_maxbits(o.maxbits[r]) : 0;
+    const int64_t stride = o.rows_p * a.kp;
+    unsigned short *out = o.out + r * a.kp + k;
+    if (a.s > 8) {
+        for (int j = 0; j < 4; j++) digits(v[j], e, a.s, out + j, stride);
+        return;
     }
-    __syncthreads();
-    const int64_t stride = rows_p * kp;
+    Digits8 d[4];
 #pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-        int64_t r = r0 + ty + i, k = k0 + tx;
-        if (r < rows_p && k < kp) digits(tile[tx][ty + i], r < rows ? e[r] : 0, s, out + r * kp + k, stride);
+    for (int j = 0; j < 4; j++) d[j] = digits8(v[j], e, a.s);
+    *reinterpret_cast<uint2 *>(out) =
+        make_uint2(bf16x2((float)d[0].top, (float)d[1].top), bf16x2((float)d[2].top, (float)d[3].top));
+#pragma unroll
+    for (int t = 1; t < 8; t++) {   // slice t + 1: digit 7 - t
+        if (t >= a.s) break;
+        const int i = 7 - t;
+        float f[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) f[j] = digit_float(i < 4 ? d[j].lo : d[j].hi, i & 3);
+        *reinterpret_cast<uint2 *>(out + t * stride) = make_uint2(bf16x2(f[0], f[1]), bf16x2(f[2], f[3]));
+    }
+}
+
+// Both operands in one launch; a CTA cuts a 64 x 64 block of (row, k), a thread
+// four consecutive k at a time (8-byte stores, 128 bytes of a slice row per
+// half warp).  Bound by HBM: 8 bytes read and 2 s written a value (two
+// operands of 8192^2, s = 8: 0.565 ms, 5.7 TB/s; cut one value a thread in
+// 128-bit integers: 1.80 ms).
+__global__ void __launch_bounds__(256) slice_kernel(const __grid_constant__ SliceArgs a) {
+    __shared__ double tile[32][65];
+    ptx::pdl_wait();   // the line maxima (returns at once when not launched as a dependent)
+    int64_t b = blockIdx.x;
+    const int w = b < a.op[0].tiles ? 0 : 1;
+    if (w) b -= a.op[0].tiles;
+    const SliceOp &o = a.op[w];
+    const int64_t r0 = (b / o.tiles_k) * 64, k0 = (b % o.tiles_k) * 64;
+    const int t = threadIdx.x, c4 = 4 * (t % 16), rl = t / 16;
+    if (k0 == 0 && t < 64 && r0 + t < o.rows_p) o.e[r0 + t] = r0 + t < o.rows ? exp_of_maxbits(o.maxbits[r0 + t]) : 0;
+    if (!o.trans) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t r = r0 + rl + 16 * i, k = k0 + c4;
+            if (r >= o.rows_p) continue;
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            if (r < o.rows) {
+                const double *src = o.X + r * o.ldx + k;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (k + j < a.K) v[j] = __ldg(src + j);
+            }
+            store_slices(a, o, r, k, v);
+        }
+        return;
+    }
+    // row-contiguous source: two halves of 32 k through tile[k][r]
+    const int kw = 4 * (t % 8), rw = t / 8;   // writer: four consecutive k of row rw (+ 32)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if (h) __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int kl = rl + 16 * i;
+            const int64_t k = k0 + 32 * h + kl, r = r0 + c4;
+            const double *src = o.X + k * o.ldx + r;
+#pragma unroll
+            for (int j = 0; j < 4; j++) tile[kl][c4 + j] = k < a.K && r + j < o.rows ? __ldg(src + j) : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int rr = rw + 32 * i;
+            if (r0 + rr >= o.rows_p) continue;
+            const double v[4] = {tile[kw][rr], tile[kw + 1][rr], tile[kw + 2][rr], tile[kw + 3][rr]};
+            store_slices(a, o, r0 + rr, k0 + 32 * h + kw, v);
+        }
     }
 }
 
@@ -222,6 +399,7 @@ struct OzParams {
     double alpha, beta;
     int semantics;
     int num_kb;                    // K blocks of 64
+    int chunk_kb;                  // K blocks summed in one accumulator, at most KCHUNK_BLOCKS
     int tiles_m, tiles_n;
     int64_t mp, np;                // padded rows of one V / W slice
     int npairs;
@@ -244,12 +422,42 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
     tn = r / gm;
 }
 
+// C = alpha 2^(e_i + f_j) sum (+ beta ...) for eight consecutive columns of a
+// row, their C loads in flight together.
+__device__ __forceinline__ void store_outputs(const OzParams &p, int64_t row, int64_t col0, int erow,
+                                              const double (&sum)[8]) {
+    const bool needc = p.semantics == GB_SEM_ACCUM_SCALAR_BETA || (p.semantics == GB_SEM_BLAS && p.beta != 0.0);
+    const bool rowok = row < p.M;
+    double *crow = p.C + row * p.ldc;
+    double cv[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) cv[j] = (rowok && needc && col0 + j < p.N) ? crow[col0 + j] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int64_t col = col0 + j;
+        if (!rowok || col >= p.N) continue;
+        const int fc = __ldg(p.fcol + col);
+        double v;
+        if (fc == kNonFiniteLineExp || erow == kNonFiniteLineExp)
+            v = p.alpha * native_dot_cold(p.A, p.lda, p.ta, row, p.B, p.ldb, p.tb, col, p.K);
+        else
+            v = p.alpha * scale_pow2(scale_pow2(sum[j], erow), fc);
+        if (p.semantics == GB_SEM_BLAS) {
+            if (p.beta != 0.0) v = fma(p.beta, cv[j], v);
+        } else if (p.semantics == GB_SEM_SCALAR_BETA) {
+            v = v + p.beta;
+        } else {
+            v = cv[j] + (v + p.beta);
+        }
+        crow[col] = v;
+    }
+}
+
 __global__ void __launch_bounds__(NT, 1)
     ozaki_gemm_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW, OzParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    double *epi = reinterpret_cast<double *>(smem + STAGES * STAGE_BYTES);
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES + EPI_BYTES);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
     uint64_t *empty = full + STAGES;
     uint64_t *acc_full = empty + STAGES;
     uint64_t *acc_empty = acc_full + 2;
@@ -257,7 +465,7 @@ __global__ void __launch_bounds__(NT, 1)
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int num_tiles = p.tiles_m * p.tiles_n;
-    const int nchunks = (p.num_kb + KCHUNK_BLOCKS - 1) / KCHUNK_BLOCKS;
+    const int nchunks = (p.num_kb + p.chunk_kb - 1) / p.chunk_kb;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -266,7 +474,7 @@ __global__ void __launch_bounds__(NT, 1)
         }
         for (int b = 0; b < 2; b++) {
             ptx::mbar_init(&acc_full[b], 1);
-            ptx::mbar_init(&acc_empty[b], 4);
+            ptx::mbar_init(&acc_empty[b], EWARPS);
         }
         ptx::fence_mbar_init();
         ptx::tma_prefetch_desc(&tmV);
@@ -277,6 +485,7 @@ __global__ void __launch_bounds__(NT, 1)
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    ptx::pdl_wait();   // the slices (and everything before them on the stream)
 
     if (warp == 0) {
         if (lane == 0) {   // TMA producer: per tile, per pair, every K block
@@ -317,8 +526,8 @@ __global__ void __launch_bounds__(NT, 1)
                         }
                         ptx::tc_fence_after();
                         const uint32_t acc = tmem + (uint32_t)(b * BN);
-                        const int kb_end = min(p.num_kb, (c + 1) * KCHUNK_BLOCKS);
-                        for (int kb = c * KCHUNK_BLOCKS; kb < kb_end; kb++, kbg++) {
+                        const int kb_end = min(p.num_kb, (c + 1) * p.chunk_kb);
+                        for (int kb = c * p.chunk_kb; kb < kb_end; kb++, kbg++) {
                             const int s = kbg % STAGES;
                             if (!ptx::mbar_wait(&full[s], (kbg / STAGES) & 1, p.err, 13)) {
                                 go = false;
@@ -331,7 +540,7 @@ __global__ void __launch_bounds__(NT, 1)
 #pragma unroll
                             for (int k = 0; k < BK / 16; k++) {
                                 const uint64_t dk = (uint64_t)((k * 32) >> 4);
-                                ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * KCHUNK_BLOCKS) || (k != 0));
+                                ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * p.chunk_kb) || (k != 0));
                             }
                             ptx::umma_commit(&empty[s]);
                         }
@@ -340,61 +549,59 @@ __global__ void __launch_bounds__(NT, 1)
                 }
             }
         }
-    } else {               // epilogue warps 2..5: TMEM lane quarter q = warp % 4
-        const int q = warp % 4;
-        double *stage = epi + q * 32 * 33;
+    } else {   // epilogue warps 2..9: TMEM lane quarter warp % 4, columns 64 * ((warp - 2) / 4) + 0..63
+        const int q = warp % 4, half = (warp - 2) / 4;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-        const uint32_t tot = tmem + 256u + lane_base;   // FP64 sum: element j at columns 2j, 2j+1
+        const uint32_t tot = tmem + 256u + lane_base + (uint32_t)(half * 128);   // FP64 sums: two columns each
         int gi = 0;
         bool go = true;
         for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
-            int tm, tn;
-            tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
             bool first_flush = true;
             // exact int32 sums of the chunk sums of consecutive pairs on one diagonal t + u (one
             // scale): one FP64 flush per diagonal, or after MAX_CHUNKS_INT32 chunk sums
-            int iacc[BN];
+            int iacc[64];
 #pragma unroll
-            for (int j = 0; j < BN; j++) iacc[j] = 0;
+            for (int j = 0; j < 64; j++) iacc[j] = 0;
             int nacc = 0;
             for (int qq = 0; qq < p.npairs && go; qq++) {
                 const int lev = p.pt[qq] + p.pu[qq];
                 const bool lev_ends = qq == p.npairs - 1 || p.pt[qq + 1] + p.pu[qq + 1] != lev;
-                const double scale = __longlong_as_double((long long)(1023 + 2 - 8 * lev) << 52);
                 for (int c = 0; c < nchunks; c++, gi++) {
                     const int b = gi & 1;
                     if (!ptx::mbar_wait(&acc_full[b], (gi >> 1) & 1, p.err, 14)) { go = false; break; }
                     ptx::tc_fence_after();
-#pragma unroll
-                    for (int cb = 0; cb < BN / 32; cb++) {
-                        uint32_t r[32];
-                        ptx::tmem_ld_32x32b_x32(tmem + (uint32_t)(b * BN) + lane_base + (uint32_t)(cb * 32), r);
-                        ptx::tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 32; j++) iacc[cb * 32 + j] += __float2int_rn(__uint_as_float(r[j]));
-                    }
+                    uint32_t r0[32], r1[32];
+                    const uint32_t acc = tmem + (uint32_t)(b * BN + half * 64) + lane_base;
+                    ptx::tmem_ld_32x32b_x32(acc, r0);
+                    ptx::tmem_ld_32x32b_x32(acc + 32u, r1);
+                    ptx::tmem_ld_wait();
                     ptx::tc_fence_before();
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(&acc_empty[b]);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        iacc[j] += __float2int_rn(__uint_as_float(r0[j]));
+                        iacc[32 + j] += __float2int_rn(__uint_as_float(r1[j]));
+                    }
                     const bool flush = (c == nchunks - 1 && lev_ends) || ++nacc == MAX_CHUNKS_INT32;
                     if (flush) {   // FP64 sum += 2^(2-8(t+u)) * iacc (exact scaling, one rounding)
                         nacc = 0;
 #pragma unroll
-                        for (int cb = 0; cb < (2 * BN) / 32; cb++) {
-                            uint32_t r[32];
+                        for (int cb = 0; cb < 8; cb++) {
+                            uint32_t r[16];
                             if (!first_flush) {
-                                ptx::tmem_ld_32x32b_x32(tot + (uint32_t)(cb * 32), r);
+                                ptx::tmem_ld_32x32b_x16(tot + (uint32_t)(cb * 16), r);
                                 ptx::tmem_ld_wait();
                             }
 #pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                double v = first_flush ? 0.0 : __hiloint2double((int)r[2 * j + 1], (int)r[2 * j]);
-                                v = fma((double)iacc[cb * 16 + j], scale, v);
+                            for (int j = 0; j < 8; j++) {
+                                double v = int_pow2(iacc[cb * 8 + j], 2 - 8 * lev);
+                                if (!first_flush) v = __dadd_rn(__hiloint2double((int)r[2 * j + 1], (int)r[2 * j]), v);
                                 r[2 * j] = (uint32_t)__double2loint(v);
                                 r[2 * j + 1] = (uint32_t)__double2hiint(v);
-                                iacc[cb * 16 + j] = 0;
+                                iacc[cb * 8 + j] = 0;
                             }
-                            ptx::tmem_st_32x32b_x32(tot + (uint32_t)(cb * 32), r);
+                            ptx::tmem_st_32x32b_x16(tot + (uint32_t)(cb * 16), r);
                         }
                         ptx::tmem_st_wait();
                         first_flush = false;
@@ -402,58 +609,21 @@ __global__ void __launch_bounds__(NT, 1)
                 }
             }
             if (!go) break;
-            // C = alpha * 2^(e_i + f_j) * sum (+ beta ...), staged for row-contiguous stores
-            const int64_t row0 = (int64_t)tm * BM + q * 32;
-            const int64_t n0 = (int64_t)tn * BN;
-            const int64_t myrow = row0 + lane;
-            const int erow = myrow < p.M ? p.erow[myrow] : 0;
-            for (int cb = 0; cb < BN / 32; cb++) {
+            // C = alpha * 2^(e_i + f_j) * sum (+ beta ...): this lane's row, 64 columns
+            int tm, tn;
+            tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+            const int64_t row = (int64_t)tm * BM + q * 32 + lane;
+            const int64_t c0 = (int64_t)tn * BN + half * 64;
+            const int erow = row < p.M ? p.erow[row] : 0;
+#pragma unroll 1
+            for (int cb = 0; cb < 8; cb++) {
+                uint32_t r[16];
+                ptx::tmem_ld_32x32b_x16(tot + (uint32_t)(cb * 16), r);
+                ptx::tmem_ld_wait();
+                double sum[8];
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    uint32_t r[32];
-                    ptx::tmem_ld_32x32b_x32(tot + (uint32_t)(cb * 64 + h * 32), r);
-                    ptx::tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        stage[lane * 33 + h * 16 + j] = mul_pow2(__hiloint2double((int)r[2 * j + 1], (int)r[2 * j]), erow);
-                }
-                __syncwarp();
-                const int64_t col = n0 + cb * 32 + lane;
-                if (col < p.N) {
-                    const int fc = p.fcol[col];
-                    const int rows = (p.M - row0) < 32 ? (int)(p.M - row0) : 32;
-                    const bool needc = p.semantics == GB_SEM_ACCUM_SCALAR_BETA ||
-                                       (p.semantics == GB_SEM_BLAS && p.beta != 0.0);
-                    for (int rb = 0; rb < rows; rb += 16) {   // sixteen rows' loads in flight at once
-                        double cv[16];
-                        int er[16];
-#pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const int rr = rb + j;
-                            er[j] = rr < rows ? __ldg(p.erow + row0 + rr) : 0;
-                            cv[j] = (rr < rows && needc) ? p.C[(row0 + rr) * p.ldc + col] : 0.0;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const int rr = rb + j;
-                            if (rr >= rows) break;
-                            double v;
-                            if (fc == kNonFiniteLineExp || er[j] == kNonFiniteLineExp)
-                                v = p.alpha * native_dot_cold(p.A, p.lda, p.ta, row0 + rr, p.B, p.ldb, p.tb, col, p.K);
-                            else
-                                v = p.alpha * mul_pow2(stage[rr * 33 + lane], fc);
-                            if (p.semantics == GB_SEM_BLAS) {
-                                if (p.beta != 0.0) v = fma(p.beta, cv[j], v);
-                            } else if (p.semantics == GB_SEM_SCALAR_BETA) {
-                                v = v + p.beta;
-                            } else {
-                                v = cv[j] + (v + p.beta);
-                            }
-                            p.C[(row0 + rr) * p.ldc + col] = v;
-                        }
-                    }
-                }
-                __syncwarp();
+                for (int j = 0; j < 8; j++) sum[j] = __hiloint2double((int)r[2 * j + 1], (int)r[2 * j]);
+                store_outputs(p, row, c0 + cb * 8, erow, sum);
             }
             ptx::tc_fence_before();
         }
@@ -501,7 +671,7 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int num_tiles = p.tiles_m * p.tiles_n;
-    const int nchunks = (p.num_kb + KCHUNK_BLOCKS - 1) / KCHUNK_BLOCKS;
+    const int nchunks = (p.num_kb + p.chunk_kb - 1) / p.chunk_kb;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES_W; s++) {
@@ -521,6 +691,7 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    ptx::pdl_wait();   // the slices (and everything before them on the stream)
 
     if (warp == 0) {
         if (lane == 0) {   // TMA producer: per tile, per pair, every K block
@@ -561,8 +732,8 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
                         }
                         ptx::tc_fence_after();
                         const uint32_t acc = tmem + (uint32_t)(b * BN_W);
-                        const int kb_end = min(p.num_kb, (c + 1) * KCHUNK_BLOCKS);
-                        for (int kb = c * KCHUNK_BLOCKS; kb < kb_end; kb++, kbg++) {
+                        const int kb_end = min(p.num_kb, (c + 1) * p.chunk_kb);
+                        for (int kb = c * p.chunk_kb; kb < kb_end; kb++, kbg++) {
                             const int s = kbg % STAGES_W;
                             if (!ptx::mbar_wait(&full[s], (kbg / STAGES_W) & 1, p.err, 13)) {
                                 go = false;
@@ -575,7 +746,7 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
 #pragma unroll
                             for (int k = 0; k < BK / 16; k++) {
                                 const uint64_t dk = (uint64_t)((k * 32) >> 4);
-                                ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * KCHUNK_BLOCKS) || (k != 0));
+                                ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * p.chunk_kb) || (k != 0));
                             }
                             ptx::umma_commit(&empty[s]);
                         }
@@ -619,13 +790,12 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
                     const bool flush = (c == nchunks - 1 && lev_ends) || ++nacc == MAX_CHUNKS_INT32;
                     if (flush) {   // FP64 sum += 2^(2-8(t+u)) * iacc (exact scaling, one rounding)
                         nacc = 0;
-                        const double scale = __longlong_as_double((long long)(1023 + 2 - 8 * lev) << 52);
                         double2 *scr = OZ_SCR;
                         if (first_flush) {
 #pragma unroll
                             for (int jp = 0; jp < 64; jp++)
-                                scr[jp * 32] = make_double2(fma((double)iacc[2 * jp], scale, 0.0),
-                                                            fma((double)iacc[2 * jp + 1], scale, 0.0));
+                                scr[jp * 32] = make_double2(int_pow2(iacc[2 * jp], 2 - 8 * lev),
+                                                            int_pow2(iacc[2 * jp + 1], 2 - 8 * lev));
                         } else {
 #pragma unroll
                             for (int g8 = 0; g8 < 64; g8 += 4) {   // four pairs' loads in flight
@@ -634,8 +804,8 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
                                 for (int i = 0; i < 4; i++) v[i] = __ldcg(scr + (g8 + i) * 32);
 #pragma unroll
                                 for (int i = 0; i < 4; i++) {
-                                    v[i].x = fma((double)iacc[2 * (g8 + i)], scale, v[i].x);
-                                    v[i].y = fma((double)iacc[2 * (g8 + i) + 1], scale, v[i].y);
+                                    v[i].x = __dadd_rn(v[i].x, int_pow2(iacc[2 * (g8 + i)], 2 - 8 * lev));
+                                    v[i].y = __dadd_rn(v[i].y, int_pow2(iacc[2 * (g8 + i) + 1], 2 - 8 * lev));
                                     __stcg(scr + (g8 + i) * 32, v[i]);
                                 }
                             }
@@ -652,42 +822,15 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
             tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
             const int64_t row = (int64_t)tm * BM + q * 32 + lane;
             const int64_t c0 = (int64_t)tn * BN_W + (w / 4) * 128;
-            const bool rowok = row < p.M;
-            const int erow = rowok ? p.erow[row] : 0;
-            const bool needc = p.semantics == GB_SEM_ACCUM_SCALAR_BETA || (p.semantics == GB_SEM_BLAS && p.beta != 0.0);
-            double *crow = p.C + row * p.ldc;
+            const int erow = row < p.M ? p.erow[row] : 0;
             const double2 *scr = OZ_SCR;
 #pragma unroll 1
-            for (int g8 = 0; g8 < 64; g8 += 4) {   // eight columns at a time, their C loads in flight together
+            for (int g8 = 0; g8 < 64; g8 += 4) {
                 double2 sm[4];
-                double cv[8];
 #pragma unroll
                 for (int i = 0; i < 4; i++) sm[i] = __ldcg(scr + (g8 + i) * 32);
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int64_t col = c0 + 2 * g8 + j;
-                    cv[j] = (rowok && needc && col < p.N) ? crow[col] : 0.0;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int64_t col = c0 + 2 * g8 + j;
-                    if (!rowok || col >= p.N) continue;
-                    const int fc = __ldg(p.fcol + col);
-                    const double sum = (j & 1) ? sm[j / 2].y : sm[j / 2].x;
-                    double v;
-                    if (fc == kNonFiniteLineExp || erow == kNonFiniteLineExp)
-                        v = p.alpha * native_dot_cold(p.A, p.lda, p.ta, row, p.B, p.ldb, p.tb, col, p.K);
-                    else
-                        v = p.alpha * mul_pow2(mul_pow2(sum, erow), fc);
-                    if (p.semantics == GB_SEM_BLAS) {
-                        if (p.beta != 0.0) v = fma(p.beta, cv[j], v);
-                    } else if (p.semantics == GB_SEM_SCALAR_BETA) {
-                        v = v + p.beta;
-                    } else {
-                        v = cv[j] + (v + p.beta);
-                    }
-                    crow[col] = v;
-                }
+                const double sum[8] = {sm[0].x, sm[0].y, sm[1].x, sm[1].y, sm[2].x, sm[2].y, sm[3].x, sm[3].y};
+                store_outputs(p, row, c0 + 2 * g8, erow, sum);
             }
         }
     }
@@ -748,9 +891,11 @@ gb_status launch_dgemm_ozaki(const GemmArgs &g, int slices) {
 }
 
 static gb_status ozaki_one(const GemmArgs &g, int s) {
-    // the wide form (128 x 256 tiles) once op(B) has 256 columns; GB_OZAKI_WIDE=0 keeps 128 x 128
+    // The wide form (128 x 256 tiles) once op(B) has 256 columns, unless 128 x 128 tiles take less time
+    // (waves of tiles, a k-block at 0.39 against 0.27 us); GB_OZAKI_WIDE=0 keeps 128 x 128
     const char *wv = getenv("GB_OZAKI_WIDE");
-    const bool wide = !(wv && wv[0] == '0') && g.N >= wide::BN_W;
+    auto waves = [&](int width) { return ceil((double)ceil_div(g.M, BM) * (double)ceil_div(g.N, width) / sm_count()); };
+    const bool wide = !(wv && wv[0] == '0') && g.N >= wide::BN_W && 0.39 * waves(wide::BN_W) <= 0.27 * waves(BN);
     const int bn = wide ? wide::BN_W : BN;
     const int64_t kp = ceil_div(g.K, BK) * BK;
     const int64_t mp = ceil_div(g.M, BM) * BM, np = ceil_div(g.N, bn) * bn;
@@ -761,39 +906,57 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     const int64_t tiles_total = (mp / BM) * (np / bn);
     const int grid = (int)(tiles_total < sm_count() ? tiles_total : sm_count());
     const size_t sbytes = wide ? (size_t)grid * wide::SCRATCH_DOUBLES * sizeof(double) : 0;
-    uint8_t *ws = (uint8_t *)workspace(vbytes + wbytes + ebytes + sbytes + 4096, g.stream);
+    const size_t mbytes = (size_t)(mp + np) * sizeof(unsigned long long);
+    uint8_t *ws = (uint8_t *)workspace(vbytes + wbytes + ebytes + sbytes + mbytes + 4096, g.stream);
     if (!ws) return (gb_status)gb_get_last_status();
     unsigned short *V = (unsigned short *)ws;
     unsigned short *W = (unsigned short *)(ws + vbytes);
     int *erow = (int *)(ws + vbytes + wbytes);
     int *fcol = erow + mp;
+    unsigned long long *maxbits = (unsigned long long *)(ws + vbytes + wbytes + ebytes + sbytes);
     double *scratch = wide ? (double *)(ws + vbytes + wbytes + ebytes) : nullptr;   // 256-byte aligned
     int *err = error_word();
     if (!err) return set_status(GB_ERR_OOM, "ozaki: no device error word");
 
-    // exponents: rows of op(A), columns of op(B)
+    // line maxima: rows of op(A), columns of op(B)
     const double *A = (const double *)g.A, *B = (const double *)g.B;
-    if (!g.ta) {
-        maxexp_contig_kernel<<<(unsigned)ceil_div(g.M, 8), 256, 0, g.stream>>>(A, g.lda, g.M, g.K, erow);
-    } else {
-        launch_maxexp_strided(A, g.lda, g.M, g.K, erow, g.stream);
-    }
-    GB_LAUNCH_CHECK("ozaki exponents A");
-    if (g.tb) {
-        maxexp_contig_kernel<<<(unsigned)ceil_div(g.N, 8), 256, 0, g.stream>>>(B, g.ldb, g.N, g.K, fcol);
-    } else {
-        launch_maxexp_strided(B, g.ldb, g.N, g.K, fcol, g.stream);
-    }
-    GB_LAUNCH_CHECK("ozaki exponents B");
-
+    GB_CUDA_TRY(cudaMemsetAsync(maxbits, 0, (size_t)(mp + np) * sizeof(unsigned long long), g.stream));
+    // blocks of 256 k, or of 64 while those would leave an SM fewer than eight
+    const int steps = (ceil_div(g.M, 64) + ceil_div(g.N, 64)) * ceil_div(g.K, 256) < 8 * sm_count() ? 4 : 16;
+    const int64_t mk = ceil_div(g.K, 16 * steps), sk = kp / 64;
+    if (ceil_div(mp, 32) > 65535 || ceil_div(np, 32) > 65535)
+        return set_status(GB_ERR_UNSUPPORTED, "ozaki: M or N too large");
+    MaxArgs ma;
+    ma.K = g.K;
+    ma.steps = steps;
+    ma.op[0] = MaxOp{A, g.lda, g.M, mk, ceil_div(g.M, 64) * mk, g.ta ? 1 : 0, maxbits};
+    ma.op[1] = MaxOp{B, g.ldb, g.N, mk, ceil_div(g.N, 64) * mk, g.tb ? 0 : 1, maxbits + mp};
+    const int64_t mblocks = ma.op[0].tiles + ma.op[1].tiles;
     // digits: V_t = digits of op(A) rows (M x K), W_u = digits of op(B)^T rows (N x K)
-    dim3 gA((unsigned)ceil_div(kp, 32), (unsigned)ceil_div(mp, 32));
-    dim3 gB((unsigned)ceil_div(kp, 32), (unsigned)ceil_div(np, 32));
-    if (gA.y > 65535u || gB.y > 65535u) return set_status(GB_ERR_UNSUPPORTED, "ozaki: M or N too large");
-    slice_kernel<<<gA, 256, 0, g.stream>>>(A, g.lda, g.ta ? 1 : 0, g.M, g.K, mp, kp, erow, s, V);
-    GB_LAUNCH_CHECK("ozaki slices A");
-    slice_kernel<<<gB, 256, 0, g.stream>>>(B, g.ldb, g.tb ? 0 : 1, g.N, g.K, np, kp, fcol, s, W);
-    GB_LAUNCH_CHECK("ozaki slices B");
+    SliceArgs sa;
+    sa.K = g.K; sa.kp = kp; sa.s = s;
+    sa.op[0] = SliceOp{A, g.lda, g.M, mp, sk, ceil_div(mp, 64) * sk, g.ta ? 1 : 0, maxbits, erow, V};
+    sa.op[1] = SliceOp{B, g.ldb, g.N, np, sk, ceil_div(np, 64) * sk, g.tb ? 0 : 1, maxbits + mp, fcol, W};
+    const int64_t sblocks = sa.op[0].tiles + sa.op[1].tiles;
+    if (mblocks > 0x7fffffff || sblocks > 0x7fffffff)
+        return set_status(GB_ERR_UNSUPPORTED, "ozaki: operands too large");
+    maxbits64_kernel<<<(unsigned)mblocks, 256, 0, g.stream>>>(ma);
+    GB_LAUNCH_CHECK("ozaki line maxima");
+    // the slices and the GEMM are launched as programmatic dependents of the kernel before: their
+    // launch and set-up overlap it (captured launches keep plain stream order)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GB_CUDA_TRY(cudaStreamIsCapturing(g.stream, &cap));
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)sblocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = g.stream;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+    GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, slice_kernel, sa));
+    GB_LAUNCH_CHECK("ozaki slices");
 
     CUtensorMap tV, tW;
     if (!make_tmap_bf16(&tV, V, kp, (uint64_t)s * mp, kp * 2, BK, BM, 128) ||
@@ -804,6 +967,8 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     p.C = (double *)g.C; p.M = g.M; p.N = g.N; p.ldc = g.ldc;
     p.alpha = g.alpha; p.beta = g.beta; p.semantics = g.semantics;
     p.num_kb = (int)(kp / BK);
+    // even chunks: the accumulator of a short last one would be drained slower than it fills
+    p.chunk_kb = (int)ceil_div(p.num_kb, ceil_div(p.num_kb, KCHUNK_BLOCKS));
     p.tiles_m = (int)(mp / BM); p.tiles_n = (int)(np / bn);
     p.mp = mp; p.np = np;
     p.erow = erow; p.fcol = fcol; p.err = err;
@@ -835,11 +1000,16 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
         GB_CUDA_TRY(cudaFuncSetAttribute(ozaki_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_W));
         device_setup_done(attr);
     }
+    cfg.gridDim = dim3((unsigned)grid);
     if (wide) {
-        ozaki_wide_kernel<<<grid, wide::NT_W, wide::SMEM_W, g.stream>>>(tV, tW, p, scratch);
+        cfg.blockDim = dim3(wide::NT_W);
+        cfg.dynamicSmemBytes = wide::SMEM_W;
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, ozaki_wide_kernel, tV, tW, p, scratch));
         GB_LAUNCH_CHECK("ozaki_wide_kernel");
     } else {
-        ozaki_gemm_kernel<<<grid, NT, SMEM_BYTES, g.stream>>>(tV, tW, p);
+        cfg.blockDim = dim3(NT);
+        cfg.dynamicSmemBytes = SMEM_BYTES;
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, ozaki_gemm_kernel, tV, tW, p));
         GB_LAUNCH_CHECK("ozaki_gemm_kernel");
     }
     return ok();
