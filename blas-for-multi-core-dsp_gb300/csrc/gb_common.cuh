@@ -209,7 +209,9 @@ struct ThinTcArgs {
     float alpha, beta;
     int semantics;
     int splits; int64_t kchunk;                    // K range of a split: a multiple of 64
-    float *part;                                   // splits x rows x nb partials (splits > 1)
+    int fold;                                      // stages of 64 k summed in one accumulator
+    int parts;                                     // > 0 (splits == 1): CTAs of equal parts
+    float *part;                                   // splits x rows x nb, or 2 parts x 128 x nb partials
     void *wpieces;                                 // thin_tc_wpieces_bytes(nb, K) of scratch
     cudaStream_t stream;
 };

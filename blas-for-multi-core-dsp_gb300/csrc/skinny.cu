@@ -23,6 +23,8 @@
 //    and read by broadcast.
 // Split-K over CTAs when the row count alone cannot fill the GPU; partial
 // sums go to scratch and a second kernel applies alpha/beta.
+#include <math.h>
+
 #include "gb_common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -572,6 +574,8 @@ struct Plan {
     bool tma;                 // FP32 n <= 8 with TMA-compatible layouts: thin::thin_tma_kernel
     bool tc;                  // FP32 8 < n <= 64, K >= 64: 3xBF16 on the tensor cores (skinny_tc.cu)
     int64_t rtiles;
+    int fold;                 // tc: stages summed in one accumulator
+    int parts;                // tc: CTAs that share all stages equally (0: a fixed split of each tile)
     size_t part_bytes;
     size_t w_bytes;           // scratch for the BF16 pieces of W (tc)
 };
@@ -609,26 +613,53 @@ bool tc_eligible(const SkParams &p) {
     return p.rows < (int64_t(1) << 31) && p.K < (int64_t(1) << 30) && (uintptr_t)p.X % 16 == 0;
 }
 
+// K ranges per tile: units for four waves and more (one range when there are as
+// many tiles), up to twice as many where that leaves the last wave fuller; at
+// least eight stages a range.
+inline int balanced_splits(int64_t tiles, int64_t nst) {
+    const double sms = sm_count();
+    int best = 1;
+    double best_fill = 0.0;
+    for (int s = 1; s <= 64 && (s == 1 || nst / s >= 8); s++) {
+        const double units = (double)(tiles * s), fill = units / (ceil(units / sms) * sms);
+        if (units >= 8.0 * sms && s > 1 && best_fill > 0.0) break;
+        if (units < 4.0 * sms || fill > best_fill + 0.02) {
+            best = s;
+            best_fill = units < 4.0 * sms ? 0.0 : fill;
+        }
+        if (tiles >= 4 * (int64_t)sms) break;
+    }
+    return best;
+}
+
 template <typename T, int NB>
 gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
     pl.w_bytes = 0;
+    pl.parts = 0;
     pl.tc = allow_tc && tc_eligible<T, NB>(p);
     if (pl.tc) {
-        // units of 128 rows (per row class) x a K range; split K until there are ~4 units per SM
+        // tiles of 128 rows (per row class) x stages of 64 k: row-major X in equal parts over the SMs;
+        // K-major X, and where the caller asks for it, in a number of K ranges per tile
         const bool classes = thin_tc_row_classes(p.tx, p.ldx);
         pl.tma = false;
         pl.rows_kernel = !p.tx;
         pl.vec = pl.wvec = true;
         pl.rtiles = ceil_div(p.rows, 128) + (classes ? 3 : 0);
         const int64_t nst = thin_tc_stages(p.K, classes);
-        int splits = 1;
-        while (pl.rtiles * splits < 4 * (int64_t)sm_count() && nst / (splits * 2) >= 8 && splits < 64) splits *= 2;
-        if (p.want_splits > 0) splits = p.want_splits;
-        const int64_t cst = ceil_div(nst, splits);
+        const int64_t sms = sm_count();
+        const bool equal = p.want_splits <= 0 && !p.tx && pl.rtiles < 4 * sms && pl.rtiles * nst >= 16 * sms;
+        const int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst);
+        const int64_t cst = ceil_div(nst, want);
         p.kchunk = cst * 64;
         p.splits = (int)ceil_div(nst, cst);
         if (p.splits < 1) p.splits = 1;
-        pl.part_bytes = p.splits > 1 ? (size_t)p.splits * p.rows * NB * sizeof(T) : 0;
+        pl.parts = equal ? (int)sms : 0;
+        // sums of at most the K range that a split into four waves of units would leave
+        int64_t ranges = 1;
+        while (pl.rtiles * ranges < 4 * (int64_t)sm_count() && nst / (ranges * 2) >= 8 && ranges < 64) ranges *= 2;
+        pl.fold = (int)ceil_div(nst, ranges);
+        pl.part_bytes = pl.parts > 0 ? (size_t)2 * pl.parts * 128 * NB * sizeof(T)
+                        : p.splits > 1 ? (size_t)p.splits * p.rows * NB * sizeof(T) : 0;
         pl.w_bytes = thin_tc_wpieces_bytes(NB, p.K, classes);
         return ok();
     }
@@ -714,7 +745,7 @@ gb_status launch_plan(const SkParams &p, const Plan &pl, cudaStream_t st) {
     if (pl.tc) {
         ThinTcArgs a{p.rows, p.K, (const float *)p.X, p.ldx, p.tx, (const float *)p.W, p.ldw, p.tw, p.n, NB,
                      (float *)p.C, p.cs_r, p.cs_c, (float)p.alpha, (float)p.beta, p.semantics, p.splits, p.kchunk,
-                     (float *)p.part, p.wpieces, st};
+                     pl.fold, pl.parts, (float *)p.part, p.wpieces, st};
         gb_status s = launch_thin_tc(a);
         if (s != GB_OK) return s;
         if (p.splits > 1) {

@@ -18,7 +18,20 @@
 //   * warp 1 issues tcgen05.mma (M = 128, N = NB, K = 16, A from TMEM, B from
 //     shared memory) into one of two TMEM accumulators of NB columns;
 //   * warps 6-9 read the finished accumulator (tcgen05.ld) and apply
-//     alpha / beta, or write split-K partials for skinny_reduce_kernel.
+//     alpha / beta, or write partial sums.
+// Work split of row-major X: the CTAs take whole tiles in turn while more than
+// two are left for each; the stages of the remaining tiles form one sequence,
+// of which every CTA takes an equal part: no tail wave, and at most two
+// partial tiles a CTA, which thin_tc_join_kernel adds up (a fixed split of every
+// tile's K leaves the last wave part empty and writes every tile `splits`
+// times: 20011 x 6007, n = 33: 126 us against 108).  With four tiles an SM and
+// more the tail costs nothing (HBM bound; 262144 x 4096: 678 us against 682 in
+// equal parts), with fewer than sixteen stages an SM the join costs more than
+// it gives (2000 x 1500, n = 40: 20.6 against 21.8): fixed split.  K-major X keeps a fixed split, summed by skinny_reduce_kernel, and
+// takes the tiles of one K range before the next, so that the CTAs at work read
+// neighbouring pieces of the same k lines (11499 rows, K = 48841: 499 us in equal
+// parts, 404 with the ranges of a tile one after the other, 367 so).  So does
+// a requested split count (gb_gemm_opts.split_k).
 // Shared-memory traffic per X value is the TMA write and one read (8 bytes).
 //
 // Row-major X whose leading dimension is not a multiple of 4 floats cannot be
@@ -66,10 +79,17 @@ struct TcParams {
     int64_t rows, K;
     int n, splits, kchunk_st;             // stages of 64 k per split
     int nst;                              // stages covering K (+ the largest phase)
+    // Stages summed in one tensor-memory accumulator; the epilogue warps add the sums in FP32
+    // registers.  The tensor cores' FP32 additions err like a truncation, so the error grows with
+    // the length of a sum (K = 6007: 1.5e-5 in one accumulator, 6.1e-6 in four).
+    int fold;
     int rstride;                          // 4 with row classes, else 1
     int64_t cls_rows[4];                  // rows in class c
     int cls_delta[4];
-    int cls_u0[5];                        // first unit of class c
+    int cls_u0[5];                        // first unit (row tile x split) of class c
+    int64_t stages;                       // equal parts of the stages of the tiles from `whole` on (splits == 1)
+    int whole;                            // tiles taken whole, in turn
+    int tile_first;                       // K-major X: row tiles (units run over the tiles of a K range first); else 0
     int kdelta[4];                        // K-major X in k-line classes: phase of class c
     float *C; int64_t cs_r, cs_c;
     float alpha, beta;
@@ -91,13 +111,67 @@ __device__ __forceinline__ void unit_coords(const TcParams &p, int u, int &c, in
     c = 0;
     while (c < 3 && u >= p.cls_u0[c + 1]) c++;
     const int v = u - p.cls_u0[c];
-    rt = v / p.splits;
-    sp = v - rt * p.splits;
+    if (p.tile_first) {   // neighbouring units: neighbouring tiles of the same K range
+        sp = v / p.tile_first;
+        rt = v - sp * p.tile_first;
+    } else {
+        rt = v / p.splits;
+        sp = v - rt * p.splits;
+    }
+}
+
+// first stage of CTA b's part of the sequence
+__device__ __forceinline__ int64_t part_start(const TcParams &p, int64_t b, int64_t ctas) { return b * p.stages / ctas; }
+
+// The work of a CTA, item by item: stages [s0, s1) of row tile rt of class c.
+// `slot`: -1, a whole tile; else where its partial sums go -- the split's
+// index, or 2 b (a part that begins inside the tile) or 2 b + 1 of CTA b.
+template <bool EQ>
+struct Work {
+    int u;              // next whole tile or unit
+    int64_t pos, end;   // next and last stage of the CTA's equal part
+    int c, rt, s0, s1, slot;
+    __device__ __forceinline__ explicit Work(const TcParams &p) : u(blockIdx.x) {
+        pos = EQ ? part_start(p, blockIdx.x, gridDim.x) : 0;
+        end = EQ ? part_start(p, blockIdx.x + 1, gridDim.x) : 0;
+    }
+    __device__ __forceinline__ bool next(const TcParams &p) {
+        int sp;
+        if (u < (EQ ? p.whole : p.cls_u0[4])) {
+            unit_coords(p, u, c, rt, sp);
+            s0 = sp * p.kchunk_st;
+            s1 = min(p.nst, s0 + p.kchunk_st);
+            slot = p.splits > 1 ? sp : -1;
+            u += gridDim.x;
+            return true;
+        }
+        if (!EQ || pos >= end) return false;
+        const int tile = (int)(pos / p.nst);
+        unit_coords(p, p.whole + tile, c, rt, sp);
+        s0 = (int)(pos - (int64_t)tile * p.nst);
+        s1 = end - pos < p.nst - s0 ? s0 + (int)(end - pos) : p.nst;
+        slot = s0 == 0 && s1 == p.nst ? -1 : 2 * (int)blockIdx.x + (s0 == 0 ? 1 : 0);
+        pos += s1 - s0;
+        return true;
+    }
+};
+
+// C(row, j) from its sum
+__device__ __forceinline__ void store_output(const TcParams &p, float *cp, float sum) {
+    float v = p.alpha * sum;
+    if (p.semantics == GB_SEM_BLAS) {
+        if (p.beta != 0.f) v = fmaf(p.beta, *cp, v);
+    } else if (p.semantics == GB_SEM_SCALAR_BETA) {
+        v = v + p.beta;
+    } else {
+        v = *cp + (v + p.beta);
+    }
+    *cp = v;
 }
 
 // XL: 0 row-major X (rows in classes when ldx % 4 != 0), 1 K-major X with
-// ldx % 4 == 0, 2 K-major X in k-line classes
-template <int NB, int XL>
+// ldx % 4 == 0, 2 K-major X in k-line classes.  EQ: equal parts.
+template <int NB, int XL, bool EQ>
 __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ Maps maps, TcParams p) {
     constexpr bool XCOLS = XL != 0;
     using C = Cfg<NB>;
@@ -112,7 +186,6 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acce + 2);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int units = p.cls_u0[4];
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -137,13 +210,12 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
 
     if (warp == 0) {
         if (lane == 0) {   // TMA producer
+            ptx::pdl_wait();   // the pieces of W
             int g = 0;
             bool go = true;
-            for (int u = blockIdx.x; u < units && go; u += gridDim.x) {
-                int c, rt, sp;
-                unit_coords(p, u, c, rt, sp);
-                const int s0 = sp * p.kchunk_st, s1 = min(p.nst, s0 + p.kchunk_st);
-                for (int ks = s0; ks < s1; ks++, g++) {
+            Work<EQ> w(p);
+            while (go && w.next(p)) {
+                for (int ks = w.s0; ks < w.s1; ks++, g++) {
                     const int s = g % STAGES;
                     if (g >= STAGES && !ptx::mbar_wait(&empty[s], ((g / STAGES) & 1) ^ 1, p.err, 51)) {
                         go = false;
@@ -154,17 +226,19 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
                         ptx::mbar_arrive_expect_tx(&full[s], 4 * CB_BYTES + 2 * C::WP);
 #pragma unroll
                         for (int kc = 0; kc < 4; kc++)
-                            ptx::tma_load_2d(st + kc * CB_BYTES, &maps.x[kc], &full[s], rt * BM, ks * CB_L);
+                            ptx::tma_load_2d(st + kc * CB_BYTES, &maps.x[kc], &full[s], w.rt * BM, ks * CB_L);
                     } else {
                         ptx::mbar_arrive_expect_tx(&full[s], 2 * BM * 32 * 4 + 2 * C::WP);
 #pragma unroll
                         for (int b = 0; b < 2; b++) {
-                            if (XCOLS) ptx::tma_load_2d(st + b * BM * 128, &maps.x[c], &full[s], rt * BM, ks * KS + 32 * b);
-                            else ptx::tma_load_2d(st + b * BM * 128, &maps.x[c], &full[s], ks * KS + 32 * b, rt * BM);
+                            if (XCOLS)
+                                ptx::tma_load_2d(st + b * BM * 128, &maps.x[w.c], &full[s], w.rt * BM, ks * KS + 32 * b);
+                            else
+                                ptx::tma_load_2d(st + b * BM * 128, &maps.x[w.c], &full[s], ks * KS + 32 * b, w.rt * BM);
                         }
                     }
-                    ptx::tma_load_2d(st + C::XS, &maps.wh[c], &full[s], ks * KS + WOFF, 0);
-                    ptx::tma_load_2d(st + C::XS + C::WP, &maps.wl[c], &full[s], ks * KS + WOFF, 0);
+                    ptx::tma_load_2d(st + C::XS, &maps.wh[w.c], &full[s], ks * KS + WOFF, 0);
+                    ptx::tma_load_2d(st + C::XS + C::WP, &maps.wl[w.c], &full[s], ks * KS + WOFF, 0);
                 }
             }
         }
@@ -173,12 +247,11 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
             constexpr uint32_t idesc = ptx::idesc_bf16_f32(BM, NB);
             int g = 0, it = 0;
             bool go = true;
-            for (int u = blockIdx.x; u < units && go; u += gridDim.x, it++) {
-                int c, rt, sp;
-                unit_coords(p, u, c, rt, sp);
-                const int s0 = sp * p.kchunk_st, s1 = min(p.nst, s0 + p.kchunk_st);
+            Work<EQ> w(p);
+            while (go && w.next(p)) for (int s0 = w.s0; s0 < w.s1 && go; s0 += p.fold) {
+                const int s1 = min(w.s1, s0 + p.fold);
                 const int b = it & 1;
-                if (it >= 2 && !ptx::mbar_wait(&acce[b], ((it >> 1) & 1) ^ 1, p.err, 52)) break;
+                if (it >= 2 && !ptx::mbar_wait(&acce[b], ((it >> 1) & 1) ^ 1, p.err, 52)) { go = false; break; }
                 ptx::tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)(b * NB);
                 for (int ks = s0; ks < s1; ks++, g++) {
@@ -205,6 +278,7 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
                     ptx::umma_commit(&aempty[a]);
                 }
                 if (go) ptx::umma_commit(&accf[b]);
+                it++;
             }
         }
     } else if (warp < 6) {   // converters: thread = row q*32 + lane of the tile
@@ -212,12 +286,10 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         int g = 0;
         bool go = true;
-        for (int u = blockIdx.x; u < units && go; u += gridDim.x) {
-            int c, rt, sp;
-            unit_coords(p, u, c, rt, sp);
-            const int s0 = sp * p.kchunk_st, s1 = min(p.nst, s0 + p.kchunk_st);
-            const int delta = p.cls_delta[c];
-            for (int ks = s0; ks < s1; ks++, g++) {
+        Work<EQ> w(p);
+        while (go && w.next(p)) {
+            const int delta = p.cls_delta[w.c];
+            for (int ks = w.s0; ks < w.s1; ks++, g++) {
                 const int s = g % STAGES, a = g % ASLOTS;
                 if (!ptx::mbar_wait(&full[s], (g / STAGES) & 1, p.err, 55) ||
                     (g >= ASLOTS && !ptx::mbar_wait(&aempty[a], ((g / ASLOTS) & 1) ^ 1, p.err, 56))) {
@@ -283,29 +355,35 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
         const int q = warp % 4;
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         int it = 0;
-        for (int u = blockIdx.x; u < units; u += gridDim.x, it++) {
-            int c, rt, sp;
-            unit_coords(p, u, c, rt, sp);
-            const int b = it & 1;
-            if (!ptx::mbar_wait(&accf[b], (it >> 1) & 1, p.err, 57)) break;
-            ptx::tc_fence_after();
+        Work<EQ> w(p);
+        bool go = true;
+        while (go && w.next(p)) {
             float acc[NB];
 #pragma unroll
-            for (int cc = 0; cc < NB; cc += 16) {
-                uint32_t v[16];
-                ptx::tmem_ld_32x32b_x16(tmem + lane_off + (uint32_t)(b * NB + cc), v);
-                ptx::tmem_ld_wait();
+            for (int j = 0; j < NB; j++) acc[j] = 0.f;
+            for (int f = w.s0; f < w.s1; f += p.fold, it++) {
+                const int b = it & 1;
+                if (!ptx::mbar_wait(&accf[b], (it >> 1) & 1, p.err, 57)) { go = false; break; }
+                ptx::tc_fence_after();
 #pragma unroll
-                for (int j = 0; j < 16; j++) acc[cc + j] = __uint_as_float(v[j]);
+                for (int cc = 0; cc < NB; cc += 16) {
+                    uint32_t v[16];
+                    ptx::tmem_ld_32x32b_x16(tmem + lane_off + (uint32_t)(b * NB + cc), v);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; j++) acc[cc + j] += __uint_as_float(v[j]);
+                }
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&acce[b]);
             }
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&acce[b]);
-            const int64_t i = (int64_t)rt * BM + q * 32 + lane;   // row within the class
-            if (i >= p.cls_rows[c]) continue;
-            const int64_t row = i * p.rstride + c;
-            if (p.splits > 1) {
-                float *pp = p.part + ((int64_t)sp * p.rows + row) * NB;
+            if (!go) break;
+            const int64_t i = (int64_t)w.rt * BM + q * 32 + lane;   // row within the class
+            if (i >= p.cls_rows[w.c]) continue;
+            const int64_t row = i * p.rstride + w.c;
+            if (w.slot >= 0) {
+                float *pp = p.part + (EQ ? (int64_t)w.slot * BM + q * 32 + lane
+                                                   : (int64_t)w.slot * p.rows + row) * NB;
 #pragma unroll
                 for (int j = 0; j < NB; j += 4)
                     *reinterpret_cast<float4 *>(pp + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
@@ -315,16 +393,7 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < NB; j++) {
                 if (j >= p.n) break;
-                float *cp = cr + (int64_t)j * p.cs_c;
-                float v = p.alpha * acc[j];
-                if (p.semantics == GB_SEM_BLAS) {
-                    if (p.beta != 0.f) v = fmaf(p.beta, *cp, v);
-                } else if (p.semantics == GB_SEM_SCALAR_BETA) {
-                    v = v + p.beta;
-                } else {
-                    v = *cp + (v + p.beta);
-                }
-                *cp = v;
+                store_output(p, cr + (int64_t)j * p.cs_c, acc[j]);
             }
         }
     }
@@ -337,37 +406,91 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
     }
 }
 
-// W (logical K x n; tw: stored n x K) -> hi / lo BF16 pieces [nb][lp] for
-// each phase d < nphase: piece_d[j][x] = W(x - WOFF - d, j), zero outside
-// 0 <= k < K, j < n.  K-major, 128-byte rows of 64 k.
-__global__ void wsplit_kernel(const float *__restrict__ W, int64_t ldw, int tw, int n, int64_t K, int64_t lp, int nb,
-                              int nphase, __nv_bfloat16 *__restrict__ pieces) {
-    const int64_t per = (int64_t)nb * lp;
-    const int64_t total = per * nphase;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t d = e / per, r = e - d * per;
-        const int64_t j = r / lp, x = r - j * lp;
-        const int64_t k = x - WOFF - d;
-        float v = 0.f;
-        if (j < n && k >= 0 && k < K) v = tw ? W[j * ldw + k] : W[k * ldw + j];
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        __nv_bfloat16 *hi = pieces + d * 2 * per, *lo = hi + per;
-        hi[r] = h;
-        lo[r] = __float2bfloat16_rn(v - __bfloat162float(h));
+// Tiles cut between CTAs: their parts added in order, then the epilogue.
+// Block (b, q): rows 32 q .. 32 q + 31 of the tile that the start of CTA b + 1's
+// part cuts, if no earlier part starts inside the tile.
+__global__ void __launch_bounds__(256) thin_tc_join_kernel(TcParams p, int nb, int ctas) {
+    ptx::pdl_wait();
+    const int64_t cut = part_start(p, (int64_t)blockIdx.x + 1, ctas);
+    const int tile = (int)(cut / p.nst);
+    const int64_t p0 = (int64_t)tile * p.nst, p1 = p0 + p.nst;
+    if (cut == p0 || part_start(p, blockIdx.x, ctas) > p0) return;
+    int last = (int)blockIdx.x + 1;   // CTAs blockIdx.x .. last hold a part
+    while (last + 1 < ctas && part_start(p, (int64_t)last + 1, ctas) < p1) last++;
+    int c, rt, sp;
+    unit_coords(p, p.whole + tile, c, rt, sp);
+    for (int e = threadIdx.x; e < 32 * p.n; e += blockDim.x) {
+        // neighbouring threads on neighbouring outputs of C: columns of a row, or rows of a column
+        const int r = blockIdx.y * 32 + (p.cs_c == 1 ? e / p.n : e % 32), j = p.cs_c == 1 ? e % p.n : e / 32;
+        const int64_t i = (int64_t)rt * BM + r;
+        if (i >= p.cls_rows[c]) continue;
+        const float *pp = p.part + (int64_t)r * nb + j;
+        float s = pp[(2 * (int64_t)blockIdx.x + 1) * BM * nb];   // the CTA that begins the tile
+        for (int b = (int)blockIdx.x + 1; b <= last; b++) s += pp[2 * (int64_t)b * BM * nb];
+        store_output(p, p.C + (i * p.rstride + c) * p.cs_r + (int64_t)j * p.cs_c, s);
     }
 }
 
-template <int NB, int XL>
-gb_status launch_nb(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, int grid) {
+// W (logical K x n; tw: stored n x K) -> hi / lo BF16 pieces [nb][lp] for
+// each phase d: piece_d[j][x] = W(x - WOFF - d, j), zero outside 0 <= k < K,
+// j < n.  K-major, 128-byte rows of 64 k.  A thread makes eight x of one row
+// (16-byte stores); blockIdx.y = row j, blockIdx.z = phase d.  The kernel that
+// reads the pieces may start beside this one.
+__global__ void __launch_bounds__(128) wsplit_kernel(const float *__restrict__ W, int64_t ldw, int tw, int n, int64_t K,
+                                                     int64_t lp, int nb, __nv_bfloat16 *__restrict__ pieces) {
+    ptx::pdl_launch_dependents();
+    const int64_t x = ((int64_t)blockIdx.x * 128 + threadIdx.x) * 8;
+    if (x >= lp) return;
+    const int j = blockIdx.y, d = blockIdx.z;
+    const int64_t k0 = x - WOFF - d, step = tw ? 1 : ldw;
+    const float *src = W + (tw ? (int64_t)j * ldw + k0 : k0 * ldw + j);
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float v[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int64_t k = k0 + 2 * i + q;
+            v[q] = j < n && k >= 0 && k < K ? __ldg(src + (2 * i + q) * step) : 0.f;
+        }
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(v[0], v[1]);
+        const float2 hf = __bfloat1622float2(hi);
+        h[i] = bf16x2_bits(hi);
+        l[i] = bf16x2_bits(__floats2bfloat162_rn(v[0] - hf.x, v[1] - hf.y));
+    }
+    const int64_t per = (int64_t)nb * lp;
+    __nv_bfloat16 *hi = pieces + d * 2 * per + (int64_t)j * lp + x;
+    *reinterpret_cast<uint4 *>(hi) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(hi + per) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+template <int NB, int XL, bool EQ>
+gb_status launch_nb(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, int grid, bool dependent) {
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
-        GB_CUDA_TRY(cudaFuncSetAttribute(thin_tc_kernel<NB, XL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        GB_CUDA_TRY(cudaFuncSetAttribute(thin_tc_kernel<NB, XL, EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg<NB>::SMEM));
         device_setup_done(attr);
     }
-    thin_tc_kernel<NB, XL><<<grid, NT, Cfg<NB>::SMEM, a.stream>>>(maps, tp);
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = Cfg<NB>::SMEM;
+    cfg.stream = a.stream;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = dependent ? 1 : 0;
+    GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, thin_tc_kernel<NB, XL, EQ>, maps, tp));
     GB_LAUNCH_CHECK("thin_tc_kernel");
+    if (EQ && grid > 1) {
+        cfg.gridDim = dim3((unsigned)(grid - 1), BM / 32);
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = 0;
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, thin_tc_join_kernel, tp, NB, grid));
+        GB_LAUNCH_CHECK("thin_tc_join_kernel");
+    }
     return ok();
 }
 
@@ -392,12 +515,12 @@ gb_status launch_thin_tc(const ThinTcArgs &a) {
     const int nphase = classes ? 4 : 1;
     const int64_t lp = pieces_len(a.K, classes);
     __nv_bfloat16 *pieces = (__nv_bfloat16 *)a.wpieces;
-    {
-        const int64_t total = (int64_t)nphase * a.nb * lp;
-        const int blocks = (int)(ceil_div(total, 256) < 2 * sm_count() ? ceil_div(total, 256) : 2 * sm_count());
-        wsplit_kernel<<<blocks, 256, 0, a.stream>>>(a.W, a.ldw, a.tw, a.n, a.K, lp, a.nb, nphase, pieces);
-        GB_LAUNCH_CHECK("wsplit_kernel");
-    }
+    const dim3 wgrid((unsigned)ceil_div(lp / 8, 128), (unsigned)a.nb, (unsigned)nphase);
+    wsplit_kernel<<<wgrid, 128, 0, a.stream>>>(a.W, a.ldw, a.tw, a.n, a.K, lp, a.nb, pieces);
+    GB_LAUNCH_CHECK("wsplit_kernel");
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;   // captured launches keep plain stream order
+    GB_CUDA_TRY(cudaStreamIsCapturing(a.stream, &cap));
+    const bool dependent = cap == cudaStreamCaptureStatusNone;
     Maps maps;
     memset(&maps, 0, sizeof(maps));
     TcParams tp;
@@ -405,6 +528,8 @@ gb_status launch_thin_tc(const ThinTcArgs &a) {
     tp.rows = a.rows; tp.K = a.K; tp.n = a.n; tp.splits = a.splits;
     tp.nst = (int)thin_tc_stages(a.K, classes);
     tp.kchunk_st = (int)(a.kchunk / KS);
+    tp.fold = a.fold;
+    tp.tile_first = a.tx ? (int)ceil_div(a.rows, BM) : 0;
     tp.rstride = classes ? 4 : 1;
     bool okm = true;
     int u = 0;
@@ -455,19 +580,28 @@ gb_status launch_thin_tc(const ThinTcArgs &a) {
     if (!err) return set_status(GB_ERR_OOM, "skinny: no device error word");
     tp.C = a.C; tp.cs_r = a.cs_r; tp.cs_c = a.cs_c; tp.alpha = a.alpha; tp.beta = a.beta;
     tp.semantics = a.semantics; tp.part = a.part; tp.err = err;
-    const int grid = u < sm_count() ? u : sm_count();
+    int grid = u < sm_count() ? u : sm_count();
+    if (a.parts > 0) {
+        const int waves = u / a.parts;
+        tp.whole = waves >= 2 ? (waves - 1) * a.parts : 0;
+        tp.stages = (int64_t)(u - tp.whole) * tp.nst;   // at least one a CTA
+        grid = (int)(a.parts < tp.stages ? a.parts : tp.stages);
+    }
     if (grid == 0) return ok();
     const int xl = !a.tx ? 0 : (kcls ? 2 : 1);
-    switch (a.nb * 4 + xl) {
-        case 64: return launch_nb<16, 0>(a, maps, tp, grid);
-        case 65: return launch_nb<16, 1>(a, maps, tp, grid);
-        case 66: return launch_nb<16, 2>(a, maps, tp, grid);
-        case 128: return launch_nb<32, 0>(a, maps, tp, grid);
-        case 129: return launch_nb<32, 1>(a, maps, tp, grid);
-        case 130: return launch_nb<32, 2>(a, maps, tp, grid);
-        case 256: return launch_nb<64, 0>(a, maps, tp, grid);
-        case 257: return launch_nb<64, 1>(a, maps, tp, grid);
-        case 258: return launch_nb<64, 2>(a, maps, tp, grid);
+    switch (a.nb * 4 + (a.parts > 0 ? 3 : xl)) {
+        case 64: return launch_nb<16, 0, false>(a, maps, tp, grid, dependent);
+        case 65: return launch_nb<16, 1, false>(a, maps, tp, grid, dependent);
+        case 66: return launch_nb<16, 2, false>(a, maps, tp, grid, dependent);
+        case 67: return launch_nb<16, 0, true>(a, maps, tp, grid, dependent);
+        case 128: return launch_nb<32, 0, false>(a, maps, tp, grid, dependent);
+        case 129: return launch_nb<32, 1, false>(a, maps, tp, grid, dependent);
+        case 130: return launch_nb<32, 2, false>(a, maps, tp, grid, dependent);
+        case 131: return launch_nb<32, 0, true>(a, maps, tp, grid, dependent);
+        case 256: return launch_nb<64, 0, false>(a, maps, tp, grid, dependent);
+        case 257: return launch_nb<64, 1, false>(a, maps, tp, grid, dependent);
+        case 258: return launch_nb<64, 2, false>(a, maps, tp, grid, dependent);
+        case 259: return launch_nb<64, 0, true>(a, maps, tp, grid, dependent);
         default: return set_status(GB_ERR_UNSUPPORTED, "skinny: no tensor-core tile for n = %d", a.n);
     }
 }

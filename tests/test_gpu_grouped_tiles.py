@@ -32,7 +32,7 @@ def test_grouped_exact(torch, count, lo, hi, bits):
         A, B, C = (mk(K, M) if ta == "T" else mk(M, K)), (mk(N, K) if tb == "T" else mk(K, N)), mk(M, N)
         opA = (A[:K, :M].t() if ta == "T" else A[:M, :K]).double()
         opB = (B[:N, :K].t() if tb == "T" else B[:K, :N]).double()
-        want = C.double()
+        want = C.double().clone()
         P = 2.0 * (opA @ opB) if K else torch.zeros((M, N), dtype=torch.float64, device="cuda:0")
         want[:, :N] = P - 3.0 * want[:, :N] if sem == 0 else P - 3.0 if sem == 1 else want[:, :N] + P - 3.0
         descs.append(gbblas.gemm_desc(str(ta), str(tb), M, N, K, 2.0, A, A.shape[1], B, B.shape[1], -3.0, C, C.shape[1],
