@@ -79,76 +79,6 @@ constexpr uint32_t TMEM_COLS = 512;            // [0,256): two FP32 accumulators
 // ------------------------------------------------------------- exponents
 // (exp_of_maxbits: the line exponent from the maximum |x| bit pattern)
 
-// one warp per line of `len` contiguous elements
-__global__ void maxexp_contig_kernel(const double *__restrict__ X, int64_t ld, int64_t lines, int64_t len,
-                                     int *__restrict__ e) {
-    const int64_t line = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const int lane = threadIdx.x % 32;
-    if (line >= lines) return;
-    unsigned long long mb = 0;
-    const unsigned long long *p = reinterpret_cast<const unsigned long long *>(X + line * ld);
-    for (int64_t k = lane; k < len; k += 32) {
-        unsigned long long b = __ldg(p + k) & 0x7FFFFFFFFFFFFFFFull;
-        mb = b > mb ? b : mb;
-    }
-    for (int o = 16; o; o >>= 1) {
-        unsigned long long v = __shfl_xor_sync(0xffffffffu, mb, o);
-        mb = v > mb ? v : mb;
-    }
-    if (lane == 0) e[line] = exp_of_maxbits(mb);
-}
-
-// Column exponents of a len x cols storage (rows strided by ld), in three
-// small kernels: e[] = INT_MIN; each block reduces 32 consecutive columns
-// (lane = column, coalesced) over kpb rows and raises e[col] to the
-// exponent of its maximum (exponents are monotone in |x|, so the maximum of
-// the partial exponents is the exponent of the maximum; an all-zero part
-// contributes INT_MIN); INT_MIN (an all-zero column) -> 0.
-__global__ void exp_init_kernel(int *__restrict__ e, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        e[i] = INT_MIN;
-}
-
-__global__ void __launch_bounds__(256) maxexp_strided_kernel(const double *__restrict__ X, int64_t ld, int64_t cols,
-                                                             int64_t len, int64_t kpb, int *__restrict__ e) {
-    __shared__ unsigned long long part[8][32];
-    const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
-    const int64_t j = (int64_t)blockIdx.x * 32 + lane;
-    const int64_t k0 = (int64_t)blockIdx.y * kpb;
-    unsigned long long mb = 0;
-    if (j < cols) {
-        const unsigned long long *p = reinterpret_cast<const unsigned long long *>(X);
-        const int64_t k1 = k0 + kpb < len ? k0 + kpb : len;
-#pragma unroll 8
-        for (int64_t k = k0 + w; k < k1; k += 8) {
-            const unsigned long long b = __ldg(p + k * ld + j) & 0x7FFFFFFFFFFFFFFFull;
-            mb = b > mb ? b : mb;
-        }
-    }
-    part[w][lane] = mb;
-    __syncthreads();
-    if (w == 0 && j < cols) {
-#pragma unroll
-        for (int i = 1; i < 8; i++) mb = part[i][lane] > mb ? part[i][lane] : mb;
-        if (mb != 0) atomicMax(e + j, exp_of_maxbits(mb));
-    }
-}
-
-__global__ void exp_finish_kernel(int *__restrict__ e, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        if (e[i] == INT_MIN) e[i] = 0;
-}
-
-static void launch_maxexp_strided(const double *X, int64_t ld, int64_t cols, int64_t len, int *e, cudaStream_t st) {
-    const unsigned nb = (unsigned)(ceil_div(cols, 256) < 4096 ? ceil_div(cols, 256) : 4096);
-    exp_init_kernel<<<nb, 256, 0, st>>>(e, cols);
-    int64_t kpb = 256;   // rows per block; more when len would need over 65535 blocks in y
-    while (ceil_div(len, kpb) > 65535) kpb *= 2;
-    dim3 grid((unsigned)ceil_div(cols, 32), (unsigned)ceil_div(len, kpb));
-    maxexp_strided_kernel<<<grid, 256, 0, st>>>(X, ld, cols, len, kpb, e);
-    exp_finish_kernel<<<nb, 256, 0, st>>>(e, cols);
-}
-
 // Largest |x| of every row of op(A) and column of op(B), as bits, by atomicMax
 // from blocks of 64 lines x 16 `steps` k, both operands in one launch (out
 // cleared before).  Element (r, k): trans ? X[k*ldx + r] : X[r*ldx + k].
@@ -847,18 +777,6 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
 }  // namespace
 
 static gb_status ozaki_one(const GemmArgs &g, int s);
-
-// Exponents e of `lines` lines of `len` FP64 values (max |x| < 2^e, 0 for an
-// all-zero line): line i at X + i*ld (contiguous) or, strided, element k of
-// line i at X[k*ld + i].
-gb_status ozaki_line_exponents(const double *X, int64_t ld, bool strided, int64_t lines, int64_t len, int *e,
-                               cudaStream_t st) {
-    if (lines <= 0) return ok();
-    if (!strided) maxexp_contig_kernel<<<(unsigned)ceil_div(lines, 8), 256, 0, st>>>(X, ld, lines, len, e);
-    else launch_maxexp_strided(X, ld, lines, len, e, st);
-    GB_LAUNCH_CHECK("ozaki exponents");
-    return ok();
-}
 
 // Slices of both operands take s * (Mp + Np) * Kp * 2 bytes of workspace.
 // Past kWorkspaceCap the K range is cut into chunks, each sliced and

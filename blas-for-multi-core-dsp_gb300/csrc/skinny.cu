@@ -615,12 +615,12 @@ bool tc_eligible(const SkParams &p) {
 
 // K ranges per tile: units for four waves and more (one range when there are as
 // many tiles), up to twice as many where that leaves the last wave fuller; at
-// least eight stages a range.
-inline int balanced_splits(int64_t tiles, int64_t nst) {
+// least `least` of the nst steps of K a range.
+inline int balanced_splits(int64_t tiles, int64_t nst, int64_t least) {
     const double sms = sm_count();
     int best = 1;
     double best_fill = 0.0;
-    for (int s = 1; s <= 64 && (s == 1 || nst / s >= 8); s++) {
+    for (int s = 1; s <= 64 && (s == 1 || nst / s >= least); s++) {
         const double units = (double)(tiles * s), fill = units / (ceil(units / sms) * sms);
         if (units >= 8.0 * sms && s > 1 && best_fill > 0.0) break;
         if (units < 4.0 * sms || fill > best_fill + 0.02) {
@@ -648,7 +648,7 @@ gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
         const int64_t nst = thin_tc_stages(p.K, classes);
         const int64_t sms = sm_count();
         const bool equal = p.want_splits <= 0 && !p.tx && pl.rtiles < 4 * sms && pl.rtiles * nst >= 16 * sms;
-        const int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst);
+        const int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst, 8);
         const int64_t cst = ceil_div(nst, want);
         p.kchunk = cst * 64;
         p.splits = (int)ceil_div(nst, cst);
@@ -905,12 +905,9 @@ gb_status dispatch(const GemmArgs &g, size_t *need = nullptr) {
     if (p.n > 64) return set_status(GB_ERR_UNSUPPORTED, "skinny: small dimension %lld > 64",
                                     (long long)(g.M < g.N ? g.M : g.N));
     if (sizeof(T) == 8 && thin_oz_eligible(p.tx, p.ldx, p.X, p.rows, p.K)) {
-        // FP64: digits on the tensor cores; units of 128 rows x K chunks of
-        // 512, split K until there are ~4 units per SM
+        // FP64: digits on the tensor cores; units of 128 rows x K chunks of 512
         const int64_t rtiles = ceil_div(p.rows, 128), nchunks = ceil_div(p.K, 512);
-        int splits = 1;
-        while (rtiles * splits < 4 * (int64_t)sm_count() && nchunks / (splits * 2) >= 2 && splits < 64) splits *= 2;
-        if (g.split_k > 0) splits = g.split_k;
+        int splits = g.split_k > 0 ? g.split_k : balanced_splits(rtiles, nchunks, 2);
         const int64_t cpc = ceil_div(nchunks, splits);
         splits = (int)ceil_div(nchunks, cpc);
         if (need) {

@@ -62,8 +62,6 @@ bool make_tmap_f64(CUtensorMap *map, const void *base, uint64_t inner, uint64_t 
                    uint32_t box_inner, uint32_t box_outer, bool sw128);
 bool make_tmap_bf16(CUtensorMap *map, const void *base, uint64_t inner, uint64_t outer, uint64_t row_bytes,
                     uint32_t box_inner, uint32_t box_outer, int swizzle_bytes);
-gb_status ozaki_line_exponents(const double *X, int64_t ld, bool strided, int64_t lines, int64_t len, int *e,
-                               cudaStream_t st);
 
 namespace {
 namespace thin_oz {
@@ -109,12 +107,18 @@ struct OzThinParams {
     int tx, tw, j0;
 };
 
-// The (unit, chunk) pairs of this CTA in order: unit u = (row tile, split),
+// Unit u = (row tile, split).  Row-major X: the splits of a tile one after the
+// other; K-major X: the tiles of a split, so that the CTAs at work read
+// neighbouring pieces of the same k lines.
+__device__ __forceinline__ int split_of(const OzThinParams &p, int u) { return p.tx ? u / p.rtiles : u % p.splits; }
+__device__ __forceinline__ int tile_of(const OzThinParams &p, int u) { return p.tx ? u % p.rtiles : u / p.splits; }
+
+// The (unit, chunk) pairs of this CTA in order:
 // chunks of CHUNK_KB k blocks from the split's first.
 struct Walk {
     int u, c0, kb1;
     __device__ __forceinline__ void set(const OzThinParams &p, int nkb) {
-        c0 = (u % p.splits) * p.kchunk_kb;
+        c0 = split_of(p, u) * p.kchunk_kb;
         kb1 = min(nkb, c0 + p.kchunk_kb);
     }
     __device__ __forceinline__ void first(const OzThinParams &p, int nkb) {
@@ -401,6 +405,7 @@ __global__ void __launch_bounds__(NT, 1)
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    ptx::pdl_wait();   // W's digits (returns at once when not launched as a dependent)
 
     if (warp == 0 || warp == 14) {
         // producers: warp 0 the converter stages (X + W digits), warp 14 the scan ring; X by TMA
@@ -412,7 +417,7 @@ __global__ void __launch_bounds__(NT, 1)
             int g = 0;
             bool go = true;
             for (int u = blockIdx.x; u < units && go; u += gridDim.x) {
-                const int rt = u / p.splits, sp = u - rt * p.splits;
+                const int rt = tile_of(p, u), sp = split_of(p, u);
                 const int kb0 = sp * p.kchunk_kb, kb1 = min(nkb, kb0 + p.kchunk_kb);
                 for (int kb = kb0; kb < kb1; kb++, g++) {
                     const int s = g % nst;
@@ -444,7 +449,7 @@ __global__ void __launch_bounds__(NT, 1)
             int g = 0, ch = 0;
             bool go = true;
             for (int u = blockIdx.x; u < units && go; u += gridDim.x) {
-                const int sp = u % p.splits;
+                const int sp = split_of(p, u);
                 const int kb0 = sp * p.kchunk_kb, kb1 = min(nkb, kb0 + p.kchunk_kb);
                 for (int c0 = kb0; c0 < kb1 && go; c0 += CHUNK_KB, ch++) {
                     const int c1 = min(kb1, c0 + CHUNK_KB);
@@ -497,7 +502,7 @@ __global__ void __launch_bounds__(NT, 1)
         int g = 0, ch = 0;
         bool go = true;
         for (int u = blockIdx.x; u < units && go; u += gridDim.x) {
-            const int sp = u % p.splits;
+            const int sp = split_of(p, u);
             const int kb0 = sp * p.kchunk_kb, kb1 = min(nkb, kb0 + p.kchunk_kb);
             int e = 0;
             bool fast = true;
@@ -605,7 +610,7 @@ __global__ void __launch_bounds__(NT, 1)
             }
             if (!go) break;
             if (dw.last()) {   // the unit's sums are complete
-                const int rt = dw.u / p.splits, sp = dw.u - rt * p.splits;
+                const int rt = tile_of(p, dw.u), sp = split_of(p, dw.u);
                 const int64_t row = (int64_t)rt * BM + r;
                 if (row < p.rows) {
                     const int er = eref == NO_EXP ? 0 : eref;
@@ -613,7 +618,7 @@ __global__ void __launch_bounds__(NT, 1)
                         double *pp = p.part + ((int64_t)sp * p.rows + row) * p.pw;
 #pragma unroll
                         for (int j = 0; j < NG * NB; j++)
-                            if (j < p.n) pp[j] = mul_pow2(acc[j], er + __ldg(p.fcol + j));
+                            if (j < p.n) pp[j] = scale_pow2(acc[j], er + __ldg(p.fcol + j));
                         if (nf) p.nfrow[row] = 1;
                     } else {
                         double *cr = p.C + row * p.cs_r;
@@ -622,7 +627,7 @@ __global__ void __launch_bounds__(NT, 1)
                             if (j >= p.n) break;
                             const int fc = __ldg(p.fcol + j);
                             if (!nf && fc != kNonFiniteLineExp)
-                                store_out(p, cr + (int64_t)j * p.cs_c, mul_pow2(acc[j], er + fc));
+                                store_out(p, cr + (int64_t)j * p.cs_c, scale_pow2(acc[j], er + fc));
                         }
 #pragma unroll 1
                         for (int j = 0; j < p.n; j++)   // a row or column that holds an Inf / NaN
@@ -703,9 +708,37 @@ __global__ void __launch_bounds__(NT, 1)
     }
 }
 
+// Exponents of W's columns (logical K x n; tw: stored n x K), a CTA each.  The
+// digits' kernel may be launched beside this one.
+__global__ void __launch_bounds__(512) wexp_kernel(const double *__restrict__ W, int64_t ldw, int tw, int64_t K,
+                                                   int *__restrict__ fcol) {
+    __shared__ unsigned long long red[16];
+    const unsigned long long *w = reinterpret_cast<const unsigned long long *>(W) + (tw ? blockIdx.x * ldw : blockIdx.x);
+    const int64_t step = tw ? 1 : ldw;
+    unsigned long long m = 0;
+#pragma unroll 8
+    for (int64_t k = threadIdx.x; k < K; k += 512) {
+        const unsigned long long v = __ldg(w + k * step) & 0x7FFFFFFFFFFFFFFFull;
+        m = v > m ? v : m;
+    }
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, s);
+        m = v > m ? v : m;
+    }
+    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 1; i < 16; i++) m = red[i] > m ? red[i] : m;
+        fcol[blockIdx.x] = exp_of_maxbits(m);
+    }
+}
+
 // Split-K: sum the parts (already scaled) in order, then the epilogue; a
 // row or column holding an Inf / NaN gets the plain dot product.
 __global__ void thin_oz_reduce_kernel(OzThinParams p) {
+    ptx::pdl_wait();
     const int64_t total = p.rows * p.n;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -727,6 +760,7 @@ __global__ void thin_oz_reduce_kernel(OzThinParams p) {
 // a digit), K-major, kp columns, zero beyond n and K.
 __global__ void wdigits_kernel(const double *__restrict__ W, int64_t ldw, int tw, int n, int j0, int pw, int64_t K,
                                int64_t kp, const int *__restrict__ fcol, unsigned short *__restrict__ out) {
+    ptx::pdl_wait();   // the exponents; an earlier pass's reads of `out`
     const int64_t total = (int64_t)pw * kp;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {
@@ -797,9 +831,20 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
     int *err = error_word();
     if (!err) return set_status(GB_ERR_OOM, "skinny: no device error word");
 
-    gb_status s = ozaki_line_exponents(W, ldw, tw == 0, n, K, fcol, st);
-    if (s != GB_OK) return s;
     if (splits > 1) GB_CUDA_TRY(cudaMemsetAsync(nfrow, 0, (size_t)rows * 4, st));
+    wexp_kernel<<<n, 512, 0, st>>>(W, ldw, tw, K, fcol);
+    GB_LAUNCH_CHECK("wexp_kernel");
+    // each further kernel is a programmatic dependent of the one before (captured ones keep plain
+    // stream order)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    cudaLaunchAttribute pdl;
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = st;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
 
     // X through TMA when its rows (or k lines) start on 16-byte boundaries, else by cp.async
     const char *force = getenv("GB_SKINNY_OZ_CPASYNC");   // "1": the cp.async loader for any X (tests)
@@ -834,29 +879,30 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
         const int pw = ng * NB, nc = n - j0 < pw ? n - j0 : pw;
         const int64_t wtot = (int64_t)pw * kp;
         const int blocks = (int)(ceil_div(wtot, 256) < 2 * sm_count() ? ceil_div(wtot, 256) : 2 * sm_count());
-        wdigits_kernel<<<blocks, 256, 0, st>>>(W, ldw, tw, n, j0, pw, K, kp, fcol + j0, wd);
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = 0;
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, wdigits_kernel, W, ldw, tw, n, j0, pw, K, kp, (const int *)(fcol + j0), wd));
         GB_LAUNCH_CHECK("wdigits_kernel");
         OzThinParams p{rows, K, nc, splits, (int)(kchunk / KB), rtiles, pw,
                        C + j0 * cs_c, cs_r, cs_c, alpha, beta, semantics, part, nfrow, fcol + j0, err,
                        X, W, ldx, ldw, tx, tw, j0};
         const CUtensorMap &twm = tw_map[ng - 1];
-        if (ng == 1) {
-            const int sm = Cfg<1>::SMEM;
-            if (tx && cpa) thin_oz_kernel<true, true, 1><<<grid, NT, sm, st>>>(tx_map, twm, p);
-            else if (tx) thin_oz_kernel<true, false, 1><<<grid, NT, sm, st>>>(tx_map, twm, p);
-            else if (cpa) thin_oz_kernel<false, true, 1><<<grid, NT, sm, st>>>(tx_map, twm, p);
-            else thin_oz_kernel<false, false, 1><<<grid, NT, sm, st>>>(tx_map, twm, p);
-        } else {
-            const int sm = Cfg<2>::SMEM;
-            if (tx && cpa) thin_oz_kernel<true, true, 2><<<grid, NT, sm, st>>>(tx_map, twm, p);
-            else if (tx) thin_oz_kernel<true, false, 2><<<grid, NT, sm, st>>>(tx_map, twm, p);
-            else if (cpa) thin_oz_kernel<false, true, 2><<<grid, NT, sm, st>>>(tx_map, twm, p);
-            else thin_oz_kernel<false, false, 2><<<grid, NT, sm, st>>>(tx_map, twm, p);
-        }
+        auto kernel = ng == 1 ? (tx ? (cpa ? thin_oz_kernel<true, true, 1> : thin_oz_kernel<true, false, 1>)
+                                    : (cpa ? thin_oz_kernel<false, true, 1> : thin_oz_kernel<false, false, 1>))
+                              : (tx ? (cpa ? thin_oz_kernel<true, true, 2> : thin_oz_kernel<true, false, 2>)
+                                    : (cpa ? thin_oz_kernel<false, true, 2> : thin_oz_kernel<false, false, 2>));
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(NT);
+        cfg.dynamicSmemBytes = ng == 1 ? Cfg<1>::SMEM : Cfg<2>::SMEM;
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tx_map, twm, p));
         GB_LAUNCH_CHECK("thin_oz_kernel");
         if (splits > 1) {
             const int rb = (int)(ceil_div(rows * nc, 256) < 4 * sm_count() ? ceil_div(rows * nc, 256) : 4 * sm_count());
-            thin_oz_reduce_kernel<<<rb, 256, 0, st>>>(p);
+            cfg.gridDim = dim3((unsigned)rb);
+            cfg.blockDim = dim3(256);
+            cfg.dynamicSmemBytes = 0;
+            GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, thin_oz_reduce_kernel, p));
             GB_LAUNCH_CHECK("thin_oz_reduce_kernel");
         }
         j0 += pw;
