@@ -568,29 +568,35 @@ __global__ void __launch_bounds__(NT, 1)
 }
 
 // ------------------------------------------------------------ wide form
-// 128 x 256 C tiles (BN_W = 256): every MMA is M128 N256 K16, twice the work
-// of the 128 x 128 form's per instruction and per byte of V staged, and the
-// W tile of a k-block serves 256 columns.  The two FP32 accumulators take all
-// 512 TMEM columns, so the FP64 running sum of each diagonal flush lives in
-// a per-CTA scratch array in global memory (256 KB per CTA, L2-resident,
-// interleaved so that a warp's access to one pair of a lane's values is 512
-// contiguous bytes).  Warps: 0 TMA, 1 MMA, 2-9 epilogue (two per TMEM lane
-// quarter, 128 columns each).  The arithmetic is that of ozaki_gemm_kernel
-// (same chunk sums, flush order, exact scalings and rounding), so the
-// results are the same bit for bit.
+// 128 x 256 C tiles of one CTA (CG = 1), or 256 x 256 of a cluster of two (CG = 2).
+// What bounds it is operand bytes into the SM's shared memory, about 64 a clock:
+// a k-block of 128 x 256 brings 48 KB for 1024 clocks of MMA at most.  Two CTAs on
+// one tile (cta_group::2) hold half of W each, 32 KB a k-block for the same work,
+// and six stages fit.  4096^3, s = 8: 4106 us one CTA, 3596 two; 8192^3 26.7 and
+// 25.5 ms, there 1.60 PFLOP/s under the power limit.  One CTA stays where tiles of
+// 256 rows would waste a wave.  The two FP32 accumulators take all 512 TMEM
+// columns, so the FP64 running sum of each diagonal flush lives in a per-CTA
+// scratch array in global memory (256 KB per CTA, L2-resident, interleaved so that
+// a warp's access to one pair of a lane's values is 512 contiguous bytes).  Warps:
+// 0 TMA, 1 MMA (of a pair's first CTA), 2-9 epilogue (two per TMEM lane quarter,
+// 128 columns each).  The arithmetic is that of ozaki_gemm_kernel (same chunk sums,
+// flush order, exact scalings and rounding), so the results are the same bit for bit.
 namespace wide {
-constexpr int BN_W = 256, STAGES_W = 4, EW = 8, NT_W = 64 + 32 * EW;
-constexpr int W_TILE = BN_W * BK * 2;                       // 32 KB
-constexpr int STAGE_W = TILE_BYTES + W_TILE;                // 48 KB
-constexpr int SMEM_W = STAGES_W * STAGE_W + 1024 + 256;
-static_assert(SMEM_W <= 232448, "shared memory");
+constexpr int BN_W = 256, EW = 8, NT_W = 64 + 32 * EW;
+// per CTA of a unit of CG: 48 KB a stage, or 32 KB with half of W's rows
+template <int CG> struct Stg {
+    static constexpr int BYTES = TILE_BYTES + BN_W / CG * BK * 2, N = CG == 2 ? 6 : 4, SMEM = N * BYTES + 1024 + 256;
+};
+static_assert(Stg<1>::SMEM <= 232448 && Stg<2>::SMEM <= 232448, "shared memory");
 constexpr size_t SCRATCH_DOUBLES = (size_t)EW * 32 * 128;   // per CTA
 }  // namespace wide
 
+template <int CG>
 __global__ void __launch_bounds__(wide::NT_W, 1)
     ozaki_wide_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW, OzParams p,
                       double *scratch) {
     using namespace wide;
+    constexpr int STAGES_W = Stg<CG>::N, STAGE_W = Stg<CG>::BYTES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES_W * STAGE_W);
@@ -600,6 +606,7 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int rank = CG == 2 ? (int)ptx::cluster_ctarank() : 0, unit = blockIdx.x / CG, units = gridDim.x / CG;
     const int num_tiles = p.tiles_m * p.tiles_n;
     const int nchunks = (p.num_kb + p.chunk_kb - 1) / p.chunk_kb;
 
@@ -610,15 +617,20 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
         }
         for (int b = 0; b < 2; b++) {
             ptx::mbar_init(&acc_full[b], 1);
-            ptx::mbar_init(&acc_empty[b], EW);
+            ptx::mbar_init(&acc_empty[b], CG * EW);
         }
         ptx::fence_mbar_init();
         ptx::tma_prefetch_desc(&tmV);
         ptx::tma_prefetch_desc(&tmW);
     }
-    if (warp == 1) ptx::tmem_alloc(tmem_slot, TMEM_COLS);
+    if (warp == 1) {
+        if (CG == 2) ptx::tmem_alloc_pair(tmem_slot, TMEM_COLS);
+        else ptx::tmem_alloc(tmem_slot, TMEM_COLS);
+    }
+    __syncwarp();
     ptx::tc_fence_before();
-    __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();
+    else __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     ptx::pdl_wait();   // the slices (and everything before them on the stream)
@@ -627,12 +639,12 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
         if (lane == 0) {   // TMA producer: per tile, per pair, every K block
             int kbg = 0;
             bool go = true;
-            for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
+            for (int t = unit; t < num_tiles && go; t += units) {
                 int tm, tn;
                 tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
                 for (int q = 0; q < p.npairs && go; q++) {
-                    const int vrow = (int)((p.pt[q] - 1) * p.mp + (int64_t)tm * BM);
-                    const int wrow = (int)((p.pu[q] - 1) * p.np + (int64_t)tn * BN_W);
+                    const int vrow = (int)((p.pt[q] - 1) * p.mp + ((int64_t)tm * CG + rank) * BM);
+                    const int wrow = (int)((p.pu[q] - 1) * p.np + (int64_t)tn * BN_W + rank * (BN_W / CG));
                     for (int kb = 0; kb < p.num_kb; kb++, kbg++) {
                         const int s = kbg % STAGES_W;
                         if (kbg >= STAGES_W && !ptx::mbar_wait(&empty[s], ((kbg / STAGES_W) & 1) ^ 1, p.err, 11)) {
@@ -640,19 +652,30 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
                             break;
                         }
                         uint8_t *st = smem + s * STAGE_W;
-                        ptx::mbar_arrive_expect_tx(&full[s], STAGE_W);
-                        ptx::tma_load_2d(st, &tmV, &full[s], kb * BK, vrow);
-                        ptx::tma_load_2d(st + TILE_BYTES, &tmW, &full[s], kb * BK, wrow);
+                        if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], CG * STAGE_W);
+                        if (CG == 2) {   // the first CTA's barrier counts both CTAs' bytes
+                            const uint32_t bar = ptx::cluster_addr(&full[s], 0);
+                            ptx::tma_load_2d_pair(st, &tmV, bar, kb * BK, vrow);
+                            ptx::tma_load_2d_pair(st + TILE_BYTES, &tmW, bar, kb * BK, wrow);
+                        } else {
+                            ptx::tma_load_2d(st, &tmV, &full[s], kb * BK, vrow);
+                            ptx::tma_load_2d(st + TILE_BYTES, &tmW, &full[s], kb * BK, wrow);
+                        }
                     }
                 }
             }
+            if (CG == 2) {   // neither CTA may leave while copies or arrivals of the other are under way
+                for (int i = max(0, kbg - STAGES_W); i < kbg && go; i++)
+                    go = ptx::mbar_wait(&empty[i % STAGES_W], (i / STAGES_W) & 1, p.err, 15);
+                for (int i = 0; i < 64 && !go; i++) __nanosleep(2000);
+            }
         }
     } else if (warp == 1) {
-        if (lane == 0) {   // MMA issuer: one accumulator per K chunk of a pair
-            constexpr uint32_t idesc = ptx::idesc_bf16_f32(BM, BN_W);
+        if (lane == 0 && rank == 0) {   // MMA issuer: one accumulator per K chunk of a pair
+            constexpr uint32_t idesc = ptx::idesc_bf16_f32(CG * BM, BN_W);
             int kbg = 0, gi = 0;
             bool go = true;
-            for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
+            for (int t = unit; t < num_tiles && go; t += units) {
                 for (int q = 0; q < p.npairs && go; q++) {
                     for (int c = 0; c < nchunks && go; c++, gi++) {
                         const int b = gi & 1;
@@ -676,11 +699,16 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
 #pragma unroll
                             for (int k = 0; k < BK / 16; k++) {
                                 const uint64_t dk = (uint64_t)((k * 32) >> 4);
-                                ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * p.chunk_kb) || (k != 0));
+                                const uint32_t add = (kb != c * p.chunk_kb) || (k != 0);
+                                if (CG == 2) ptx::umma_f16_pair(acc, vd + dk, wd + dk, idesc, add);
+                                else ptx::umma_f16(acc, vd + dk, wd + dk, idesc, add);
                             }
-                            ptx::umma_commit(&empty[s]);
+                            if (CG == 2) ptx::umma_commit_pair(&empty[s]);
+                            else ptx::umma_commit(&empty[s]);
                         }
-                        if (go) ptx::umma_commit(&acc_full[b]);
+                        if (!go) break;
+                        if (CG == 2) ptx::umma_commit_pair(&acc_full[b]);
+                        else ptx::umma_commit(&acc_full[b]);
                     }
                 }
             }
@@ -692,7 +720,7 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
                 (size_t)(threadIdx.x / 32 - 2) * 64 * 32 + threadIdx.x % 32)
         int gi = 0;
         bool go = true;
-        for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
+        for (int t = unit; t < num_tiles && go; t += units) {
             bool first_flush = true;
             int iacc[128];
 #pragma unroll
@@ -716,7 +744,10 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
                     }
                     ptx::tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&acc_empty[b]);
+                    if (lane == 0) {
+                        if (CG == 2) ptx::mbar_arrive_cluster(ptx::cluster_addr(&acc_empty[b], 0));
+                        else ptx::mbar_arrive(&acc_empty[b]);
+                    }
                     const bool flush = (c == nchunks - 1 && lev_ends) || ++nacc == MAX_CHUNKS_INT32;
                     if (flush) {   // FP64 sum += 2^(2-8(t+u)) * iacc (exact scaling, one rounding)
                         nacc = 0;
@@ -750,7 +781,7 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
             // C = alpha * 2^(e_i + f_j) * sum (+ beta ...): this lane's row, 128 columns
             int tm, tn;
             tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-            const int64_t row = (int64_t)tm * BM + q * 32 + lane;
+            const int64_t row = ((int64_t)tm * CG + rank) * BM + q * 32 + lane;
             const int64_t c0 = (int64_t)tn * BN_W + (w / 4) * 128;
             const int erow = row < p.M ? p.erow[row] : 0;
             const double2 *scr = OZ_SCR;
@@ -766,11 +797,14 @@ __global__ void __launch_bounds__(wide::NT_W, 1)
     }
 
 #undef OZ_SCR
+    __syncwarp();
     ptx::tc_fence_before();
-    __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();
+    else __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem, TMEM_COLS);
+        if (CG == 2) ptx::tmem_dealloc_pair(tmem, TMEM_COLS);
+        else ptx::tmem_dealloc(tmem, TMEM_COLS);
     }
 }
 
@@ -809,11 +843,27 @@ gb_status launch_dgemm_ozaki(const GemmArgs &g, int slices) {
 }
 
 static gb_status ozaki_one(const GemmArgs &g, int s) {
-    // The wide form (128 x 256 tiles) once op(B) has 256 columns, unless 128 x 128 tiles take less time
-    // (waves of tiles, a k-block at 0.39 against 0.27 us); GB_OZAKI_WIDE=0 keeps 128 x 128
+    // 128 x 128 tiles, 128 x 256 ones of one CTA, or 256 x 256 ones of two, whichever takes the least
+    // time: waves of tiles times (a k-block of a digit pair, us, and the part of a level's flush that
+    // the next chunk does not hide, which decides for short K).  GB_OZAKI_WIDE=0 keeps 128 x 128.
+    // Measured, us:             128 x 128   one CTA   two CTAs
+    //   4096x1024x4096              1435      1103       997
+    //   3301x4098x3621              3628      2855      2574
+    //   4000x1270x2000              1082      1073      1010
+    //   384x12800x1024               485       483       710
+    //   2305x2305x1300               770       826       805
+    //   3900x1293x605                436       515       527
+    //   1500x1500x1500               313       441       430
     const char *wv = getenv("GB_OZAKI_WIDE");
-    auto waves = [&](int width) { return ceil((double)ceil_div(g.M, BM) * (double)ceil_div(g.N, width) / sm_count()); };
-    const bool wide = !(wv && wv[0] == '0') && g.N >= wide::BN_W && 0.39 * waves(wide::BN_W) <= 0.27 * waves(BN);
+    const double pair_kbs = 0.5 * s * (s + 1) * (double)ceil_div(g.K, BK);
+    auto cost = [&](int bm, int bn, int ctas, double kb_us, double level_us) {
+        const double waves = ceil((double)ceil_div(g.M, bm) * (double)ceil_div(g.N, bn) / (sm_count() / ctas));
+        return waves * (pair_kbs * kb_us + s * level_us);
+    };
+    const double c128 = cost(BM, BN, 1, 0.27, 3.5), c256 = cost(BM, wide::BN_W, 1, 0.41, 8.75);
+    const double cpair = g.M > BM ? cost(2 * BM, wide::BN_W, 2, 0.36, 10.6) : 1e30;
+    const bool wide = !(wv && wv[0] == '0') && g.N >= wide::BN_W && std::min(c256, cpair) <= c128;
+    const int cg = wide && cpair <= c256 ? 2 : 1;   // CTAs per tile
     const int bn = wide ? wide::BN_W : BN;
     const int64_t kp = ceil_div(g.K, BK) * BK;
     const int64_t mp = ceil_div(g.M, BM) * BM, np = ceil_div(g.N, bn) * bn;
@@ -821,8 +871,8 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
         return set_status(GB_ERR_UNSUPPORTED, "ozaki: problem too large for 32-bit TMA coordinates");
     const size_t ebytes = ((size_t)(mp + np) * sizeof(int) + 255) / 256 * 256;
     const size_t vbytes = (size_t)s * mp * kp * 2, wbytes = (size_t)s * np * kp * 2;
-    const int64_t tiles_total = (mp / BM) * (np / bn);
-    const int grid = (int)(tiles_total < sm_count() ? tiles_total : sm_count());
+    const int64_t tiles_total = ceil_div(mp, cg * BM) * (np / bn);
+    const int grid = cg * (int)std::min<int64_t>(tiles_total, sm_count() / cg);
     const size_t sbytes = wide ? (size_t)grid * wide::SCRATCH_DOUBLES * sizeof(double) : 0;
     const size_t mbytes = (size_t)(mp + np) * sizeof(unsigned long long);
     uint8_t *ws = (uint8_t *)workspace(vbytes + wbytes + ebytes + sbytes + mbytes + 4096, g.stream);
@@ -864,21 +914,21 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     // launch and set-up overlap it (captured launches keep plain stream order)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     GB_CUDA_TRY(cudaStreamIsCapturing(g.stream, &cap));
-    cudaLaunchAttribute pdl;
-    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)sblocks);
     cfg.blockDim = dim3(256);
     cfg.stream = g.stream;
-    cfg.attrs = &pdl;
+    cfg.attrs = attrs;
     cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
     GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, slice_kernel, sa));
     GB_LAUNCH_CHECK("ozaki slices");
 
     CUtensorMap tV, tW;
     if (!make_tmap_bf16(&tV, V, kp, (uint64_t)s * mp, kp * 2, BK, BM, 128) ||
-        !make_tmap_bf16(&tW, W, kp, (uint64_t)s * np, kp * 2, BK, bn, 128))
+        !make_tmap_bf16(&tW, W, kp, (uint64_t)s * np, kp * 2, BK, bn / cg, 128))
         return set_status(GB_ERR_CUDA, "ozaki: cuTensorMapEncodeTiled failed");
 
     OzParams p{};
@@ -887,7 +937,7 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     p.num_kb = (int)(kp / BK);
     // even chunks: the accumulator of a short last one would be drained slower than it fills
     p.chunk_kb = (int)ceil_div(p.num_kb, ceil_div(p.num_kb, KCHUNK_BLOCKS));
-    p.tiles_m = (int)(mp / BM); p.tiles_n = (int)(np / bn);
+    p.tiles_m = (int)ceil_div(mp, cg * BM); p.tiles_n = (int)(np / bn);
     p.mp = mp; p.np = np;
     p.erow = erow; p.fcol = fcol; p.err = err;
     p.A = A; p.B = B; p.lda = g.lda; p.ldb = g.ldb; p.K = g.K; p.ta = g.ta ? 1 : 0; p.tb = g.tb ? 1 : 0;
@@ -915,14 +965,23 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
         GB_CUDA_TRY(cudaFuncSetAttribute(ozaki_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        GB_CUDA_TRY(cudaFuncSetAttribute(ozaki_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_W));
+        GB_CUDA_TRY(cudaFuncSetAttribute(ozaki_wide_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         wide::Stg<1>::SMEM));
+        GB_CUDA_TRY(cudaFuncSetAttribute(ozaki_wide_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         wide::Stg<2>::SMEM));
         device_setup_done(attr);
     }
     cfg.gridDim = dim3((unsigned)grid);
     if (wide) {
         cfg.blockDim = dim3(wide::NT_W);
-        cfg.dynamicSmemBytes = wide::SMEM_W;
-        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, ozaki_wide_kernel, tV, tW, p, scratch));
+        cfg.dynamicSmemBytes = cg == 2 ? wide::Stg<2>::SMEM : wide::Stg<1>::SMEM;
+        if (cg == 2) {
+            attrs[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+            attrs[cfg.numAttrs].val.clusterDim.x = 2;
+            attrs[cfg.numAttrs].val.clusterDim.y = attrs[cfg.numAttrs].val.clusterDim.z = 1;
+            cfg.numAttrs++;
+        }
+        GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, cg == 2 ? ozaki_wide_kernel<2> : ozaki_wide_kernel<1>, tV, tW, p, scratch));
         GB_LAUNCH_CHECK("ozaki_wide_kernel");
     } else {
         cfg.blockDim = dim3(NT);
