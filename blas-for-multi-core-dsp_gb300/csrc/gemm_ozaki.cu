@@ -334,6 +334,8 @@ struct OzParams {
     int64_t mp, np;                // padded rows of one V / W slice
     int npairs;
     signed char pt[MAXPAIRS], pu[MAXPAIRS];   // 1-based digit indices per pair
+    int s, parts;                  // 128 x 128 form: CTAs that share a tile's chunks
+    int *sums;                     // parts > 1: int32 sums, [tile][level + part][128 x 128]
     const int *erow, *fcol;
     int *err;
     // operands, for the outputs that a non-finite row or column reaches
@@ -383,6 +385,15 @@ __device__ __forceinline__ void store_outputs(const OzParams &p, int64_t row, in
     }
 }
 
+// First unit (a chunk of a digit pair) of part j of a tile.
+__device__ __forceinline__ int part_start(int units, int parts, int j) { return (int)((int64_t)units * j / parts); }
+
+// Diagonal t + u of the pair that unit u belongs to.
+__device__ __forceinline__ int unit_level(const OzParams &p, int u, int nchunks) {
+    const int q = u / nchunks;
+    return q < p.npairs ? p.pt[q] + p.pu[q] : 0;
+}
+
 __global__ void __launch_bounds__(NT, 1)
     ozaki_gemm_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW, OzParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -394,8 +405,8 @@ __global__ void __launch_bounds__(NT, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int num_tiles = p.tiles_m * p.tiles_n;
-    const int nchunks = (p.num_kb + p.chunk_kb - 1) / p.chunk_kb;
+    const int items = p.tiles_m * p.tiles_n * p.parts;
+    const int nchunks = (p.num_kb + p.chunk_kb - 1) / p.chunk_kb, units = p.npairs * nchunks;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -421,13 +432,16 @@ __global__ void __launch_bounds__(NT, 1)
         if (lane == 0) {   // TMA producer: per tile, per pair, every K block
             int kbg = 0;
             bool go = true;
-            for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
+            for (int it = blockIdx.x; it < items && go; it += gridDim.x) {
                 int tm, tn;
-                tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-                for (int q = 0; q < p.npairs && go; q++) {
+                tile_coords(it / p.parts, p.tiles_m, p.tiles_n, tm, tn);
+                const int u1 = part_start(units, p.parts, it % p.parts + 1);
+                for (int u = part_start(units, p.parts, it % p.parts); u < u1 && go; u++) {
+                    const int q = u / nchunks, c = u - q * nchunks;
                     const int vrow = (int)((p.pt[q] - 1) * p.mp + (int64_t)tm * BM);
                     const int wrow = (int)((p.pu[q] - 1) * p.np + (int64_t)tn * BN);
-                    for (int kb = 0; kb < p.num_kb; kb++, kbg++) {
+                    const int kb_end = min(p.num_kb, (c + 1) * p.chunk_kb);
+                    for (int kb = c * p.chunk_kb; kb < kb_end; kb++, kbg++) {
                         const int s = kbg % STAGES;
                         if (kbg >= STAGES && !ptx::mbar_wait(&empty[s], ((kbg / STAGES) & 1) ^ 1, p.err, 11)) {
                             go = false;
@@ -446,36 +460,36 @@ __global__ void __launch_bounds__(NT, 1)
             constexpr uint32_t idesc = ptx::idesc_bf16_f32(BM, BN);
             int kbg = 0, gi = 0;
             bool go = true;
-            for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
-                for (int q = 0; q < p.npairs && go; q++) {
-                    for (int c = 0; c < nchunks && go; c++, gi++) {
-                        const int b = gi & 1;
-                        if (gi >= 2 && !ptx::mbar_wait(&acc_empty[b], ((gi >> 1) & 1) ^ 1, p.err, 12)) {
+            for (int it = blockIdx.x; it < items && go; it += gridDim.x) {
+                const int u1 = part_start(units, p.parts, it % p.parts + 1);
+                for (int u = part_start(units, p.parts, it % p.parts); u < u1 && go; u++, gi++) {
+                    const int c = u % nchunks;
+                    const int b = gi & 1;
+                    if (gi >= 2 && !ptx::mbar_wait(&acc_empty[b], ((gi >> 1) & 1) ^ 1, p.err, 12)) {
+                        go = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    const uint32_t acc = tmem + (uint32_t)(b * BN);
+                    const int kb_end = min(p.num_kb, (c + 1) * p.chunk_kb);
+                    for (int kb = c * p.chunk_kb; kb < kb_end; kb++, kbg++) {
+                        const int s = kbg % STAGES;
+                        if (!ptx::mbar_wait(&full[s], (kbg / STAGES) & 1, p.err, 13)) {
                             go = false;
                             break;
                         }
                         ptx::tc_fence_after();
-                        const uint32_t acc = tmem + (uint32_t)(b * BN);
-                        const int kb_end = min(p.num_kb, (c + 1) * p.chunk_kb);
-                        for (int kb = c * p.chunk_kb; kb < kb_end; kb++, kbg++) {
-                            const int s = kbg % STAGES;
-                            if (!ptx::mbar_wait(&full[s], (kbg / STAGES) & 1, p.err, 13)) {
-                                go = false;
-                                break;
-                            }
-                            ptx::tc_fence_after();
-                            const uint32_t st = ptx::smem_u32(smem + s * STAGE_BYTES);
-                            const uint64_t vd = ptx::sdesc_kmajor_sw128(st);
-                            const uint64_t wd = ptx::sdesc_kmajor_sw128(st + TILE_BYTES);
+                        const uint32_t st = ptx::smem_u32(smem + s * STAGE_BYTES);
+                        const uint64_t vd = ptx::sdesc_kmajor_sw128(st);
+                        const uint64_t wd = ptx::sdesc_kmajor_sw128(st + TILE_BYTES);
 #pragma unroll
-                            for (int k = 0; k < BK / 16; k++) {
-                                const uint64_t dk = (uint64_t)((k * 32) >> 4);
-                                ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * p.chunk_kb) || (k != 0));
-                            }
-                            ptx::umma_commit(&empty[s]);
+                        for (int k = 0; k < BK / 16; k++) {
+                            const uint64_t dk = (uint64_t)((k * 32) >> 4);
+                            ptx::umma_f16(acc, vd + dk, wd + dk, idesc, (kb != c * p.chunk_kb) || (k != 0));
                         }
-                        if (go) ptx::umma_commit(&acc_full[b]);
+                        ptx::umma_commit(&empty[s]);
                     }
+                    if (go) ptx::umma_commit(&acc_full[b]);
                 }
             }
         }
@@ -485,7 +499,8 @@ __global__ void __launch_bounds__(NT, 1)
         const uint32_t tot = tmem + 256u + lane_base + (uint32_t)(half * 128);   // FP64 sums: two columns each
         int gi = 0;
         bool go = true;
-        for (int t = blockIdx.x; t < num_tiles && go; t += gridDim.x) {
+        for (int it = blockIdx.x; it < items && go; it += gridDim.x) {
+            const int t = it / p.parts, part = it % p.parts;
             bool first_flush = true;
             // exact int32 sums of the chunk sums of consecutive pairs on one diagonal t + u (one
             // scale): one FP64 flush per diagonal, or after MAX_CHUNKS_INT32 chunk sums
@@ -493,52 +508,64 @@ __global__ void __launch_bounds__(NT, 1)
 #pragma unroll
             for (int j = 0; j < 64; j++) iacc[j] = 0;
             int nacc = 0;
-            for (int qq = 0; qq < p.npairs && go; qq++) {
-                const int lev = p.pt[qq] + p.pu[qq];
-                const bool lev_ends = qq == p.npairs - 1 || p.pt[qq + 1] + p.pu[qq + 1] != lev;
-                for (int c = 0; c < nchunks; c++, gi++) {
-                    const int b = gi & 1;
-                    if (!ptx::mbar_wait(&acc_full[b], (gi >> 1) & 1, p.err, 14)) { go = false; break; }
-                    ptx::tc_fence_after();
-                    uint32_t r0[32], r1[32];
-                    const uint32_t acc = tmem + (uint32_t)(b * BN + half * 64) + lane_base;
-                    ptx::tmem_ld_32x32b_x32(acc, r0);
-                    ptx::tmem_ld_32x32b_x32(acc + 32u, r1);
-                    ptx::tmem_ld_wait();
-                    ptx::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&acc_empty[b]);
+            const int u1 = part_start(units, p.parts, part + 1);
+            for (int u = part_start(units, p.parts, part); u < u1; u++, gi++) {
+                const int lev = unit_level(p, u, nchunks);
+                const bool lev_ends = u == u1 - 1 || unit_level(p, u + 1, nchunks) != lev;
+                const int b = gi & 1;
+                if (!ptx::mbar_wait(&acc_full[b], (gi >> 1) & 1, p.err, 14)) { go = false; break; }
+                ptx::tc_fence_after();
+                uint32_t r0[32], r1[32];
+                const uint32_t acc = tmem + (uint32_t)(b * BN + half * 64) + lane_base;
+                ptx::tmem_ld_32x32b_x32(acc, r0);
+                ptx::tmem_ld_32x32b_x32(acc + 32u, r1);
+                ptx::tmem_ld_wait();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&acc_empty[b]);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        iacc[j] += __float2int_rn(__uint_as_float(r0[j]));
-                        iacc[32 + j] += __float2int_rn(__uint_as_float(r1[j]));
+                for (int j = 0; j < 32; j++) {
+                    iacc[j] += __float2int_rn(__uint_as_float(r0[j]));
+                    iacc[32 + j] += __float2int_rn(__uint_as_float(r1[j]));
+                }
+                if (p.parts > 1) {   // a level's sum, or this part's share of it, to the join
+                    if (!lev_ends) continue;
+                    int4 *dst = reinterpret_cast<int4 *>(p.sums) +
+                                ((size_t)t * (p.s + p.parts - 1) + (p.s + 1 - lev + part)) * (BM * BN / 4) +
+                                (size_t)(half * 4 + q) * 16 * 32 + lane;
+#pragma unroll
+                    for (int g = 0; g < 16; g++) {
+                        __stcg(dst + g * 32, make_int4(iacc[4 * g], iacc[4 * g + 1], iacc[4 * g + 2], iacc[4 * g + 3]));
+                        iacc[4 * g] = iacc[4 * g + 1] = iacc[4 * g + 2] = iacc[4 * g + 3] = 0;
                     }
-                    const bool flush = (c == nchunks - 1 && lev_ends) || ++nacc == MAX_CHUNKS_INT32;
-                    if (flush) {   // FP64 sum += 2^(2-8(t+u)) * iacc (exact scaling, one rounding)
-                        nacc = 0;
+                    continue;
+                }
+                const bool flush = lev_ends || ++nacc == MAX_CHUNKS_INT32;
+                if (flush) {   // FP64 sum += 2^(2-8(t+u)) * iacc (exact scaling, one rounding)
+                    nacc = 0;
 #pragma unroll
-                        for (int cb = 0; cb < 8; cb++) {
-                            uint32_t r[16];
-                            if (!first_flush) {
-                                ptx::tmem_ld_32x32b_x16(tot + (uint32_t)(cb * 16), r);
-                                ptx::tmem_ld_wait();
-                            }
-#pragma unroll
-                            for (int j = 0; j < 8; j++) {
-                                double v = int_pow2(iacc[cb * 8 + j], 2 - 8 * lev);
-                                if (!first_flush) v = __dadd_rn(__hiloint2double((int)r[2 * j + 1], (int)r[2 * j]), v);
-                                r[2 * j] = (uint32_t)__double2loint(v);
-                                r[2 * j + 1] = (uint32_t)__double2hiint(v);
-                                iacc[cb * 8 + j] = 0;
-                            }
-                            ptx::tmem_st_32x32b_x16(tot + (uint32_t)(cb * 16), r);
+                    for (int cb = 0; cb < 8; cb++) {
+                        uint32_t r[16];
+                        if (!first_flush) {
+                            ptx::tmem_ld_32x32b_x16(tot + (uint32_t)(cb * 16), r);
+                            ptx::tmem_ld_wait();
                         }
-                        ptx::tmem_st_wait();
-                        first_flush = false;
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            double v = int_pow2(iacc[cb * 8 + j], 2 - 8 * lev);
+                            if (!first_flush) v = __dadd_rn(__hiloint2double((int)r[2 * j + 1], (int)r[2 * j]), v);
+                            r[2 * j] = (uint32_t)__double2loint(v);
+                            r[2 * j + 1] = (uint32_t)__double2hiint(v);
+                            iacc[cb * 8 + j] = 0;
+                        }
+                        ptx::tmem_st_32x32b_x16(tot + (uint32_t)(cb * 16), r);
                     }
+                    ptx::tmem_st_wait();
+                    first_flush = false;
                 }
             }
             if (!go) break;
+            if (p.parts > 1) continue;
             // C = alpha * 2^(e_i + f_j) * sum (+ beta ...): this lane's row, 64 columns
             int tm, tn;
             tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
@@ -565,6 +592,53 @@ __global__ void __launch_bounds__(NT, 1)
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem, TMEM_COLS);
     }
+}
+
+// The parts' int32 sums of every level, added up and taken into FP64 level by level:
+// the same integers, order and roundings as one CTA's flushes, so the same bits.
+// A thread has eight columns of a row.  Bound by the FP64 pipe's additions (2 a clock
+// and SM), which here all SMs share.
+__global__ void __launch_bounds__(256) ozaki_join_kernel(const __grid_constant__ OzParams p) {
+    const int nchunks = (p.num_kb + p.chunk_kb - 1) / p.chunk_kb, units = p.npairs * nchunks;
+    const int t = blockIdx.x / 8, e = (blockIdx.x % 8) * 256 + threadIdx.x;   // eight CTAs a tile
+    const int lane = e % 32, cb = e / 32 % 8, q = e / 256 % 4, half = e / 1024;
+    const int4 *src = reinterpret_cast<const int4 *>(p.sums) + (size_t)t * (p.s + p.parts - 1) * (BM * BN / 4) +
+                      (size_t)(half * 4 + q) * 16 * 32 + cb * 2 * 32 + lane;
+    ptx::pdl_wait();
+    double sum[8];
+    int acc[8], level = 0;   // level 0: nothing yet
+    bool first = true;
+#pragma unroll
+    for (int j = 0; j < 8; j++) { acc[j] = 0; sum[j] = 0.0; }
+    for (int part = 0; part < p.parts; part++) {
+        const int last = unit_level(p, part_start(units, p.parts, part + 1) - 1, nchunks);
+        for (int lev = unit_level(p, part_start(units, p.parts, part), nchunks); lev >= last; lev--) {
+            const int4 *at = src + (size_t)(p.s + 1 - lev + part) * (BM * BN / 4);
+            const int4 x = __ldcg(at), y = __ldcg(at + 32);
+            const int v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            if (lev != level && level) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const double d = int_pow2(acc[j], 2 - 8 * level);
+                    sum[j] = first ? d : __dadd_rn(sum[j], d);
+                    acc[j] = 0;
+                }
+                first = false;
+            }
+            level = lev;
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[j] += v[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const double d = int_pow2(acc[j], 2 - 8 * level);
+        sum[j] = first ? d : __dadd_rn(sum[j], d);
+    }
+    int tm, tn;
+    tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+    const int64_t row = (int64_t)tm * BM + q * 32 + lane;
+    store_outputs(p, row, (int64_t)tn * BN + half * 64 + cb * 8, row < p.M ? p.erow[row] : 0, sum);
 }
 
 // ------------------------------------------------------------ wide form
@@ -862,7 +936,33 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     };
     const double c128 = cost(BM, BN, 1, 0.27, 3.5), c256 = cost(BM, wide::BN_W, 1, 0.41, 8.75);
     const double cpair = g.M > BM ? cost(2 * BM, wide::BN_W, 2, 0.36, 10.6) : 1e30;
-    const bool wide = !(wv && wv[0] == '0') && g.N >= wide::BN_W && std::min(c256, cpair) <= c128;
+    // 128 x 128 tiles that leave SMs idle are shared by several CTAs, each with an equal part of the
+    // (pair, chunk) units, and joined by a launch of its own.  The parts' sums take no more than the
+    // wide form's scratch and stay exact in 32 bits; a part has 1.5 us for each level that it stores.
+    // GB_OZAKI_SPLIT=0 keeps one CTA per tile.  Measured, us (tiles; whole call):
+    //   512^3 (16)            150 whole   76 two   48 six   45 nine   56 nineteen
+    //   800^3 (49)            198        117      102 three 125 four
+    //   1000^3 (64)           228        151
+    //   300x300x4000 (9)      722        375      124 nine   99 sixteen  117 thirty-three
+    //   1000x1000x4000 (64)   766        440
+    const char *ord = getenv("GB_OZAKI_PAIR_ORDER"), *sv = getenv("GB_OZAKI_SPLIT");
+    const bool by_w = ord && ord[0] == 'w';
+    // even chunks: the accumulator of a short last one would be drained slower than it fills
+    const int num_kb = (int)ceil_div(g.K, BK), chunk_kb = (int)ceil_div(num_kb, ceil_div(num_kb, KCHUNK_BLOCKS));
+    const int nchunks = (int)ceil_div(num_kb, chunk_kb), units = s * (s + 1) / 2 * nchunks;
+    const int64_t tiles128 = ceil_div(g.M, BM) * ceil_div(g.N, BN);
+    const double unit_us = 0.27 * chunk_kb;
+    double csplit = 1e30;
+    int parts = 1;
+    for (int n = 2; !by_w && !(sv && sv[0] == '0') && s * nchunks <= MAX_CHUNKS_INT32 && n <= units; n++) {
+        if ((double)tiles128 * (s + n - 1) * (BM * BN * 4) > (double)sm_count() * wide::SCRATCH_DOUBLES * 8) break;
+        const double waves = ceil((double)tiles128 * n / sm_count());
+        const double c = waves * (ceil((double)units / n) * unit_us + (1.0 + (double)s / n) * 1.5) + 6.0 +
+                         (double)g.M * (double)g.N * (s + 2) / (2.0 * 1900.0 * sm_count());
+        if (c < csplit) { csplit = c; parts = n; }
+    }
+    if (csplit >= std::min(c128, std::min(c256, cpair))) parts = 1;
+    const bool wide = parts == 1 && !(wv && wv[0] == '0') && g.N >= wide::BN_W && std::min(c256, cpair) <= c128;
     const int cg = wide && cpair <= c256 ? 2 : 1;   // CTAs per tile
     const int bn = wide ? wide::BN_W : BN;
     const int64_t kp = ceil_div(g.K, BK) * BK;
@@ -872,10 +972,17 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     const size_t ebytes = ((size_t)(mp + np) * sizeof(int) + 255) / 256 * 256;
     const size_t vbytes = (size_t)s * mp * kp * 2, wbytes = (size_t)s * np * kp * 2;
     const int64_t tiles_total = ceil_div(mp, cg * BM) * (np / bn);
-    const int grid = cg * (int)std::min<int64_t>(tiles_total, sm_count() / cg);
-    const size_t sbytes = wide ? (size_t)grid * wide::SCRATCH_DOUBLES * sizeof(double) : 0;
+    int grid = cg * (int)std::min<int64_t>(tiles_total * parts, sm_count() / cg);
+    const size_t sums = (size_t)tiles_total * (s + parts - 1) * (BM * BN * 4);
+    size_t sbytes = wide ? (size_t)grid * wide::SCRATCH_DOUBLES * sizeof(double) : parts > 1 ? sums : 0;
     const size_t mbytes = (size_t)(mp + np) * sizeof(unsigned long long);
     uint8_t *ws = (uint8_t *)workspace(vbytes + wbytes + ebytes + sbytes + mbytes + 4096, g.stream);
+    if (!ws && parts > 1) {   // no room for the parts' sums
+        parts = 1;
+        sbytes = 0;
+        grid = (int)std::min<int64_t>(tiles_total, sm_count());
+        ws = (uint8_t *)workspace(vbytes + wbytes + ebytes + mbytes + 4096, g.stream);
+    }
     if (!ws) return (gb_status)gb_get_last_status();
     unsigned short *V = (unsigned short *)ws;
     unsigned short *W = (unsigned short *)(ws + vbytes);
@@ -935,8 +1042,7 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     p.C = (double *)g.C; p.M = g.M; p.N = g.N; p.ldc = g.ldc;
     p.alpha = g.alpha; p.beta = g.beta; p.semantics = g.semantics;
     p.num_kb = (int)(kp / BK);
-    // even chunks: the accumulator of a short last one would be drained slower than it fills
-    p.chunk_kb = (int)ceil_div(p.num_kb, ceil_div(p.num_kb, KCHUNK_BLOCKS));
+    p.chunk_kb = chunk_kb;
     p.tiles_m = (int)ceil_div(mp, cg * BM); p.tiles_n = (int)(np / bn);
     p.mp = mp; p.np = np;
     p.erow = erow; p.fcol = fcol; p.err = err;
@@ -948,9 +1054,8 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     // groups the pairs by the W digit u instead: the tiles in flight (8 tile
     // rows x 19 tile columns) keep W_u's panels hot in L2, halving the DRAM
     // reads, at one flush per pair.
-    const char *ord = getenv("GB_OZAKI_PAIR_ORDER");
     int n = 0;
-    if (!(ord && ord[0] == 'w')) {
+    if (!by_w) {
         for (int d = s + 1; d >= 2; d--)
             for (int t = 1; t <= s; t++) {
                 int u = d - t;
@@ -961,6 +1066,9 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
             for (int t = s + 1 - u; t >= 1; t--) { p.pt[n] = (signed char)t; p.pu[n] = (signed char)u; n++; }
     }
     p.npairs = n;
+    p.s = s;
+    p.parts = parts;
+    p.sums = parts > 1 ? (int *)(ws + vbytes + wbytes + ebytes) : nullptr;
 
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
@@ -988,6 +1096,13 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
         cfg.dynamicSmemBytes = SMEM_BYTES;
         GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, ozaki_gemm_kernel, tV, tW, p));
         GB_LAUNCH_CHECK("ozaki_gemm_kernel");
+        if (parts > 1) {
+            cfg.gridDim = dim3((unsigned)(8 * tiles_total));
+            cfg.blockDim = dim3(256);
+            cfg.dynamicSmemBytes = 0;
+            GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, ozaki_join_kernel, p));
+            GB_LAUNCH_CHECK("ozaki_join_kernel");
+        }
     }
     return ok();
 }
