@@ -496,10 +496,10 @@ constexpr int EPI_BYTES = 4 * 32 * 33 * 4;     // four warps' 32 x 32 staging, p
 // EW epilogue warps: 4 (one per TMEM lane quarter, all BN columns) or 8 (two
 // per lane quarter, 128 columns each: the wide folding form); both stage C
 // through shared memory so that loads and stores of C are coalesced.
-template <int NP, int BN, int EW, int BK>
+template <int NP, int BN, int EW, int BK, int CG>
 struct TwoPass {
     static_assert(BK == 32 || BK == 64, "64- or 128-byte swizzle atoms");
-    static constexpr int A_TILE = BM * BK * 2, B_TILE = BN * BK * 2;
+    static constexpr int A_TILE = BM * BK * 2, B_TILE = BN / CG * BK * 2;   // of one of CG CTAs
     static constexpr int STAGE_BYTES = NP * A_TILE + NP * B_TILE;
     static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;   // 2, 3 or 4
     static constexpr int NT = 64 + 32 * EW;
@@ -540,10 +540,11 @@ struct EpiParams {
     int ta, tb;
 };
 
-// Work item i of this CTA: a whole tile (half = -1) or the left / right 128
+// Work item i of this CTA (or pair of CTAs): a whole tile (half = -1) or the left / right 128
 // columns of a tail tile (half 0 / 1).
+template <int CG>
 __device__ __forceinline__ bool next_item(const EpiParams &p, int num_tiles, int &i, int &tile, int &half) {
-    const int t = blockIdx.x + i * gridDim.x;
+    const int t = blockIdx.x / CG + i * (int)(gridDim.x / CG);
     i++;
     half = -1;
     if (t < p.half_start) {
@@ -607,6 +608,19 @@ __device__ __forceinline__ void store_recomputed(const EpiParams &p, int64_t row
     *c = epi_value(p, x, reads_c(p) ? *c : 0.f);
 }
 
+// An epilogue warp is done with an accumulator: the issuing CTA's barrier.
+template <int CG>
+__device__ __forceinline__ void free_acc(uint64_t *bar) {
+    if (CG == 2) ptx::mbar_arrive_cluster(ptx::cluster_addr(bar, 0));
+    else ptx::mbar_arrive(bar);
+}
+
+// First row of C of this CTA's share of tile row tm.
+template <int CG>
+__device__ __forceinline__ int64_t tile_row0(int tm) {
+    return ((int64_t)tm * CG + (CG == 2 ? ptx::cluster_ctarank() : 0u)) * BM;
+}
+
 // FOLD: the tensor cores add each MMA into the FP32 accumulator with an
 // error of about one unit in the last place of the accumulator, biased like
 // a truncation, so over a long K the error grows with the number of MMAs and
@@ -622,18 +636,21 @@ __device__ __forceinline__ void store_recomputed(const EpiParams &p, int64_t row
 //    accumulator of 256 columns, two chunk buffers; each epilogue warp keeps
 //    the totals of 32 rows x 128 columns and writes C through shared memory
 //    16 columns at a time.
+// CG = 2: the two CTAs of a cluster share a tile of 256 x 256 (cta_group::2); each holds
+// its 128 rows of A, half of B's and its 128 rows of the accumulators.
 // The MMAs of chunk c+1 overlap the fold of chunk c.
 // F16: FP16 pieces of scaled lines (FP16X3), the epilogue applies the scales.
-template <int NP, int BN, bool FOLD, bool F16, int EW, int BK>
+template <int NP, int BN, bool FOLD, bool F16, int EW, int BK, int CG>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
     bf16x3_gemm_kernel(const __grid_constant__ PieceMaps maps, EpiParams p) {
     // the next call's split pass may start beside this grid (it writes the other workspace half)
     if (threadIdx.x == 0) ptx::pdl_launch_dependents();
-    using CF = TwoPass<NP, BN, EW, BK>;
+    using CF = TwoPass<NP, BN, EW, BK, CG>;
     constexpr int A_TILE = CF::A_TILE;
     constexpr bool SEP = FOLD && EW == 4;   // hi*hi apart from the cross products
     static_assert(!SEP || BN == 128, "the separated folding form keeps a 128-column total per thread");
     static_assert(EW == 4 || (FOLD && BN == 256), "eight epilogue warps: the wide folding form");
+    static_assert(CG == 1 || (NP == 2 && BN == 256), "pairs of CTAs: 256-column tiles of two pieces");
     static_assert(!F16 || EW == 8, "FP16 pieces: the wide folding form");
     constexpr int B_TILE = CF::B_TILE, STAGE_BYTES = CF::STAGE_BYTES, STAGES = CF::STAGES;
     constexpr uint32_t ACC_COLS = SEP ? 256 : BN, TMEM_COLS = 2 * ACC_COLS;
@@ -659,7 +676,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
         }
         for (int b = 0; b < 2; b++) {
             ptx::mbar_init(&acc_full[b], 1);
-            ptx::mbar_init(&acc_empty[b], EW);   // one arrive per epilogue warp
+            ptx::mbar_init(&acc_empty[b], CG * EW);   // one arrive per epilogue warp
         }
         ptx::fence_mbar_init();
         for (int i = 0; i < NP; i++) {
@@ -667,9 +684,14 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
             ptx::tma_prefetch_desc(&maps.b[i]);
         }
     }
-    if (warp == 1) ptx::tmem_alloc(tmem_slot, TMEM_COLS);
+    if (warp == 1) {
+        if (CG == 2) ptx::tmem_alloc_pair(tmem_slot, TMEM_COLS);
+        else ptx::tmem_alloc(tmem_slot, TMEM_COLS);
+    }
+    __syncwarp();
     ptx::tc_fence_before();
-    __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();
+    else __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     // launched as a dependent of the split pass: the set-up above overlaps it, its pieces are waited
@@ -681,11 +703,12 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
             int kbg = 0;   // running k-block counter across tiles (stage / phase)
             bool go = true;
             int it = 0, t, half;
-            while (go && next_item(p, num_tiles, it, t, half)) {
+            while (go && next_item<CG>(p, num_tiles, it, t, half)) {
                 int tm, tn;
                 tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-                const int m0 = tm * BM, n0 = tn * BN + (half > 0 ? BN / 2 : 0);
-                const uint32_t bytes = half < 0 ? STAGE_BYTES : NP * A_TILE + NP * (B_TILE / 2);
+                const int rank = CG == 2 ? (int)ptx::cluster_ctarank() : 0;
+                const int m0 = (tm * CG + rank) * BM, n0 = tn * BN + (half > 0 || rank ? BN / 2 : 0);
+                const uint32_t bytes = half < 0 ? CG * STAGE_BYTES : NP * A_TILE + NP * (B_TILE / 2);
                 for (int kb = 0; kb < p.num_kb; kb++, kbg++) {
                     const int s = kbg % STAGES;
                     if (kbg >= STAGES && !ptx::mbar_wait(&empty[s], ((kbg / STAGES) & 1) ^ 1, p.err, 1)) {
@@ -693,7 +716,16 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                         break;
                     }
                     uint8_t *st = smem + s * STAGE_BYTES;
-                    ptx::mbar_arrive_expect_tx(&full[s], bytes);
+                    if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], bytes);
+                    if (CG == 2) {   // the first CTA's barrier counts both CTAs' bytes
+                        const uint32_t bar = ptx::cluster_addr(&full[s], 0);
+#pragma unroll
+                        for (int i = 0; i < NP; i++) {
+                            ptx::tma_load_2d_pair(st + i * A_TILE, &maps.a[i], bar, kb * BK, m0);
+                            ptx::tma_load_2d_pair(st + NP * A_TILE + i * B_TILE, &maps.bh[i], bar, kb * BK, n0);
+                        }
+                        continue;
+                    }
 #pragma unroll
                     for (int i = 0; i < NP; i++) {
                         ptx::tma_load_2d(st + i * A_TILE, &maps.a[i], &full[s], kb * BK, m0);
@@ -702,15 +734,20 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                     }
                 }
             }
+            if (CG == 2) {   // neither CTA may leave while copies or arrivals of the other are under way
+                for (int i = max(0, kbg - STAGES); i < kbg && go; i++)
+                    go = ptx::mbar_wait(&empty[i % STAGES], (i / STAGES) & 1, p.err, 5);
+                for (int i = 0; i < 64 && !go; i++) __nanosleep(2000);
+            }
         }
     } else if (warp == 1) {
-        if (lane == 0) {   // MMA issuer
-            constexpr uint32_t idesc = idesc_f32acc<F16>(BM, BN);
+        if (lane == 0 && (CG == 1 || ptx::cluster_ctarank() == 0)) {   // MMA issuer (of a pair's first CTA)
+            constexpr uint32_t idesc = idesc_f32acc<F16>(CG * BM, BN);
             constexpr uint32_t idesc_half = idesc_f32acc<F16>(BM, BN / 2);
             int kbg = 0, ch = 0;   // running k-block and accumulator-chunk counters
             bool go = true;
             int it = 0, t, half;
-            while (go && next_item(p, num_tiles, it, t, half)) {
+            while (go && next_item<CG>(p, num_tiles, it, t, half)) {
                 const uint32_t id = half < 0 ? idesc : idesc_half;
                 const int nch = (p.num_kb + chunk_kb - 1) / chunk_kb;
                 for (int c = 0; c < nch && go; c++, ch++) {
@@ -747,13 +784,17 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
 #pragma unroll
                                 for (int i = d; i >= 0; i--) {
                                     const bool lead = SEP ? (d == NP - 1 && i == d) || d == 0 : d == NP - 1 && i == d;
-                                    ptx::umma_f16(d == 0 ? acc : acc_lo, ad[i] + dk, bd[d - i] + dk, id,
-                                                  !(first && k == 0 && lead));
+                                    const uint32_t into = d == 0 ? acc : acc_lo, add = !(first && k == 0 && lead);
+                                    if (CG == 2) ptx::umma_f16_pair(into, ad[i] + dk, bd[d - i] + dk, id, add);
+                                    else ptx::umma_f16(into, ad[i] + dk, bd[d - i] + dk, id, add);
                                 }
                         }
-                        ptx::umma_commit(&empty[s]);
+                        if (CG == 2) ptx::umma_commit_pair(&empty[s]);
+                        else ptx::umma_commit(&empty[s]);
                     }
-                    if (go) ptx::umma_commit(&acc_full[b]);
+                    if (!go) break;
+                    if (CG == 2) ptx::umma_commit_pair(&acc_full[b]);
+                    else ptx::umma_commit(&acc_full[b]);
                 }
             }
         }
@@ -765,10 +806,10 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
         float total[FOLD ? BN : 1];
         bool go = true;
         int it = 0, t, half;
-        while (go && next_item(p, num_tiles, it, t, half)) {
+        while (go && next_item<CG>(p, num_tiles, it, t, half)) {
             int tm, tn;
             tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-            const int64_t row0 = (int64_t)tm * BM + q * 32;
+            const int64_t row0 = tile_row0<CG>(tm) + q * 32;
             const int64_t n0 = (int64_t)tn * BN + (half > 0 ? BN / 2 : 0);
             const int ncols = half < 0 ? BN : BN / 2;
             uint32_t accb = 0;
@@ -792,7 +833,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                     }
                     ptx::tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(&acc_empty[b]);
+                    if (lane == 0) free_acc<CG>(&acc_empty[b]);
                 }
                 if (!go) break;
             } else {
@@ -839,7 +880,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
             if (!FOLD) {
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&acc_empty[ch & 1]);
+                if (lane == 0) free_acc<CG>(&acc_empty[ch & 1]);
                 ch++;
             }
         }
@@ -851,11 +892,11 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
         float total[128];
         bool go = true;
         int it = 0, t, half;
-        while (go && next_item(p, num_tiles, it, t, half)) {
+        while (go && next_item<CG>(p, num_tiles, it, t, half)) {
             if (F16) {   // the scales of the warp's rows and columns, once per tile
                 int tm, tn;
                 tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-                const int64_t row0 = (int64_t)tm * BM + (warp % 4) * 32;
+                const int64_t row0 = tile_row0<CG>(tm) + (warp % 4) * 32;
                 const int64_t c0 = (int64_t)tn * BN + (half < 0 ? ((warp - 2) / 4) * 128 : half * 128);
                 unsigned cb[4];
 #pragma unroll
@@ -890,18 +931,18 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&acc_empty[b]);
+                if (lane == 0) free_acc<CG>(&acc_empty[b]);
             }
             if (!go) break;
             // a half tile of the tail (128 columns in accumulator columns 0..127) is stored by the
             // warps of column half 0; the other four folded columns the MMA did not write
-            const int tl = blockIdx.x + (it - 1) * gridDim.x;
+            const int tl = blockIdx.x / CG + (it - 1) * (int)(gridDim.x / CG);
             const int hf = tl < p.half_start ? -1 : ((tl - p.half_start) & 1);
             if (hf >= 0 && warp >= 6) continue;
             int tm, tn;
             tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
             const int wi = warp - 2;
-            const int64_t row0 = (int64_t)tm * BM + (warp % 4) * 32;
+            const int64_t row0 = tile_row0<CG>(tm) + (warp % 4) * 32;
             const int64_t c0 = (int64_t)tn * BN + (hf < 0 ? (wi / 4) * 128 : hf * 128);
             const int *cs_w = col_scale + wi * 128;
             const int *rs_w = row_scale + wi * 32;
@@ -1014,11 +1055,14 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
         }
     }
 
+    __syncwarp();
     ptx::tc_fence_before();
-    __syncthreads();
+    if (CG == 2) ptx::cluster_sync_all();
+    else __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem, TMEM_COLS);
+        if (CG == 2) ptx::tmem_dealloc_pair(tmem, TMEM_COLS);
+        else ptx::tmem_dealloc(tmem, TMEM_COLS);
     }
     if (threadIdx.x == 0 && p.done) atomicAdd(p.done, 1ull);   // last: this CTA is done
 }
@@ -1461,21 +1505,21 @@ static void span(const void *p, bool trans, int64_t rows, int64_t cols, int64_t 
 }
 
 // bn: tile width; 128 with the 256-wide folding kernel runs every tile as two halves
-template <int NP, int BN, bool FOLD, bool F16, int EW, int BK>
+template <int NP, int BN, bool FOLD, bool F16, int EW, int BK, int CG = 1>
 static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64_t kp, const EpiParams &base, int bn,
                                  bool dependent, int *grid_out) {
-    using CF = TwoPass<NP, BN, EW, BK>;
-    auto kernel = bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW, BK>;
+    using CF = TwoPass<NP, BN, EW, BK, CG>;
+    auto kernel = bf16x3_gemm_kernel<NP, BN, FOLD, F16, EW, BK, CG>;
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
         GB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM_BYTES));
         device_setup_done(attr);
     }
-    const int tiles_m = (int)ceil_div(g.M, BM), tiles_n = (int)ceil_div(g.N, BN);
+    const int tiles_m = (int)ceil_div(g.M, CG * BM), tiles_n = (int)ceil_div(g.N, BN);
     const int tiles = tiles_m * tiles_n;
     const bool halves = bn < BN;
     const int64_t items = halves ? 2 * (int64_t)tiles : tiles;
-    const int grid = items < sm_count() ? (int)items : sm_count();
+    const int grid = CG * (int)std::min<int64_t>(items, sm_count() / CG);
     // half-tile tail when the last wave is at most half full (whole tiles
     // would leave most of the GPU idle for a tile time); GB_BF16X3_HALF=0 off.
     // The folding form keeps whole tiles unless GB_BF16X3_HALF=1: its halves
@@ -1486,7 +1530,7 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
         const char *e = getenv("GB_BF16X3_HALF");
         const int rem = tiles % grid;
         const bool on = FOLD ? (EW == 8 && e && e[0] == '1') : !(e && e[0] == '0');
-        if (BN == 256 && on && rem > 0 && 2 * rem <= grid) half_start = tiles - rem;
+        if (CG == 1 && BN == 256 && on && rem > 0 && 2 * rem <= grid) half_start = tiles - rem;
     }
     EpiParams p = base;
     p.num_kb = (int)(kp / BK);
@@ -1494,79 +1538,107 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
     p.tiles_n = tiles_n;
     p.chunk_kb = FOLD ? (p.chunk_kb > 0 ? p.chunk_kb * KB / BK : p.num_kb) : 1;
     p.half_start = half_start;
-    cudaLaunchAttribute pdl;
-    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attrs[2];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(CF::NT);
     cfg.dynamicSmemBytes = CF::SMEM_BYTES;
     cfg.stream = g.stream;
-    cfg.attrs = &pdl;
-    cfg.numAttrs = dependent ? 1 : 0;
+    cfg.attrs = attrs;
+    if (CG == 2) {
+        attrs[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attrs[cfg.numAttrs].val.clusterDim.x = 2;
+        attrs[cfg.numAttrs].val.clusterDim.y = attrs[cfg.numAttrs].val.clusterDim.z = 1;
+        cfg.numAttrs++;
+    }
+    if (dependent) {
+        attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs++;
+    }
     GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, p));
     GB_LAUNCH_CHECK("bf16x3_gemm_kernel");
     *grid_out = grid;
     return ok();
 }
 
-// k of a pipeline stage: 64 for tiles (or halves) narrower than 256 columns,
+// k of a pipeline stage: 64 for tiles (or halves) narrower than 256 columns and for pairs,
 // where the accumulator chunk is whole in it.
-static int block_k(int np, bool fold, int fold_kb, int bn) {
-    return np == 2 && bn < 256 && (!fold || fold_kb % 2 == 0) ? 64 : 32;
+static int block_k(int np, bool fold, int fold_kb, int bn, bool pair) {
+    return np == 2 && (bn < 256 || pair) && (!fold || fold_kb % 2 == 0) ? 64 : 32;
 }
 
 template <bool F16>
 static gb_status gemm_launch(const GemmArgs &g, int np, int fold_kb, const PieceMaps &maps, int64_t kp,
-                             const EpiParams &p, int bn, bool dependent, int *grid) {
+                             const EpiParams &p, int bn, bool pair, bool dependent, int *grid) {
     if constexpr (!F16) {   // three pieces are BF16 only
         if (np == 3)
             return fold_kb > 0 ? two_pass_launch<3, 128, true, false, 4, 32>(g, maps, kp, p, bn, dependent, grid)
                                : two_pass_launch<3, 128, false, false, 4, 32>(g, maps, kp, p, bn, dependent, grid);
     }
-    const bool k64 = block_k(np, F16 || fold_kb > 0, fold_kb, bn) == 64;
-    if constexpr (F16) {   // always the wide folding form (fold_kb 0: one chunk over all of K)
-        return k64 ? two_pass_launch<2, 256, true, true, 8, 64>(g, maps, kp, p, bn, dependent, grid)
-                   : two_pass_launch<2, 256, true, true, 8, 32>(g, maps, kp, p, bn, dependent, grid);
-    } else {
-        if (fold_kb > 0)
-            return k64 ? two_pass_launch<2, 256, true, false, 8, 64>(g, maps, kp, p, bn, dependent, grid)
-                       : two_pass_launch<2, 256, true, false, 8, 32>(g, maps, kp, p, bn, dependent, grid);
+    const bool k64 = block_k(np, F16 || fold_kb > 0, fold_kb, bn, pair) == 64;
+    if (F16 || fold_kb > 0) {   // the wide folding form (fold_kb 0: one chunk over all of K)
+        if constexpr (!F16)
+            if (pair) return two_pass_launch<2, 256, true, false, 8, 64, 2>(g, maps, kp, p, bn, dependent, grid);
+        return k64 ? two_pass_launch<2, 256, true, F16, 8, 64>(g, maps, kp, p, bn, dependent, grid)
+                   : two_pass_launch<2, 256, true, F16, 8, 32>(g, maps, kp, p, bn, dependent, grid);
+    }
+    if constexpr (!F16) {
+        if (pair) return two_pass_launch<2, 256, false, false, 4, 64, 2>(g, maps, kp, p, bn, dependent, grid);
         switch (bn) {
             case 64: return two_pass_launch<2, 64, false, false, 4, 64>(g, maps, kp, p, bn, dependent, grid);
             case 128: return two_pass_launch<2, 128, false, false, 4, 64>(g, maps, kp, p, bn, dependent, grid);
             default: return two_pass_launch<2, 256, false, false, 4, 32>(g, maps, kp, p, bn, dependent, grid);
         }
     }
+    return GB_ERR_INVALID_ARG;   // not reached
 }
 
 // Width of the C tiles.  256 columns need the least operand traffic per
 // product, narrow ones fill more SMs: the width of least estimated time
 // (waves of tiles x k-blocks of 32 at 0.27 / 0.315 / 0.60 us for 64 / 128 /
 // 256 columns, a tail wave of 256 at most half full counted half, plus launch
-// and epilogue).  Measured, us:
+// and epilogue).  `pair`: 256 x 256 tiles of two CTAs, a k-block at 0.53 us:
+// each CTA brings half of B, and with 32 KB a k-block of 32 instead of 48 the
+// stages have room for 128-byte rows.  Measured, us:
 //
-//                     64      128     256
+//                     64      128     256     256 x 256 of two
 //   513^3             12.0    15.9    27.1
 //   1111x937x1500     20.5    23.8    39.2
 //   1280^3            28.2    21.0    35.1
 //   2048^3            75.3    49.0    60.0
 //   2500^3            134     84.5    86.8
-//   4096^3            468     282     270
+//   3000^3                            123     117
+//   4096^3            468     282     282     278  (303 and 281 with odd leading dimensions)
+//   4096x2048x1000                    61.1    55.5
+//   8192x8192x2048                    539     477
 //
 // The folding form has 256-wide tiles only; as halves (128) they pay while
 // all of them run at once with SMs to spare: 1024^3 23.4 against 31.8 us,
 // 1280^3 26.6 / 37.7, 1500^3 (144 halves on 152 SMs) 45.2 / 46.4, 3000x700x1000
-// 38.8 / 37.9.
-static int tile_width(const GemmArgs &g, int np, bool fold) {
+// 38.8 / 37.9.  Its pairs pay over several waves of a long K (BF16, chunks of
+// 1024: 4096^3 286 -> 263, 2500^3 99.7 -> 91.4; but 2048^3, one wave, 56.9 -> 58.3
+// and 3500x2900x700 60.7 -> 63.4).  FP16 pieces keep one CTA: 4096^3 350 against
+// 346, but 8192x8192x2048 700 against 733.
+static int tile_width(const GemmArgs &g, int np, bool f16, int fold_kb, bool &pair) {
+    pair = false;
     if (np == 3) return 128;
     const double sms = sm_count(), kb = (double)ceil_div(g.K, KB);
     auto waves = [&](int bn) { return (double)ceil_div(g.M, BM) * (double)ceil_div(g.N, bn) / sms; };
-    if (fold) return 2.0 * waves(256) <= 0.9 ? 128 : 256;
+    if (f16 || fold_kb > 0) {
+        pair = !f16 && fold_kb % 2 == 0 && g.K > 1024 && waves(256) > 1.0;
+        return 2.0 * waves(256) <= 0.9 ? 128 : 256;
+    }
     const double whole = floor(waves(256)), rest = waves(256) - whole;
+    const double pairs = (double)ceil_div(g.M, 2 * BM) * (double)ceil_div(g.N, 256) / floor(0.5 * sms);
     const double t64 = 7.0 + ceil(waves(64)) * kb * 0.27, t128 = 8.0 + ceil(waves(128)) * kb * 0.315,
-                 t256 = 12.0 + (whole + (rest == 0.0 ? 0.0 : whole > 0.0 && rest <= 0.5 ? 0.5 : 1.0)) * kb * 0.60;
-    return t64 < t128 && t64 < t256 ? 64 : t128 < t256 ? 128 : 256;
+                 t256 = 12.0 + (whole + (rest == 0.0 ? 0.0 : whole > 0.0 && rest <= 0.5 ? 0.5 : 1.0)) * kb * 0.60,
+                 tpair = g.M > BM ? 12.0 + ceil(pairs) * kb * 0.53 : 1e30;
+    const double wide = t256 < tpair ? t256 : tpair;
+    if (t64 < t128 && t64 < wide) return 64;
+    if (t128 < wide) return 128;
+    pair = tpair < t256;
+    return 256;
 }
 
 // Split pass (NP 16-bit pieces per operand, K-major) + MMA kernel; fold_kb >
@@ -1711,8 +1783,9 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
         GB_LAUNCH_CHECK("bf16x3 split");
     }
 
-    const int bn = tile_width(g, np, fold_kb > 0 || f16);
-    const int bk = block_k(np, fold_kb > 0 || f16, fold_kb, bn);
+    bool pair;   // 256 x 256 tiles of two CTAs
+    const int bn = tile_width(g, np, f16, fold_kb, pair);
+    const int bk = block_k(np, fold_kb > 0 || f16, fold_kb, bn, pair);
     const int box = np == 2 && (fold_kb > 0 || f16) ? 256 : bn;   // rows of a B box (the halves have half boxes)
     PieceMaps maps;
     memset(&maps, 0, sizeof(maps));
@@ -1738,8 +1811,8 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     }
     int grid = 0;
     const bool dependent = pdl_env && !capturing;
-    gb_status s = f16 ? gemm_launch<true>(g, np, fold_kb, maps, kp, p, bn, dependent, &grid)
-                      : gemm_launch<false>(g, np, fold_kb, maps, kp, p, bn, dependent, &grid);
+    gb_status s = f16 ? gemm_launch<true>(g, np, fold_kb, maps, kp, p, bn, pair, dependent, &grid)
+                      : gemm_launch<false>(g, np, fold_kb, maps, kp, p, bn, pair, dependent, &grid);
     if (s != GB_OK) return s;
     if (done) st.launched += (unsigned long long)grid;
     st.valid = done != nullptr;
