@@ -522,6 +522,8 @@ struct EpiParams {
     int semantics;
     int num_kb;
     int tiles_m, tiles_n;
+    int parts;       // CTAs that share a tile's k-blocks; > 1: their sums go to C + part * part_stride
+    int64_t part_stride;
     int *err;
     int chunk_kb;    // k-blocks per accumulator chunk (folding form)
     // Half-tile tail: tiles [half_start, tiles) (a last wave at most half
@@ -640,6 +642,9 @@ __device__ __forceinline__ int64_t tile_row0(int tm) {
 // its 128 rows of A, half of B's and its 128 rows of the accumulators.
 // The MMAs of chunk c+1 overlap the fold of chunk c.
 // F16: FP16 pieces of scaled lines (FP16X3), the epilogue applies the scales.
+// First k-block of part j of a tile.
+__device__ __forceinline__ int part_kb(int num_kb, int parts, int j) { return num_kb * j / parts; }
+
 template <int NP, int BN, bool FOLD, bool F16, int EW, int BK, int CG>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
     bf16x3_gemm_kernel(const __grid_constant__ PieceMaps maps, EpiParams p) {
@@ -666,7 +671,9 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
     int *row_scale = col_scale + 8 * 128;                                                     // [8][32]
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int num_tiles = p.tiles_m * p.tiles_n;
+    constexpr bool PARTS = !FOLD && NP == 2 && CG == 1;   // forms whose tiles may be shared
+    const int parts = PARTS ? p.parts : 1;
+    const int num_tiles = p.tiles_m * p.tiles_n * parts;
     const int chunk_kb = FOLD ? p.chunk_kb : p.num_kb;
 
     if (threadIdx.x == 0) {
@@ -705,11 +712,12 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
             int it = 0, t, half;
             while (go && next_item<CG>(p, num_tiles, it, t, half)) {
                 int tm, tn;
-                tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+                tile_coords(t / parts, p.tiles_m, p.tiles_n, tm, tn);
                 const int rank = CG == 2 ? (int)ptx::cluster_ctarank() : 0;
                 const int m0 = (tm * CG + rank) * BM, n0 = tn * BN + (half > 0 || rank ? BN / 2 : 0);
                 const uint32_t bytes = half < 0 ? CG * STAGE_BYTES : NP * A_TILE + NP * (B_TILE / 2);
-                for (int kb = 0; kb < p.num_kb; kb++, kbg++) {
+                const int kb1 = part_kb(p.num_kb, parts, t % parts + 1);
+                for (int kb = part_kb(p.num_kb, parts, t % parts); kb < kb1; kb++, kbg++) {
                     const int s = kbg % STAGES;
                     if (kbg >= STAGES && !ptx::mbar_wait(&empty[s], ((kbg / STAGES) & 1) ^ 1, p.err, 1)) {
                         go = false;
@@ -759,8 +767,9 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                     ptx::tc_fence_after();
                     const uint32_t acc = tmem + (uint32_t)(b * ACC_COLS);
                     const uint32_t acc_lo = SEP ? acc + 128u : acc;   // cross products
-                    const int kbc = c * chunk_kb;
-                    const int kb1 = kbc + chunk_kb < p.num_kb ? kbc + chunk_kb : p.num_kb;
+                    const int kbc = PARTS ? part_kb(p.num_kb, parts, t % parts) : c * chunk_kb;
+                    const int kb1 = PARTS ? part_kb(p.num_kb, parts, t % parts + 1)
+                                          : kbc + chunk_kb < p.num_kb ? kbc + chunk_kb : p.num_kb;
                     for (int kb = kbc; kb < kb1; kb++, kbg++) {
                         const int s = kbg % STAGES;
                         if (!ptx::mbar_wait(&full[s], (kbg / STAGES) & 1, p.err, 3)) { go = false; break; }
@@ -808,7 +817,8 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
         int it = 0, t, half;
         while (go && next_item<CG>(p, num_tiles, it, t, half)) {
             int tm, tn;
-            tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+            tile_coords(t / parts, p.tiles_m, p.tiles_n, tm, tn);
+            float *const C = p.C + (int64_t)(t % parts) * p.part_stride;
             const int64_t row0 = tile_row0<CG>(tm) + q * 32;
             const int64_t n0 = (int64_t)tn * BN + (half > 0 ? BN / 2 : 0);
             const int ncols = half < 0 ? BN : BN / 2;
@@ -864,15 +874,15 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
                     if (!reads_c(p)) {
                         const float add = p.semantics == GB_SEM_SCALAR_BETA ? p.beta : 0.f;
                         for (int rr = 0; rr < rows; rr++)
-                            p.C[(row0 + rr) * p.ldc + col] = p.alpha * stage[rr * 33 + lane] + add;
+                            C[(row0 + rr) * p.ldc + col] = p.alpha * stage[rr * 33 + lane] + add;
                     } else {
                         float cin[32];
 #pragma unroll
                         for (int rr = 0; rr < 32; rr++)
-                            cin[rr] = rr < rows ? p.C[(row0 + rr) * p.ldc + col] : 0.f;
+                            cin[rr] = rr < rows ? C[(row0 + rr) * p.ldc + col] : 0.f;
 #pragma unroll
                         for (int rr = 0; rr < 32; rr++)
-                            if (rr < rows) p.C[(row0 + rr) * p.ldc + col] = epi_value(p, stage[rr * 33 + lane], cin[rr]);
+                            if (rr < rows) C[(row0 + rr) * p.ldc + col] = epi_value(p, stage[rr * 33 + lane], cin[rr]);
                     }
                 }
                 __syncwarp();
@@ -1065,6 +1075,26 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
         else ptx::tmem_dealloc(tmem, TMEM_COLS);
     }
     if (threadIdx.x == 0 && p.done) atomicAdd(p.done, 1ull);   // last: this CTA is done
+}
+
+// C from the parts' sums, added in order of K (round to nearest), with the epilogue.
+// Bound by reading them: a column per thread, four rows' loads in flight.
+__global__ void __launch_bounds__(256)
+    parts_join_kernel(const float *__restrict__ sums, int64_t lds, int64_t stride, int parts, EpiParams p) {
+    const int64_t col = (int64_t)blockIdx.x * 64 + threadIdx.x % 64, row0 = (int64_t)blockIdx.y * 16 + threadIdx.x / 64;
+    if (col >= p.N) return;
+    const bool rc = reads_c(p);
+    float x[4] = {0.f, 0.f, 0.f, 0.f}, c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (rc && row0 + 4 * i < p.M) c[i] = p.C[(row0 + 4 * i) * p.ldc + col];
+    for (int j = 0; j < parts; j++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (row0 + 4 * i < p.M) x[i] += __ldcg(sums + j * stride + (row0 + 4 * i) * lds + col);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (row0 + 4 * i < p.M) p.C[(row0 + 4 * i) * p.ldc + col] = epi_value(p, x[i], c[i]);
 }
 
 // ============================================================ fused split
@@ -1516,7 +1546,7 @@ static gb_status two_pass_launch(const GemmArgs &g, const PieceMaps &maps, int64
         device_setup_done(attr);
     }
     const int tiles_m = (int)ceil_div(g.M, CG * BM), tiles_n = (int)ceil_div(g.N, BN);
-    const int tiles = tiles_m * tiles_n;
+    const int tiles = tiles_m * tiles_n * base.parts;
     const bool halves = bn < BN;
     const int64_t items = halves ? 2 * (int64_t)tiles : tiles;
     const int grid = CG * (int)std::min<int64_t>(items, sm_count() / CG);
@@ -1613,6 +1643,11 @@ static gb_status gemm_launch(const GemmArgs &g, int np, int fold_kb, const Piece
 //   4096x2048x1000                    61.1    55.5
 //   8192x8192x2048                    539     477
 //
+// Shared tiles: 256x256x4096 39.1 -> 18.5 us (64 columns, eight parts), 300x400x4000
+// 38.9 -> 20.6, 512x512x4096 39.6 -> 24.0 (128, eight), 400x400x1500 19.4 -> 16.5 (64,
+// three), 800x800x3000 31.7 -> 28.7; but 1000x1000x4000 42.4 -> 43.4.  Shorter sums are
+// also the more exact ones (4.1e-6 against 1.4e-5 at K = 4000).
+//
 // The folding form has 256-wide tiles only; as halves (128) they pay while
 // all of them run at once with SMs to spare: 1024^3 23.4 against 31.8 us,
 // 1280^3 26.6 / 37.7, 1500^3 (144 halves on 152 SMs) 45.2 / 46.4, 3000x700x1000
@@ -1620,8 +1655,9 @@ static gb_status gemm_launch(const GemmArgs &g, int np, int fold_kb, const Piece
 // 1024: 4096^3 286 -> 263, 2500^3 99.7 -> 91.4; but 2048^3, one wave, 56.9 -> 58.3
 // and 3500x2900x700 60.7 -> 63.4).  FP16 pieces keep one CTA: 4096^3 350 against
 // 346, but 8192x8192x2048 700 against 733.
-static int tile_width(const GemmArgs &g, int np, bool f16, int fold_kb, bool &pair) {
+static int tile_width(const GemmArgs &g, int np, bool f16, int fold_kb, bool &pair, int &parts) {
     pair = false;
+    parts = 1;
     if (np == 3) return 128;
     const double sms = sm_count(), kb = (double)ceil_div(g.K, KB);
     auto waves = [&](int bn) { return (double)ceil_div(g.M, BM) * (double)ceil_div(g.N, bn) / sms; };
@@ -1635,6 +1671,20 @@ static int tile_width(const GemmArgs &g, int np, bool f16, int fold_kb, bool &pa
                  t256 = 12.0 + (whole + (rest == 0.0 ? 0.0 : whole > 0.0 && rest <= 0.5 ? 0.5 : 1.0)) * kb * 0.60,
                  tpair = g.M > BM ? 12.0 + ceil(pairs) * kb * 0.53 : 1e30;
     const double wide = t256 < tpair ? t256 : tpair;
+    // tiles that leave SMs idle: `parts` CTAs share a tile's k-blocks, each with sums of its own that
+    // a join launch adds up (6 us with the overlap that it ends, and their bytes through the L2; a
+    // tenth to be gained at least).  The sums take no more workspace than a third piece would.
+    double best = 0.9 * std::min(std::min(t64, t128), wide);
+    int bn = 0;
+    const double room = (double)(g.M + g.N) * 2.0 * 64.0 * (double)ceil_div(g.K, 64);
+    const double part_bytes = 4.0 * (double)g.M * (double)(ceil_div(g.N, 4) * 4);
+    for (int w : {64, 128})
+        for (int n = 2; n <= 16 && 2.0 * n <= kb && n * part_bytes <= room; n++) {
+            const double t = 14.0 + ceil(waves(w) * n) * 2.0 * ceil(0.5 * kb / n) * (w == 64 ? 0.27 : 0.315) +
+                             2.0 * n * part_bytes / 4e6;
+            if (t < best) { best = t; parts = n; bn = w; }
+        }
+    if (bn) return bn;
     if (t64 < t128 && t64 < wide) return 64;
     if (t128 < wide) return 128;
     pair = tpair < t256;
@@ -1649,7 +1699,11 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     const int64_t kp = ceil_div(g.K, 64) * 64;   // a multiple of either k-block, zero-padded
     const size_t a_bytes = (size_t)g.M * kp * 2, b_bytes = (size_t)g.N * kp * 2;
     const size_t piece_bytes = (np * (a_bytes + b_bytes) + 255) / 256 * 256;
-    const size_t pieces = piece_bytes;
+    bool pair;   // 256 x 256 tiles of two CTAs
+    int parts;   // CTAs that share a tile's k-blocks
+    const int bn = tile_width(g, np, f16, fold_kb, pair, parts);
+    const int64_t lds = ceil_div(g.N, 4) * 4;   // the parts' sums follow the pieces
+    const size_t pieces = piece_bytes + (parts > 1 ? ((size_t)parts * g.M * lds * 4 + 255) / 256 * 256 : 0);
     // The buffer is [half 0 | half 1], the same for every call of any form (the halves move only
     // when the buffer grows, which first drains its stream).  Calls alternate between the halves,
     // so a split may run beside the previous GEMM; one half when two do not fit in 16 GiB.
@@ -1783,8 +1837,6 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
         GB_LAUNCH_CHECK("bf16x3 split");
     }
 
-    bool pair;   // 256 x 256 tiles of two CTAs
-    const int bn = tile_width(g, np, f16, fold_kb, pair);
     const int bk = block_k(np, fold_kb > 0 || f16, fold_kb, bn, pair);
     const int box = np == 2 && (fold_kb > 0 || f16) ? 256 : bn;   // rows of a B box (the halves have half boxes)
     PieceMaps maps;
@@ -1809,11 +1861,23 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
         p.lda = g.lda; p.ldb = g.ldb; p.K = g.K;
         p.ta = g.ta ? 1 : 0; p.tb = g.tb ? 1 : 0;
     }
+    p.parts = parts;
+    const EpiParams final = p;
+    float *const sums = (float *)(pw + piece_bytes);
+    if (parts > 1) {   // each part's plain sums
+        p.C = sums; p.ldc = lds; p.part_stride = g.M * lds;
+        p.alpha = 1.f; p.beta = 0.f; p.semantics = GB_SEM_BLAS;
+    }
     int grid = 0;
     const bool dependent = pdl_env && !capturing;
     gb_status s = f16 ? gemm_launch<true>(g, np, fold_kb, maps, kp, p, bn, pair, dependent, &grid)
                       : gemm_launch<false>(g, np, fold_kb, maps, kp, p, bn, pair, dependent, &grid);
     if (s != GB_OK) return s;
+    if (parts > 1) {   // launched in plain stream order: the next call's split starts after it
+        const dim3 jg((unsigned)ceil_div(g.N, 64), (unsigned)ceil_div(g.M, 16));
+        parts_join_kernel<<<jg, 256, 0, g.stream>>>(sums, lds, g.M * lds, parts, final);
+        GB_LAUNCH_CHECK("parts_join_kernel");
+    }
     if (done) st.launched += (unsigned long long)grid;
     st.valid = done != nullptr;
     st.c_lo = clo;
