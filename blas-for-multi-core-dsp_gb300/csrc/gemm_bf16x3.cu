@@ -623,6 +623,12 @@ __device__ __forceinline__ int64_t tile_row0(int tm) {
     return ((int64_t)tm * CG + (CG == 2 ? ptx::cluster_ctarank() : 0u)) * BM;
 }
 
+// Last group of 8 columns whose C is loaded before group g is stored (direct store): one ahead
+// at first, and two steps at a time once four stored groups have freed their totals' registers.
+// 4096^3 with leading dimension 4112: 351 us a call against 359 for one ahead throughout; more
+// at an earlier group spills.
+__host__ __device__ constexpr int c_ahead(int g) { return g < 0 ? 0 : g < 4 ? g + 1 : 2 * g - 2; }
+
 // FOLD: the tensor cores add each MMA into the FP32 accumulator with an
 // error of about one unit in the last place of the accumulator, biased like
 // a truncation, so over a long K the error grows with the number of MMAs and
@@ -957,7 +963,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
             const int *cs_w = col_scale + wi * 128;
             const int *rs_w = row_scale + wi * 32;
             // Direct store (FP16 pieces): lane l writes its row's 128 columns as 16-byte vectors,
-            // the C loads one group of 8 columns ahead.  Taken when the 128 columns are inside C,
+            // the C loads ahead by groups of 8 columns (c_ahead).  Taken when the 128 columns are inside C,
             // the rows' starts 16-byte aligned and every scale 2^-(row + column scale) a normal
             // float; else the store through shared memory below.  (The BF16 folding form keeps
             // the shared-memory store: with C read, the direct store measured 0.56 ms against
@@ -979,18 +985,23 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1)
             if (__all_sync(0xffffffffu, fast)) {
                 const bool rc = reads_c(p), rowok = row0 + lane < p.M;
                 float *crow = p.C + (row0 + lane) * p.ldc + c0;
-                float4 cn0 = make_float4(0.f, 0.f, 0.f, 0.f), cn1 = cn0;
+                float4 cn[16][2];
+#pragma unroll
+                for (int g = 0; g < 16; g++) cn[g][0] = cn[g][1] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (rc && rowok) {
-                    cn0 = ldg_v4(crow);
-                    cn1 = ldg_v4(crow + 4);
+                    cn[0][0] = ldg_v4(crow);
+                    cn[0][1] = ldg_v4(crow + 4);
                 }
 #pragma unroll
                 for (int g = 0; g < 16; g++) {
-                    const float cc[8] = {cn0.x, cn0.y, cn0.z, cn0.w, cn1.x, cn1.y, cn1.z, cn1.w};
-                    if (g + 1 < 16 && rc && rowok) {   // issued before this group's stores (ordered asm)
-                        cn0 = ldg_v4(crow + 8 * (g + 1));
-                        cn1 = ldg_v4(crow + 8 * (g + 1) + 4);
-                    }
+#pragma unroll
+                    for (int h = c_ahead(g - 1) + 1; h <= c_ahead(g); h++)   // issued before this group's stores (ordered asm)
+                        if (h < 16 && rc && rowok) {
+                            cn[h][0] = ldg_v4(crow + 8 * h);
+                            cn[h][1] = ldg_v4(crow + 8 * h + 4);
+                        }
+                    const float cc[8] = {cn[g][0].x, cn[g][0].y, cn[g][0].z, cn[g][0].w,
+                                         cn[g][1].x, cn[g][1].y, cn[g][1].z, cn[g][1].w};
                     float *o = total + 8 * g;   // the outputs replace their totals
                     if (F16) {
                         const int4 s0 = *reinterpret_cast<const int4 *>(cs_w + 8 * g);
