@@ -127,7 +127,8 @@ __global__ void __launch_bounds__(NT) stencil_tb_kernel(const T *__restrict__ sr
 // (a warp alone on a scheduler would otherwise wait for L2 at every row).
 // Only warps whose window touches the grid's boundary (EDGE) test for fixed
 // cells.
-constexpr int RS_W = 128, RS_T = 6, RS_U = 4, RS_WARPS = 16;   // strip, most sweeps a pass, rows unrolled, warps an SM holds
+constexpr int RS_W = 128, RS_T = 6, RS_TLAST = 8, RS_U = 4;   // strip, most sweeps a pass, and of an odd last one, rows unrolled
+constexpr int RS_WARPS = 16;   // warps an SM holds
 
 template <int ORDER, int PAR>
 __device__ __forceinline__ uint64_t update2(uint64_t top, uint64_t left, uint64_t right, uint64_t down, uint64_t mid,
@@ -256,7 +257,7 @@ __device__ __forceinline__ void rs_walk(const float *__restrict__ src, float *__
 // launched as a programmatic dependent: its launch overlaps the pass before,
 // whose rows it waits for here.
 template <int T, int ORDER>
-__global__ void __launch_bounds__(32, RS_WARPS) stencil_rs_kernel(const float *__restrict__ src,
+__global__ void __launch_bounds__(32, T > RS_T ? 12 : RS_WARPS) stencil_rs_kernel(const float *__restrict__ src,
                                                                   float *__restrict__ dst, int64_t M, int64_t N,
                                                                   int strips, int seg) {
     ptx::pdl_wait();   // returns at once when not launched as a dependent
@@ -453,13 +454,13 @@ gb_status stencil9(int64_t M, int64_t N, E *A, E *B, int iters, const E *w_host,
 struct RsPlan {
     int launches, seg;
 };
-RsPlan rs_plan(int64_t M, int64_t N, int iters) {
+RsPlan rs_plan(int64_t M, int64_t N, int iters, int parity) {
     RsPlan best{1, 8};
     double best_cost = 1e300;
     const double sched = 4.0 * sm_count(), wave = (double)RS_WARPS * sm_count();
     for (int t = RS_T < iters ? RS_T : iters; t >= 1; t--) {
         int launches = (int)ceil_div(iters, t);
-        if ((launches & 1) != (iters & 1)) launches++;   // the result lands in B for odd iters, in A for even
+        if ((launches & 1) != parity) launches++;   // the result lands in B for odd iters, in A for even
         const int tt = (int)ceil_div(iters, launches);
         const double strips = (double)ceil_div(N, RS_W - 2 * tt);
         for (int seg = 8; seg <= 256; seg += seg < 64 ? 4 : 8) {
@@ -488,13 +489,23 @@ gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *
     cudaStream_t st = as_stream(stream);
     if (sizeof(T) == 4) {
         GB_CHECK_ARG(ceil_div(M, 64) <= 65535, "stencil2d: M too large");
-        const RsPlan pl = rs_plan(M, N, iters);
+        // An odd number of sweeps ends with a pass of up to eight of its own: it leaves in A the
+        // sweep that an even spread of passes of at most eight does, which is what a caller that
+        // passes the same A again starts from.  The passes before it are as for an even number.
+        int last = 0;
+        if (iters & 1) {
+            const int passes = (int)ceil_div(iters, RS_TLAST);
+            last = iters / (passes + 1 - (passes & 1));
+        }
+        const int rest = iters - last;
+        RsPlan pl = rs_plan(M, N, rest > 0 ? rest : last, rest > 0 ? 0 : 1);
+        if (rest == 0) pl.launches = 0;
         // captured launches keep plain stream order
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         GB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
         int done = 0;
-        for (int l = 0; l < pl.launches; l++) {
-            const int t = (int)ceil_div(iters - done, pl.launches - l);   // spread evenly
+        for (int l = 0; l < pl.launches + (last > 0); l++) {
+            const int t = l < pl.launches ? (int)ceil_div(rest - done, pl.launches - l) : last;   // spread evenly
             const float *src = (const float *)(l % 2 == 0 ? A : B);
             float *dst = (float *)(l % 2 == 0 ? B : A);
             const bool dep = l > 0 && cap == cudaStreamCaptureStatusNone;
@@ -505,7 +516,9 @@ gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *
                 case 3: e = launch_rs<3>(src, dst, M, N, pl.seg, order, dep, st); break;
                 case 4: e = launch_rs<4>(src, dst, M, N, pl.seg, order, dep, st); break;
                 case 5: e = launch_rs<5>(src, dst, M, N, pl.seg, order, dep, st); break;
-                default: e = launch_rs<RS_T>(src, dst, M, N, pl.seg, order, dep, st); break;
+                case 6: e = launch_rs<6>(src, dst, M, N, pl.seg, order, dep, st); break;
+                case 7: e = launch_rs<7>(src, dst, M, N, pl.seg, order, dep, st); break;
+                default: e = launch_rs<RS_TLAST>(src, dst, M, N, pl.seg, order, dep, st); break;
             }
             GB_CUDA_TRY(e);
             GB_LAUNCH_CHECK("stencil_rs_kernel");
