@@ -647,17 +647,28 @@ gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
         pl.rtiles = ceil_div(p.rows, 128) + (classes ? 3 : 0);
         const int64_t nst = thin_tc_stages(p.K, classes);
         const int64_t sms = sm_count();
-        const bool equal = p.want_splits <= 0 && !p.tx && pl.rtiles < 4 * sms && pl.rtiles * nst >= 16 * sms;
-        const int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst, 8);
+        // sums of at most the K range that a split into four waves of units would leave
+        int64_t ranges = 1;
+        while (pl.rtiles * ranges < 4 * sms && nst / (ranges * 2) >= 8 && ranges < 64) ranges *= 2;
+        pl.fold = (int)ceil_div(nst, ranges);
+        // equal parts cut the ranges anywhere, so not the long ones (20011 x 6007, n 33: 107 against
+        // 125 us; but 33440 x 32109, n 34: 810 against 758)
+        const bool equal = p.want_splits <= 0 && !p.tx && pl.rtiles < 4 * sms && pl.rtiles * nst >= 16 * sms &&
+                           64 * pl.fold <= 6144;
+        // an accumulator's error grows with its range, about 6.4e-9 of the result a k: another split may
+        // change the ranges' mean length (weighted by themselves) by 1536 k, 1e-5, for a fuller last
+        // wave, no more
+        int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst, 8);
+        if (p.want_splits <= 0 && !equal) {
+            const double len = (double)ceil_div(nst, want), whole = floor(len / pl.fold), rem = len - whole * pl.fold;
+            const double mean = (whole * pl.fold * pl.fold + rem * rem) / len;
+            if (64.0 * (pl.fold - mean) > 1536.0) want = ranges;
+        }
         const int64_t cst = ceil_div(nst, want);
         p.kchunk = cst * 64;
         p.splits = (int)ceil_div(nst, cst);
         if (p.splits < 1) p.splits = 1;
         pl.parts = equal ? (int)sms : 0;
-        // sums of at most the K range that a split into four waves of units would leave
-        int64_t ranges = 1;
-        while (pl.rtiles * ranges < 4 * (int64_t)sm_count() && nst / (ranges * 2) >= 8 && ranges < 64) ranges *= 2;
-        pl.fold = (int)ceil_div(nst, ranges);
         pl.part_bytes = pl.parts > 0 ? (size_t)2 * pl.parts * 128 * NB * sizeof(T)
                         : p.splits > 1 ? (size_t)p.splits * p.rows * NB * sizeof(T) : 0;
         pl.w_bytes = thin_tc_wpieces_bytes(NB, p.K, classes);
