@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(NT) stencil_tb_kernel(const T *__restrict__ sr
 // (a warp alone on a scheduler would otherwise wait for L2 at every row).
 // Only warps whose window touches the grid's boundary (EDGE) test for fixed
 // cells.
-constexpr int RS_W = 128, RS_T = 6, RS_TLAST = 8, RS_U = 4;   // strip, most sweeps a pass, and of an odd last one, rows unrolled
+constexpr int RS_W = 128, RS_T = 6, RS_U = 4;   // strip, most sweeps a pass, rows unrolled
 constexpr int RS_WARPS = 16;   // warps an SM holds
 
 template <int ORDER, int PAR>
@@ -489,12 +489,13 @@ gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *
     cudaStream_t st = as_stream(stream);
     if (sizeof(T) == 4) {
         GB_CHECK_ARG(ceil_div(M, 64) <= 65535, "stencil2d: M too large");
-        // An odd number of sweeps ends with a pass of up to eight of its own: it leaves in A the
-        // sweep that an even spread of passes of at most eight does, which is what a caller that
-        // passes the same A again starts from.  The passes before it are as for an even number.
+        // An odd number of sweeps ends with a pass of its own: it leaves in A the sweep that an even
+        // spread over an odd number of passes of at most eight does (seven at the end at most), which
+        // is what a caller that passes the same A again starts from.  The passes before it are as for
+        // an even number.
         int last = 0;
         if (iters & 1) {
-            const int passes = (int)ceil_div(iters, RS_TLAST);
+            const int passes = (int)ceil_div(iters, 8);
             last = iters / (passes + 1 - (passes & 1));
         }
         const int rest = iters - last;
@@ -517,8 +518,7 @@ gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *
                 case 4: e = launch_rs<4>(src, dst, M, N, pl.seg, order, dep, st); break;
                 case 5: e = launch_rs<5>(src, dst, M, N, pl.seg, order, dep, st); break;
                 case 6: e = launch_rs<6>(src, dst, M, N, pl.seg, order, dep, st); break;
-                case 7: e = launch_rs<7>(src, dst, M, N, pl.seg, order, dep, st); break;
-                default: e = launch_rs<RS_TLAST>(src, dst, M, N, pl.seg, order, dep, st); break;
+                default: e = launch_rs<7>(src, dst, M, N, pl.seg, order, dep, st); break;
             }
             GB_CUDA_TRY(e);
             GB_LAUNCH_CHECK("stencil_rs_kernel");
