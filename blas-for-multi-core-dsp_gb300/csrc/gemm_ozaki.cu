@@ -368,7 +368,7 @@ __device__ __forceinline__ void store_outputs(const OzParams &p, int64_t row, in
     for (int j = 0; j < 8; j++) {
         const int64_t col = col0 + j;
         if (!rowok || col >= p.N) continue;
-        const int fc = __ldg(p.fcol + col);
+        const int fc = ptx::ld_after_wait(p.fcol + col);
         double v;
         if (fc == kNonFiniteLineExp || erow == kNonFiniteLineExp)
             v = p.alpha * native_dot_cold(p.A, p.lda, p.ta, row, p.B, p.ldb, p.tb, col, p.K);

@@ -618,20 +618,20 @@ __global__ void __launch_bounds__(NT, 1)
                         double *pp = p.part + ((int64_t)sp * p.rows + row) * p.pw;
 #pragma unroll
                         for (int j = 0; j < NG * NB; j++)
-                            if (j < p.n) pp[j] = scale_pow2(acc[j], er + __ldg(p.fcol + j));
+                            if (j < p.n) pp[j] = scale_pow2(acc[j], er + ptx::ld_after_wait(p.fcol + j));
                         if (nf) p.nfrow[row] = 1;
                     } else {
                         double *cr = p.C + row * p.cs_r;
 #pragma unroll
                         for (int j = 0; j < NG * NB; j++) {
                             if (j >= p.n) break;
-                            const int fc = __ldg(p.fcol + j);
+                            const int fc = ptx::ld_after_wait(p.fcol + j);
                             if (!nf && fc != kNonFiniteLineExp)
                                 store_out(p, cr + (int64_t)j * p.cs_c, scale_pow2(acc[j], er + fc));
                         }
 #pragma unroll 1
                         for (int j = 0; j < p.n; j++)   // a row or column that holds an Inf / NaN
-                            if (nf || __ldg(p.fcol + j) == kNonFiniteLineExp)
+                            if (nf || ptx::ld_after_wait(p.fcol + j) == kNonFiniteLineExp)
                                 store_out(p, cr + (int64_t)j * p.cs_c,
                                           native_dot(p.X, p.ldx, p.tx, row, p.W, p.ldw, p.tw, (int64_t)p.j0 + j, p.K));
                     }
@@ -745,7 +745,7 @@ __global__ void thin_oz_reduce_kernel(OzThinParams p) {
         const int64_t r = e / p.n;
         const int j = (int)(e - r * p.n);
         double s = 0.0;
-        if (p.nfrow[r] || __ldg(p.fcol + j) == kNonFiniteLineExp) {
+        if (p.nfrow[r] || ptx::ld_after_wait(p.fcol + j) == kNonFiniteLineExp) {
             s = native_dot(p.X, p.ldx, p.tx, r, p.W, p.ldw, p.tw, (int64_t)p.j0 + j, p.K);
         } else {
             for (int sp = 0; sp < p.splits; sp++) s += p.part[((int64_t)sp * p.rows + r) * p.pw + j];

@@ -35,6 +35,20 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // operations are visible.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Plain (coherent) loads of what a grid waited for by pdl_wait has written: that data is not
+// read-only for the lifetime of a grid that starts beside its writer, as ld.global.nc asks, and
+// the loads stay behind the wait.
+__device__ __forceinline__ float ld_after_wait(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ int ld_after_wait(const int *p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // ------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -181,10 +181,10 @@ __device__ __forceinline__ void rs_walk(const float *__restrict__ src, float *__
         if (EDGE) {
             const unsigned m = k >= klo && k < khi ? cload : 0u;
 #pragma unroll
-            for (int b = 0; b < 4; b++) x[b] = (m >> b) & 1u ? __ldg(pin + (b & 1) + 64 * (b >> 1)) : 0.f;
+            for (int b = 0; b < 4; b++) x[b] = (m >> b) & 1u ? ptx::ld_after_wait(pin + (b & 1) + 64 * (b >> 1)) : 0.f;
         } else if (k < kn) {
 #pragma unroll
-            for (int b = 0; b < 4; b++) x[b] = __ldg(pin + (b & 1) + 64 * (b >> 1));
+            for (int b = 0; b < 4; b++) x[b] = ptx::ld_after_wait(pin + (b & 1) + 64 * (b >> 1));
         }
         pin += ld;
     };
