@@ -44,6 +44,7 @@
 #include <vector>
 
 #include "gb_common.cuh"
+#include "piece_halves.h"
 #include "sm100_ptx.cuh"
 
 namespace gb {
@@ -1474,11 +1475,11 @@ gb_status launch_sgemm_fp16x3(const GemmArgs &g) {
 // ------------------------------------------------------------ stream state
 // Per (device, stream): a counter of finished GEMM CTAs (a slot of a static
 // device array, so tracking needs no allocation), how many CTAs the stream's
-// GEMMs launched so far, the byte range of the last GEMM's C and the
-// workspace half its pieces are in.  A split pass is launched beside the
-// previous GEMM only when that GEMM was this library's, this call's A and B
-// do not overlap its C, and the two halves fit; split_entry_guard covers
-// work the caller queued in between.
+// GEMMs launched so far, the byte range of the last GEMM's C and where in the
+// workspace its pieces are.  A split pass is launched beside the previous
+// GEMM only when that GEMM was this library's, this call's A and B do not
+// overlap its C, and the two calls' pieces lie apart (piece_halves.h);
+// split_entry_guard covers work the caller queued in between.
 constexpr int kDoneSlots = 1024;
 static __device__ unsigned long long g_gemm_done[kDoneSlots];
 static __device__ unsigned long long g_scan_done[kDoneSlots];   // finished FP16 scan CTAs
@@ -1490,7 +1491,7 @@ struct StreamState {
     unsigned long long launched; // CTAs of this stream's GEMMs launched so far
     bool valid;                  // the stream's last two-pass GEMM is known
     uintptr_t c_lo, c_hi;        // its C
-    unsigned parity;             // its workspace half
+    PieceRange pieces;           // its pieces (and parts' sums)
     unsigned long long scanned;  // CTAs of this stream's FP16 scans launched so far
     unsigned gen;                // generation of its last FP16 scan (captured scans use 1)
 };
@@ -1504,7 +1505,7 @@ static StreamState &stream_state(int dev, void *stream) {
         if (s.dev == dev && s.stream == stream) return s;
         if (s.dev == dev) used++;
     }
-    g_tp.push_back(StreamState{dev, stream, used < kDoneSlots ? used : -1, 0ull, false, 0, 0, 0u, 0ull, 1u});
+    g_tp.push_back(StreamState{dev, stream, used < kDoneSlots ? used : -1, 0ull, false, 0, 0, {0, 0, 0u}, 0ull, 1u});
     return g_tp.back();
 }
 
@@ -1715,9 +1716,7 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     const int bn = tile_width(g, np, f16, fold_kb, pair, parts);
     const int64_t lds = ceil_div(g.N, 4) * 4;   // the parts' sums follow the pieces
     const size_t pieces = piece_bytes + (parts > 1 ? ((size_t)parts * g.M * lds * 4 + 255) / 256 * 256 : 0);
-    // The buffer is [half 0 | half 1], the same for every call of any form (the halves move only
-    // when the buffer grows, which first drains its stream).  Calls alternate between the halves,
-    // so a split may run beside the previous GEMM; one half when two do not fit in 16 GiB.
+    // The buffer is [half 0 | half 1] (piece_halves.h); one half when two do not fit in 16 GiB.
     const char *pe = getenv("GB_BF16X3_PDL");
     const bool pdl_env = !(pe && pe[0] == '0');
     const size_t want = pieces <= (size_t(8) << 30) ? 2 * pieces : pieces;
@@ -1725,8 +1724,6 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     size_t ws_size = 0;
     uint8_t *ws = (uint8_t *)workspace(want, g.stream, &seq_unused, &ws_size);
     if (!ws) return (gb_status)gb_get_last_status();
-    const size_t half = ws_size / 2 / 256 * 256;
-    const bool two_halves = half >= pieces;
     // FP16 form: the line maxima, [half 0 | half 1] of lm_cap entries, in a buffer of their own
     unsigned long long *lm_base = nullptr;
     size_t lm_cap = 0;
@@ -1763,16 +1760,16 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     span(g.A, g.ta, g.M, g.K, g.lda, 4, alo, ahi);
     span(g.B, g.tb, g.K, g.N, g.ldb, 4, blo, bhi);
     span(g.C, false, g.M, g.N, g.ldc, 4, clo, chi);
-    const bool pdl = pdl_env && two_halves && done != nullptr && st.valid &&
+    const PiecePlace place = place_pieces(st.pieces, pieces, ws_size);
+    const bool pdl = pdl_env && place.apart && done != nullptr && st.valid &&
                      (ahi <= st.c_lo || alo >= st.c_hi) && (bhi <= st.c_lo || blo >= st.c_hi);
-    const unsigned parity = two_halves ? (st.parity ^ 1u) : 0u;
-    uint8_t *pw = ws + (size_t)parity * half;
+    uint8_t *pw = ws + place.at.lo;
     uint16_t *ap[3], *bp[3];
     for (int i = 0; i < np; i++) {
         ap[i] = (uint16_t *)(pw + i * a_bytes);
         bp[i] = (uint16_t *)(pw + np * a_bytes + i * b_bytes);
     }
-    unsigned long long *bits = f16 ? lm_base + (size_t)parity * lm_cap : nullptr;   // op(A) rows, op(B) columns
+    unsigned long long *bits = f16 ? lm_base + (size_t)place.at.parity * lm_cap : nullptr;   // op(A) rows, op(B) columns
     const unsigned long long *gdone = pdl ? done : nullptr;
     const unsigned long long expect = st.launched;
     unsigned long long *scan_done = f16 && done ? scan_counter(dev, st.slot) : nullptr;
@@ -1893,7 +1890,7 @@ static gb_status two_pass(const GemmArgs &g, int np, int fold_kb, bool f16) {
     st.valid = done != nullptr;
     st.c_lo = clo;
     st.c_hi = chi;
-    st.parity = parity;
+    st.pieces = place.at;
     return ok();
 }
 
