@@ -1674,7 +1674,7 @@ static int tile_width(const GemmArgs &g, int np, bool f16, int fold_kb, bool &pa
     const double sms = sm_count(), kb = (double)ceil_div(g.K, KB);
     auto waves = [&](int bn) { return (double)ceil_div(g.M, BM) * (double)ceil_div(g.N, bn) / sms; };
     if (f16 || fold_kb > 0) {
-        pair = !f16 && fold_kb % 2 == 0 && g.K > 1024 && waves(256) > 1.0;
+        pair = !f16 && sms >= 2.0 && fold_kb % 2 == 0 && g.K > 1024 && waves(256) > 1.0;   // a pair takes two SMs
         return 2.0 * waves(256) <= 0.9 ? 128 : 256;
     }
     const double whole = floor(waves(256)), rest = waves(256) - whole;
