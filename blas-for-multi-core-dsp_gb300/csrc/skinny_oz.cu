@@ -759,7 +759,7 @@ __global__ void thin_oz_reduce_kernel(OzThinParams p) {
 // and u = 1..8 (the least significant digit first, the pass's columns within
 // a digit), K-major, kp columns, zero beyond n and K.
 __global__ void wdigits_kernel(const double *__restrict__ W, int64_t ldw, int tw, int n, int j0, int pw, int64_t K,
-                               int64_t kp, const int *__restrict__ fcol, unsigned short *__restrict__ out) {
+                               int64_t kp, const int *fcol, unsigned short *__restrict__ out) {
     ptx::pdl_wait();   // the exponents; an earlier pass's reads of `out`
     const int64_t total = (int64_t)pw * kp;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
@@ -771,7 +771,7 @@ __global__ void wdigits_kernel(const double *__restrict__ W, int64_t ldw, int tw
         int f = 0;
         if (j < n && k < K) {
             x = tw ? W[(int64_t)j * ldw + k] : W[k * ldw + j];
-            f = fcol[jp];
+            f = ptx::ld_after_wait(fcol + jp);
         }
         uint32_t sg;
         const uint64_t F = scaled_mantissa(x, f, sg);
