@@ -50,11 +50,14 @@
 // normwise bound.  An output whose row of X or column of W holds an Inf or a
 // NaN is recomputed as a plain FP64 dot product, so non-finite values
 // propagate.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 
 #include "gb_common.cuh"
 #include "sm100_ptx.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace gb {
 
@@ -77,6 +80,7 @@ constexpr uint32_t TMEM_COLS = 512;
 constexpr int XS = BM * KB * 8;             // 32 KB: two 16-k boxes of FP64
 constexpr int BAR_BYTES = 512, EXP_BYTES = 2 * BM * 4;
 constexpr int NO_EXP = -100000;             // chunk exponent of an all-zero row chunk
+constexpr int64_t WEXP_K = 32768;           // values of a column of W for one CTA (wexp_kernel)
 
 // NG groups of 16 columns of W per pass.  NG = 1: two level sets alternate per
 // chunk (tensor memory: 2 x 128 level columns + 2 x 128 digit-slot columns);
@@ -708,31 +712,59 @@ __global__ void __launch_bounds__(NT, 1)
     }
 }
 
-// Exponents of W's columns (logical K x n; tw: stored n x K), a CTA each.  The
-// digits' kernel may be launched beside this one.
-__global__ void __launch_bounds__(512) wexp_kernel(const double *__restrict__ W, int64_t ldw, int tw, int64_t K,
-                                                   int *__restrict__ fcol) {
-    __shared__ unsigned long long red[16];
-    const unsigned long long *w = reinterpret_cast<const unsigned long long *>(W) + (tw ? blockIdx.x * ldw : blockIdx.x);
-    const int64_t step = tw ? 1 : ldw;
+// Exponents of W's columns (logical K x n; tw: stored n x K), a cluster of CTAs
+// for COLS columns, a CTA an equal part of K.  Bound by the latency of its loads,
+// eight in flight a thread, and over a long K stored K x n by the sectors that the
+// columns share (two columns a CTA read them half as often).  1024 x 16 with W
+// stored K x n takes 434 us at K = 131072 and 932 at 262144; with one CTA a column
+// whatever K it took 481 and 1033.
+template <int COLS>
+__global__ void __launch_bounds__(512 * COLS) wexp_kernel(const double *__restrict__ W, int64_t ldw, int tw, int n,
+                                                          int64_t K, int *__restrict__ fcol) {
+    constexpr int WARPS = 16 * COLS;
+    __shared__ unsigned long long red[COLS][WARPS];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int parts = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int c = threadIdx.x % COLS;
+    const int64_t col = blockIdx.x / (unsigned)parts * COLS + c;
+    const unsigned long long *w = reinterpret_cast<const unsigned long long *>(W) + (tw ? col * ldw : col);
+    const int64_t step = tw ? 1 : ldw, per = (K + parts - 1) / parts;
+    const int64_t k1 = col >= n ? 0 : (rank + 1) * per < K ? (rank + 1) * per : K;
     unsigned long long m = 0;
-#pragma unroll 8
-    for (int64_t k = threadIdx.x; k < K; k += 512) {
-        const unsigned long long v = __ldg(w + k * step) & 0x7FFFFFFFFFFFFFFFull;
+    int64_t k = rank * per + threadIdx.x / COLS;
+    w += k * step;
+    for (; k + 7 * 512 < k1; k += 8 * 512, w += 8 * 512 * step) {
+        unsigned long long v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __ldg(w + i * 512 * step) & 0x7FFFFFFFFFFFFFFFull;
+#pragma unroll
+        for (int i = 0; i < 8; i++) m = v[i] > m ? v[i] : m;
+    }
+    for (; k < k1; k += 512, w += 512 * step) {
+        const unsigned long long v = __ldg(w) & 0x7FFFFFFFFFFFFFFFull;
         m = v > m ? v : m;
     }
 #pragma unroll
-    for (int s = 16; s; s >>= 1) {
+    for (int s = 16; s >= COLS; s >>= 1) {
         const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, s);
         m = v > m ? v : m;
     }
-    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = m;
+    if (threadIdx.x % 32 < COLS) red[c][threadIdx.x / 32] = m;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < COLS) {
 #pragma unroll
-        for (int i = 1; i < 16; i++) m = red[i] > m ? red[i] : m;
-        fcol[blockIdx.x] = exp_of_maxbits(m);
+        for (int i = 1; i < WARPS; i++) m = red[c][i] > m ? red[c][i] : m;
+        red[c][0] = m;
     }
+    if (parts > 1) cluster.sync();
+    if (rank == 0 && threadIdx.x < COLS && col < n) {
+        for (int i = 1; i < parts; i++) {
+            const unsigned long long v = *cluster.map_shared_rank(&red[c][0], i);
+            m = v > m ? v : m;
+        }
+        fcol[col] = exp_of_maxbits(m);
+    }
+    if (parts > 1) cluster.sync();   // the first CTA may still read this one's maxima
 }
 
 // Split-K: sum the parts (already scaled) in order, then the epilogue; a
@@ -832,8 +864,24 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
     if (!err) return set_status(GB_ERR_OOM, "skinny: no device error word");
 
     if (splits > 1) GB_CUDA_TRY(cudaMemsetAsync(nfrow, 0, (size_t)rows * 4, st));
-    wexp_kernel<<<n, 512, 0, st>>>(W, ldw, tw, K, fcol);
-    GB_LAUNCH_CHECK("wexp_kernel");
+    {
+        // a CTA per column for every WEXP_K values of it, up to a portable cluster
+        int parts = 1;
+        while (parts < 8 && K > parts * WEXP_K) parts *= 2;
+        const int cols = tw || parts < 8 ? 1 : 2;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)parts;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t wc = {};
+        wc.gridDim = dim3((unsigned)(ceil_div(n, cols) * parts));
+        wc.blockDim = dim3(512 * cols);
+        wc.stream = st;
+        wc.attrs = &at;
+        wc.numAttrs = parts > 1 ? 1 : 0;
+        GB_CUDA_TRY(cudaLaunchKernelEx(&wc, cols == 2 ? wexp_kernel<2> : wexp_kernel<1>, W, ldw, tw, n, K, fcol));
+        GB_LAUNCH_CHECK("wexp_kernel");
+    }
     // each further kernel is a programmatic dependent of the one before (captured ones keep plain
     // stream order)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
