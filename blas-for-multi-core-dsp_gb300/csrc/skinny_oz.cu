@@ -718,17 +718,20 @@ __global__ void __launch_bounds__(NT, 1)
 // columns share (two columns a CTA read them half as often).  1024 x 16 with W
 // stored K x n takes 434 us at K = 131072 and 932 at 262144; with one CTA a column
 // whatever K it took 481 and 1033.
-template <int COLS>
+template <int COLS, bool SHARED>
 __global__ void __launch_bounds__(512 * COLS) wexp_kernel(const double *__restrict__ W, int64_t ldw, int tw, int n,
                                                           int64_t K, int *__restrict__ fcol) {
     constexpr int WARPS = 16 * COLS;
     __shared__ unsigned long long red[COLS][WARPS];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int parts = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    int parts = 1, rank = 0;
+    if (SHARED) {
+        parts = (int)cg::this_cluster().num_blocks();
+        rank = (int)cg::this_cluster().block_rank();
+    }
     const int c = threadIdx.x % COLS;
-    const int64_t col = blockIdx.x / (unsigned)parts * COLS + c;
+    const int64_t col = (int64_t)(blockIdx.x / (unsigned)parts) * COLS + c;
     const unsigned long long *w = reinterpret_cast<const unsigned long long *>(W) + (tw ? col * ldw : col);
-    const int64_t step = tw ? 1 : ldw, per = (K + parts - 1) / parts;
+    const int64_t step = tw ? 1 : ldw, per = SHARED ? (K + parts - 1) / parts : K;
     const int64_t k1 = col >= n ? 0 : (rank + 1) * per < K ? (rank + 1) * per : K;
     unsigned long long m = 0;
     int64_t k = rank * per + threadIdx.x / COLS;
@@ -756,15 +759,15 @@ __global__ void __launch_bounds__(512 * COLS) wexp_kernel(const double *__restri
         for (int i = 1; i < WARPS; i++) m = red[c][i] > m ? red[c][i] : m;
         red[c][0] = m;
     }
-    if (parts > 1) cluster.sync();
+    if (SHARED) cg::this_cluster().sync();
     if (rank == 0 && threadIdx.x < COLS && col < n) {
         for (int i = 1; i < parts; i++) {
-            const unsigned long long v = *cluster.map_shared_rank(&red[c][0], i);
+            const unsigned long long v = *cg::this_cluster().map_shared_rank(&red[c][0], i);
             m = v > m ? v : m;
         }
         fcol[col] = exp_of_maxbits(m);
     }
-    if (parts > 1) cluster.sync();   // the first CTA may still read this one's maxima
+    if (SHARED) cg::this_cluster().sync();   // the first CTA may still read this one's maxima
 }
 
 // Split-K: sum the parts (already scaled) in order, then the epilogue; a
@@ -879,7 +882,7 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
         wc.stream = st;
         wc.attrs = &at;
         wc.numAttrs = parts > 1 ? 1 : 0;
-        GB_CUDA_TRY(cudaLaunchKernelEx(&wc, cols == 2 ? wexp_kernel<2> : wexp_kernel<1>, W, ldw, tw, n, K, fcol));
+        GB_CUDA_TRY(cudaLaunchKernelEx(&wc, parts == 1 ? wexp_kernel<1, false> : cols == 1 ? wexp_kernel<1, true> : wexp_kernel<2, true>, W, ldw, tw, n, K, fcol));
         GB_LAUNCH_CHECK("wexp_kernel");
     }
     // each further kernel is a programmatic dependent of the one before (captured ones keep plain
