@@ -27,6 +27,7 @@
 
 #include "gb_common.cuh"
 #include "sm100_ptx.cuh"
+#include "split_plan.h"
 
 namespace gb {
 
@@ -613,25 +614,6 @@ bool tc_eligible(const SkParams &p) {
     return p.rows < (int64_t(1) << 31) && p.K < (int64_t(1) << 30) && (uintptr_t)p.X % 16 == 0;
 }
 
-// K ranges per tile: units for four waves and more (one range when there are as
-// many tiles), up to twice as many where that leaves the last wave fuller; at
-// least `least` of the nst steps of K a range.
-inline int balanced_splits(int64_t tiles, int64_t nst, int64_t least) {
-    const double sms = sm_count();
-    int best = 1;
-    double best_fill = 0.0;
-    for (int s = 1; s <= 64 && (s == 1 || nst / s >= least); s++) {
-        const double units = (double)(tiles * s), fill = units / (ceil(units / sms) * sms);
-        if (units >= 8.0 * sms && s > 1 && best_fill > 0.0) break;
-        if (units < 4.0 * sms || fill > best_fill + 0.02) {
-            best = s;
-            best_fill = units < 4.0 * sms ? 0.0 : fill;
-        }
-        if (tiles >= 4 * (int64_t)sms) break;
-    }
-    return best;
-}
-
 template <typename T, int NB>
 gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
     pl.w_bytes = 0;
@@ -648,8 +630,7 @@ gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
         const int64_t nst = thin_tc_stages(p.K, classes);
         const int64_t sms = sm_count();
         // sums of at most the K range that a split into four waves of units would leave
-        int64_t ranges = 1;
-        while (pl.rtiles * ranges < 4 * sms && nst / (ranges * 2) >= 8 && ranges < 64) ranges *= 2;
+        const int64_t ranges = doubled_splits(pl.rtiles, nst, 8, (int)sms);
         pl.fold = (int)ceil_div(nst, ranges);
         // equal parts cut the ranges anywhere, so not the long ones (20011 x 6007, n 33: 107 against
         // 125 us; but 33440 x 32109, n 34: 810 against 758)
@@ -658,7 +639,7 @@ gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
         // an accumulator's error grows with its range, about 6.4e-9 of the result a k: another split may
         // change the ranges' mean length (weighted by themselves) by 1536 k, 1e-5, for a fuller last
         // wave, no more
-        int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst, 8);
+        int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst, 8, (int)sms);
         if (p.want_splits <= 0 && !equal) {
             const double len = (double)ceil_div(nst, want), whole = floor(len / pl.fold), rem = len - whole * pl.fold;
             const double mean = (whole * pl.fold * pl.fold + rem * rem) / len;
@@ -920,7 +901,7 @@ gb_status dispatch(const GemmArgs &g, size_t *need = nullptr) {
     if (sizeof(T) == 8 && thin_oz_eligible(p.tx, p.ldx, p.X, p.rows, p.K)) {
         // FP64: digits on the tensor cores; units of 128 rows x K chunks of 512
         const int64_t rtiles = ceil_div(p.rows, 128), nchunks = ceil_div(p.K, 512);
-        int splits = g.split_k > 0 ? g.split_k : balanced_splits(rtiles, nchunks, 2);
+        int splits = g.split_k > 0 ? g.split_k : oz_splits(rtiles, nchunks, p.tx, sm_count());
         const int64_t cpc = ceil_div(nchunks, splits);
         splits = (int)ceil_div(nchunks, cpc);
         if (need) {
