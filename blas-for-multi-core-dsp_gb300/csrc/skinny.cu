@@ -633,9 +633,11 @@ gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
         const int64_t ranges = doubled_splits(pl.rtiles, nst, 8, (int)sms);
         pl.fold = (int)ceil_div(nst, ranges);
         // equal parts cut the ranges anywhere, so not the long ones (20011 x 6007, n 33: 107 against
-        // 125 us; but 33440 x 32109, n 34: 810 against 758)
-        const bool equal = p.want_splits <= 0 && !p.tx && pl.rtiles < 4 * sms && pl.rtiles * nst >= 24 * sms &&
-                           64 * pl.fold <= 6144;
+        // 125 us; but 33440 x 32109, n 34: 810 against 758); nor tiles that are one range, whose
+        // stages the join outlasts (54752 x 668, n 64: 49 against 35 us in whole tiles; at 9 to 15
+        // stages 5 to 29 per cent)
+        const bool equal = p.want_splits <= 0 && !p.tx && ranges > 1 && pl.rtiles < 4 * sms &&
+                           pl.rtiles * nst >= 24 * sms && 64 * pl.fold <= 6144;
         // an accumulator's error grows with its range, about 6.4e-9 of the result a k: another split may
         // change the ranges' mean length (weighted by themselves) by 1536 k, 1e-5, for a fuller last
         // wave, no more

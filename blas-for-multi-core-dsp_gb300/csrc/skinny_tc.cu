@@ -156,22 +156,23 @@ struct Work {
     }
 };
 
-// C(row, j) from its sum
-__device__ __forceinline__ void store_output(const TcParams &p, float *cp, float sum) {
-    float v = p.alpha * sum;
-    if (p.semantics == GB_SEM_BLAS) {
-        if (p.beta != 0.f) v = fmaf(p.beta, *cp, v);
-    } else if (p.semantics == GB_SEM_SCALAR_BETA) {
-        v = v + p.beta;
-    } else {
-        v = *cp + (v + p.beta);
-    }
-    *cp = v;
+// C(row, j) from its sum, reading its old value c where the semantics ask for it
+__device__ __forceinline__ float output(const TcParams &p, const float *c, float sum) {
+    const float v = p.alpha * sum;
+    if (p.semantics == GB_SEM_BLAS) return p.beta != 0.f ? fmaf(p.beta, *c, v) : v;
+    if (p.semantics == GB_SEM_SCALAR_BETA) return v + p.beta;
+    return *c + (v + p.beta);
 }
+__device__ __forceinline__ void store_output(const TcParams &p, float *cp, float sum) { *cp = output(p, cp, sum); }
 
 // XL: 0 row-major X (rows in classes when ldx % 4 != 0), 1 K-major X with
-// ldx % 4 == 0, 2 K-major X in k-line classes.  EQ: equal parts.
-template <int NB, int XL, bool EQ>
+// ldx % 4 == 0, 2 K-major X in k-line classes.  EQ: equal parts.  CG: C is read,
+// sixteen columns' loads in flight at a time: where a tile's store is not hidden by
+// the next tiles' stages (equal parts: 49177 x 1133, n 61, beta 1: 105 us one after
+// the other, 77 so) or every column is another line of C; else one after the other,
+// which spreads them between the loads of X (rows of C, 211268 x 1214, n 48: 195 us
+// against 205).  An instance of its own, since the code alone costs a short call 0.6 us.
+template <int NB, int XL, bool EQ, bool CG>
 __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ Maps maps, TcParams p) {
     constexpr bool XCOLS = XL != 0;
     using C = Cfg<NB>;
@@ -390,6 +391,18 @@ __global__ void __launch_bounds__(NT, 1) thin_tc_kernel(const __grid_constant__ 
                 continue;
             }
             float *cr = p.C + row * p.cs_r;
+            if (CG) {
+#pragma unroll
+                for (int j0 = 0; j0 < NB; j0 += 16) {
+                    float c[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) c[j] = j0 + j < p.n ? cr[(int64_t)(j0 + j) * p.cs_c] : 0.f;
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (j0 + j < p.n) cr[(int64_t)(j0 + j) * p.cs_c] = output(p, c + j, acc[j0 + j]);
+                }
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < NB; j++) {
                 if (j >= p.n) break;
@@ -464,11 +477,11 @@ __global__ void __launch_bounds__(128) wsplit_kernel(const float *__restrict__ W
     *reinterpret_cast<uint4 *>(hi + per) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-template <int NB, int XL, bool EQ>
-gb_status launch_nb(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, int grid, bool dependent) {
+template <int NB, int XL, bool EQ, bool CG>
+gb_status launch_cg(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, int grid, bool dependent) {
     static std::atomic<uint64_t> attr{0};
     if (device_setup_needed(attr)) {
-        GB_CUDA_TRY(cudaFuncSetAttribute(thin_tc_kernel<NB, XL, EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        GB_CUDA_TRY(cudaFuncSetAttribute(thin_tc_kernel<NB, XL, EQ, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg<NB>::SMEM));
         device_setup_done(attr);
     }
@@ -482,7 +495,7 @@ gb_status launch_nb(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, i
     cfg.stream = a.stream;
     cfg.attrs = &pdl;
     cfg.numAttrs = dependent ? 1 : 0;
-    GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, thin_tc_kernel<NB, XL, EQ>, maps, tp));
+    GB_CUDA_TRY(cudaLaunchKernelEx(&cfg, thin_tc_kernel<NB, XL, EQ, CG>, maps, tp));
     GB_LAUNCH_CHECK("thin_tc_kernel");
     if (EQ && grid > 1) {
         cfg.gridDim = dim3((unsigned)(grid - 1), BM / 32);
@@ -492,6 +505,14 @@ gb_status launch_nb(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, i
         GB_LAUNCH_CHECK("thin_tc_join_kernel");
     }
     return ok();
+}
+
+template <int NB, int XL, bool EQ>
+gb_status launch_nb(const ThinTcArgs &a, const Maps &maps, const TcParams &tp, int grid, bool dependent) {
+    // (a split's sums go to `part`, and the kernel reads no C)
+    const bool reads_c = a.semantics == GB_SEM_ACCUM_SCALAR_BETA || (a.semantics == GB_SEM_BLAS && a.beta != 0.f);
+    return reads_c && a.splits == 1 && (EQ || a.cs_c != 1) ? launch_cg<NB, XL, EQ, true>(a, maps, tp, grid, dependent)
+                                          : launch_cg<NB, XL, EQ, false>(a, maps, tp, grid, dependent);
 }
 
 }  // namespace thin_tc
