@@ -242,10 +242,11 @@ __device__ __forceinline__ void chain(const T *__restrict__ A, const T *__restri
     }
 }
 
-// (FP32: two CTAs of 64 x 64 an SM, 128 registers a thread: 4.5 TFLOP/s at 2048 x 2048 x 1024, 3.8
-// with one)
+// 512 threads an SM at least.  FP32, two CTAs of 64 x 64 and 128 registers a thread: 4.5 TFLOP/s
+// at 2048 x 2048 x 1024, 3.8 with one.  FP64 in slabs would take 136 registers and one CTA:
+// 297 x 1876 x 3122 in slabs of 512 3577 us, 3369 with two.  (FP32 in slabs needs its 222.)
 template <typename T, int TM, int TN, int RM, int RN, bool SLABS>
-__global__ void __launch_bounds__(TM / RM * (TN / RN), sizeof(T) == 4 && !SLABS ? 512 * RM * RN / (TM * TN) : 1)
+__global__ void __launch_bounds__(TM / RM * (TN / RN), sizeof(T) == 8 || !SLABS ? 512 * RM * RN / (TM * TN) : 1)
     gemm_ordered_kernel(const T *__restrict__ A, const T *__restrict__ B, T *__restrict__ C, OrdParams p, T alpha,
                         T beta, unsigned tiles_n) {
     __shared__ __align__(16) Stage<T, TM, TN> s;
