@@ -16,6 +16,15 @@ gb_status set_status(gb_status st, const char *fmt, ...);
 gb_status ok();
 gb_status cuda_status(cudaError_t e, const char *where);
 
+// The calling thread's status as it was, for a call that fails at one way of doing its work
+// and then succeeds at another.
+struct StatusKeeper {
+    int st;
+    char msg[512];
+    StatusKeeper();
+    void restore() const;
+};
+
 #define GB_CHECK_ARG(cond, ...)                                                \
     do {                                                                       \
         if (!(cond)) return ::gb::set_status(GB_ERR_INVALID_ARG, __VA_ARGS__); \

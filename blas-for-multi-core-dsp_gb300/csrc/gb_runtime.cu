@@ -19,7 +19,7 @@
 namespace gb {
 
 static thread_local int t_status = GB_OK;
-static thread_local char t_msg[512] = "";
+static thread_local char t_msg[sizeof(StatusKeeper::msg)] = "";
 
 gb_status set_status(gb_status st, const char *fmt, ...) {
     t_status = st;
@@ -31,6 +31,12 @@ gb_status set_status(gb_status st, const char *fmt, ...) {
 }
 
 gb_status ok() { return GB_OK; }
+
+StatusKeeper::StatusKeeper() : st(t_status) { memcpy(msg, t_msg, sizeof(msg)); }
+void StatusKeeper::restore() const {
+    t_status = st;
+    memcpy(t_msg, msg, sizeof(msg));
+}
 
 static std::atomic<unsigned long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }

@@ -976,8 +976,10 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
     const size_t sums = (size_t)tiles_total * (s + parts - 1) * (BM * BN * 4);
     size_t sbytes = wide ? (size_t)grid * wide::SCRATCH_DOUBLES * sizeof(double) : parts > 1 ? sums : 0;
     const size_t mbytes = (size_t)(mp + np) * sizeof(unsigned long long);
+    const StatusKeeper before;
     uint8_t *ws = (uint8_t *)workspace(vbytes + wbytes + ebytes + sbytes + mbytes + 4096, g.stream);
     if (!ws && parts > 1) {   // no room for the parts' sums
+        before.restore();
         parts = 1;
         sbytes = 0;
         grid = (int)std::min<int64_t>(tiles_total, sm_count());
