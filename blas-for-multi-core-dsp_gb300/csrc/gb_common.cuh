@@ -231,6 +231,7 @@ gb_status launch_thin_tc(const ThinTcArgs &a);
 
 // FP64 skinny product from integer digits on the tensor cores (skinny_oz.cu).
 bool thin_oz_eligible(int tx, int64_t ldx, const void *X, int64_t rows, int64_t K);
+bool thin_oz_pieces(int64_t ldx, const void *X);   // X copied in 8-byte pieces, not by TMA
 size_t thin_oz_workspace_bytes(int64_t rows, int64_t K, int n, int splits);
 gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, int tx, const double *W, int64_t ldw,
                          int tw, int n, double *C, int64_t cs_r, int64_t cs_c, double alpha, double beta,

@@ -903,7 +903,8 @@ gb_status dispatch(const GemmArgs &g, size_t *need = nullptr) {
     if (sizeof(T) == 8 && thin_oz_eligible(p.tx, p.ldx, p.X, p.rows, p.K)) {
         // FP64: digits on the tensor cores; units of 128 rows x K chunks of 512
         const int64_t rtiles = ceil_div(p.rows, 128), nchunks = ceil_div(p.K, 512);
-        int splits = g.split_k > 0 ? g.split_k : oz_splits(rtiles, nchunks, p.tx, sm_count());
+        const bool by_range = oz_by_range(p.tx, thin_oz_pieces(p.ldx, p.X), rtiles, sm_count());
+        int splits = g.split_k > 0 ? g.split_k : oz_splits(rtiles, nchunks, by_range, sm_count());
         const int64_t cpc = ceil_div(nchunks, splits);
         splits = (int)ceil_div(nchunks, cpc);
         if (need) {

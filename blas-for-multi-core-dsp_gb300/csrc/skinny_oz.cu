@@ -56,6 +56,7 @@
 
 #include "gb_common.cuh"
 #include "sm100_ptx.cuh"
+#include "split_plan.h"
 
 namespace cg = cooperative_groups;
 
@@ -109,13 +110,13 @@ struct OzThinParams {
     const double *X, *W;
     int64_t ldx, ldw;
     int tx, tw, j0;
+    int by_range;   // order of the units
 };
 
-// Unit u = (row tile, split).  Row-major X: the splits of a tile one after the
-// other; K-major X: the tiles of a split, so that the CTAs at work read
-// neighbouring pieces of the same k lines.
-__device__ __forceinline__ int split_of(const OzThinParams &p, int u) { return p.tx ? u / p.rtiles : u % p.splits; }
-__device__ __forceinline__ int tile_of(const OzThinParams &p, int u) { return p.tx ? u % p.rtiles : u / p.splits; }
+// Unit u = (row tile, split): the splits of a tile one after the other, or the tiles of
+// a split (oz_by_range).
+__device__ __forceinline__ int split_of(const OzThinParams &p, int u) { return p.by_range ? u / p.rtiles : u % p.splits; }
+__device__ __forceinline__ int tile_of(const OzThinParams &p, int u) { return p.by_range ? u % p.rtiles : u / p.splits; }
 
 // The (unit, chunk) pairs of this CTA in order:
 // chunks of CHUNK_KB k blocks from the split's first.
@@ -851,6 +852,11 @@ bool thin_oz_eligible(int tx, int64_t ldx, const void *X, int64_t rows, int64_t 
     return K >= 64 && rows < (int64_t(1) << 31) && K < (int64_t(1) << 30) && (uintptr_t)X % 8 == 0;
 }
 
+bool thin_oz_pieces(int64_t ldx, const void *X) {
+    const char *force = getenv("GB_SKINNY_OZ_CPASYNC");   // "1": the cp.async loader for any X (tests)
+    return ldx % 2 != 0 || (uintptr_t)X % 16 != 0 || (force && force[0] == '1');
+}
+
 gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, int tx, const double *W, int64_t ldw,
                          int tw, int n, double *C, int64_t cs_r, int64_t cs_c, double alpha, double beta,
                          int semantics, int splits, int64_t kchunk, void *ws, cudaStream_t st) {
@@ -898,8 +904,7 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
     cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
 
     // X through TMA when its rows (or k lines) start on 16-byte boundaries, else by cp.async
-    const char *force = getenv("GB_SKINNY_OZ_CPASYNC");   // "1": the cp.async loader for any X (tests)
-    const bool cpa = ldx % 2 != 0 || (uintptr_t)X % 16 != 0 || (force && force[0] == '1');
+    const bool cpa = thin_oz_pieces(ldx, X);
     CUtensorMap tx_map, tw_map[2];   // W digit boxes of one or two column groups
     const bool okw =
         make_tmap_bf16(&tw_map[0], wd, (uint64_t)kp, (uint64_t)2 * S * NB, (uint64_t)kp * 2, KB, S * NB, 64) &&
@@ -937,7 +942,7 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
         GB_LAUNCH_CHECK("wdigits_kernel");
         OzThinParams p{rows, K, nc, splits, (int)(kchunk / KB), rtiles, pw,
                        C + j0 * cs_c, cs_r, cs_c, alpha, beta, semantics, part, nfrow, fcol + j0, err,
-                       X, W, ldx, ldw, tx, tw, j0};
+                       X, W, ldx, ldw, tx, tw, j0, oz_by_range(tx, cpa, rtiles, sm_count()) ? 1 : 0};
         const CUtensorMap &twm = tw_map[ng - 1];
         auto kernel = ng == 1 ? (tx ? (cpa ? thin_oz_kernel<true, true, 1> : thin_oz_kernel<true, false, 1>)
                                     : (cpa ? thin_oz_kernel<false, true, 1> : thin_oz_kernel<false, false, 1>))

@@ -6,6 +6,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <numeric>
+
 namespace gb {
 
 // K ranges per tile: units for four waves and more (one range when there are as
@@ -36,12 +38,12 @@ inline int doubled_splits(int64_t tiles, int64_t nst, int64_t least, int sm_coun
 
 // Steps of K that the CTA with the most work walks when each tile has (up to) `splits`
 // ranges, all but the last range of a tile of the same length.  CTA b takes units b,
-// b + SMs, ...  kmajor: units in the order of their ranges, the short ones last; else
+// b + SMs, ...  by_range: units in the order of their ranges, the short ones last; else
 // the ranges of a tile in a row.
-inline int64_t walked_steps(int64_t tiles, int64_t nst, int splits, bool kmajor, int sm_count) {
+inline int64_t walked_steps(int64_t tiles, int64_t nst, int splits, bool by_range, int sm_count) {
     const int64_t per = (nst + splits - 1) / splits, ranges = (nst + per - 1) / per, units = tiles * ranges;
     const int64_t less = per - (nst - (ranges - 1) * per), most = (units + sm_count - 1) / sm_count;
-    if (kmajor) {   // of the CTAs with the most units the first has the fewest short ones
+    if (by_range) {   // of the CTAs with the most units the first has the fewest short ones
         const int64_t whole = (units - tiles + sm_count - 1) / sm_count;
         return most * per - (most - whole) * less;
     }
@@ -58,17 +60,28 @@ inline int64_t walked_steps(int64_t tiles, int64_t nst, int splits, bool kmajor,
     return worst;
 }
 
+// Whether FP64 units are taken in the order of their K ranges (K-major X: CTAs at work
+// read neighbouring pieces of the same k lines) or the ranges of a tile in a row.  X
+// that is copied in 8-byte pieces (odd leading dimensions) loses by the former where a
+// CTA meets only few row tiles, i.e. the tile and SM counts share a large factor: us,
+// by ranges / in a row, 2358 x 215593, n 10 (19 tiles) 2241 / 1887; 4850 x 98864, n 3
+// (38) 2105 / 1701; 1976 x 204156, n 5 (16) 1525 / 1445; factors up to 4 gain 4 per cent by
+// ranges.  X read by TMA gains 2 to 7 per cent throughout.
+inline bool oz_by_range(bool kmajor, bool pieces, int64_t tiles, int sm_count) {
+    return kmajor && !(pieces && std::gcd(tiles, (int64_t)sm_count) >= 8);
+}
+
 // FP64 (steps of 512 k).  With few tiles more ranges can spill units into another
 // wave, and every SM then waits for those: the doubled count where its longest walk is
 // shorter by more than a twentieth.  Row-major X, us, balanced / doubled: 3919 x 4701,
 // n 43, 355 / 282 (155 units of 2 steps on 152 SMs against 124 of 3); 4419 x 7256, n 15,
 // 169 / 125; 1088 x 19414, n 42, 280 / 222; but 6482 x 3073, n 54, 244 / 281 (walks of 4).
-inline int oz_splits(int64_t tiles, int64_t nchunks, bool kmajor, int sm_count) {
+inline int oz_splits(int64_t tiles, int64_t nchunks, bool by_range, int sm_count) {
     const int balanced = balanced_splits(tiles, nchunks, 2, sm_count);
     const int doubled = doubled_splits(tiles, nchunks, 2, sm_count);
     if (balanced == doubled) return balanced;
-    const int64_t walk = walked_steps(tiles, nchunks, balanced, kmajor, sm_count);
-    return 1.05 * (double)walked_steps(tiles, nchunks, doubled, kmajor, sm_count) < (double)walk ? doubled : balanced;
+    const int64_t walk = walked_steps(tiles, nchunks, balanced, by_range, sm_count);
+    return 1.05 * (double)walked_steps(tiles, nchunks, doubled, by_range, sm_count) < (double)walk ? doubled : balanced;
 }
 
 }  // namespace gb

@@ -24,3 +24,18 @@ def test_column_maximum_in_any_part(K, tw):
     gbblas.dgemm("N", tw, M, n, K, 1.0, X, K, stored, stored.shape[1], 0.0, C, n, algo=gbblas.ALGO_SKINNY)
     gbblas.sync()
     assert torch.equal(C, X @ W)
+
+
+@pytest.mark.parametrize("rows", [2358, 1976, 4850, 2300])    # 19, 16 and 38 row tiles: ranges in a row; 18: by ranges
+@pytest.mark.parametrize("split", [0, 1, 5])
+def test_order_of_units_in_pieces(rows, split):
+    """K-major X of an odd leading dimension, in either order of its units."""
+    K, n, ld = 2700, 7, rows + (rows + 1) % 2
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    X = torch.randint(-9, 10, (K, ld), generator=g, device="cuda").double()
+    W = torch.randint(-9, 10, (K, n), generator=g, device="cuda").double()
+    C = torch.randint(-9, 10, (rows, n), generator=g, device="cuda").double()
+    want = X[:, :rows].t() @ W - 2.0 * C
+    gbblas.dgemm("T", "N", rows, n, K, 1.0, X, ld, W, n, -2.0, C, n, algo=gbblas.ALGO_SKINNY, split_k=split)
+    gbblas.sync()
+    assert torch.equal(C, want)

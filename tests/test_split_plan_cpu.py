@@ -18,11 +18,11 @@ PROGRAM = r"""
 #include <vector>
 #include "split_plan.h"
 
-static int64_t walk(int64_t tiles, int64_t nst, int splits, bool kmajor, int sms) {
+static int64_t walk(int64_t tiles, int64_t nst, int splits, bool by_range, int sms) {
     const int64_t per = (nst + splits - 1) / splits, r = (nst + per - 1) / per;
     std::vector<int64_t> sum(sms, 0);
     for (int64_t u = 0; u < tiles * r; u++) {
-        const int64_t sp = kmajor ? u / tiles : u % r;
+        const int64_t sp = by_range ? u / tiles : u % r;
         sum[u % sms] += std::min(per, nst - sp * per);
     }
     return *std::max_element(sum.begin(), sum.end());
@@ -31,14 +31,14 @@ static int64_t walk(int64_t tiles, int64_t nst, int splits, bool kmajor, int sms
 int main(int, char **argv) {
     const int sms = atoi(argv[1]);
     long long worse = 0, other = 0, out_of_range = 0;
-    for (int kmajor = 0; kmajor < 2; kmajor++)
+    for (int by_range = 0; by_range < 2; by_range++)
         for (int64_t tiles = 1; tiles <= 9 * sms; tiles += tiles < 2 * sms ? 1 : 7)
             for (int64_t steps = 1; steps <= 600; steps += steps < 60 ? 1 : 37) {
-                const int s = gb::oz_splits(tiles, steps, kmajor, sms), d = gb::doubled_splits(tiles, steps, 2, sms);
-                const int64_t chosen = walk(tiles, steps, s, kmajor, sms);
+                const int s = gb::oz_splits(tiles, steps, by_range, sms), d = gb::doubled_splits(tiles, steps, 2, sms);
+                const int64_t chosen = walk(tiles, steps, s, by_range, sms);
                 out_of_range += s < 1 || s > 64 || s > steps;
-                other += gb::walked_steps(tiles, steps, s, kmajor, sms) != chosen;
-                worse += chosen > 1.05 * gb::walked_steps(tiles, steps, d, kmajor, sms);
+                other += gb::walked_steps(tiles, steps, s, by_range, sms) != chosen;
+                worse += chosen > 1.05 * gb::walked_steps(tiles, steps, d, by_range, sms);
             }
     printf("%lld %lld %lld\n", worse, other, out_of_range);
 }
