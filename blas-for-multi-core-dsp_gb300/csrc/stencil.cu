@@ -38,72 +38,49 @@ __device__ __forceinline__ T update(T top, T left, T right, T down, T mid, int64
     return O::mul(O::add(right, O::add(O::add(left, down), O::add(top, mid))), O::fifth());
 }
 
-constexpr int NT = 256;   // 32 columns x 8 row bands
+constexpr int NT = 256;            // 32 columns x 8 row bands
+constexpr int TH = 32, TW = 64;    // output tile
 
-// One CTA: a TH x TW output tile, loaded with a halo of `tsweeps` cells,
-// `tsweeps` sweeps in shared memory, the final tile written back.  In each
-// sweep warp w walks row band w of the still-valid region and lane l the
-// columns l, l+32, ...; a thread keeps (top, middle, down) of its column in
-// registers while it moves down the band, so a point costs three shared
-// loads (down, left, right) and one store.  Cells on the grid boundary keep
-// their value; cells outside the grid are computed but never read by an
-// interior cell and never written back.
+// FP64 form: one CTA per TH x TW output tile, loaded with a halo of one cell
+// into shared memory.  Warp w walks row band w of the tile and lane l the
+// columns l and l+32; a thread keeps (top, middle, down) of its column in
+// registers while it moves down the band, so a point costs three shared loads
+// (down, left, right).  Bound by the FP64 pipe, where the halos of several
+// sweeps a pass would only be computed twice: one sweep per launch (the FP32
+// form's streaming measured slower, 1.38 against 1.64 TB/s at 8192 x 8192).
 template <typename T, int ORDER>
 __global__ void __launch_bounds__(NT) stencil_tb_kernel(const T *__restrict__ src, T *__restrict__ dst, int64_t M,
-                                                        int64_t N, int tsweeps, int TH, int TW) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int H = TH + 2 * tsweeps, W = TW + 2 * tsweeps;
-    T *cur = reinterpret_cast<T *>(smem_raw);
-    T *nxt = cur + H * W;
+                                                        int64_t N) {
+    constexpr int H = TH + 2, W = TW + 2, ROWS = TH / (NT / 32);
+    __shared__ T tile[H * W];
     const int64_t ld = N + 2;
-    const int64_t R0 = 1 + (int64_t)blockIdx.y * TH - tsweeps;   // padded coords of local (0,0)
-    const int64_t C0 = 1 + (int64_t)blockIdx.x * TW - tsweeps;
+    const int64_t R0 = (int64_t)blockIdx.y * TH;   // padded coords of the halo's corner
+    const int64_t C0 = (int64_t)blockIdx.x * TW;
     const int lane = threadIdx.x % 32, band = threadIdx.x / 32;
 
     for (int lr = band; lr < H; lr += NT / 32) {
         const int64_t r = R0 + lr;
-        if (r < 0 || r > M + 1) continue;
+        if (r > M + 1) break;
         const T *srow = src + r * ld;
         for (int lc = lane; lc < W; lc += 32) {
             const int64_t c = C0 + lc;
-            if (c >= 0 && c <= N + 1) cur[lr * W + lc] = srow[c];
+            if (c <= N + 1) tile[lr * W + lc] = srow[c];
         }
     }
     __syncthreads();
 
-    for (int s = 1; s <= tsweeps; s++) {
-        const int h = H - 2 * s;
-        const int per = (h + NT / 32 - 1) / (NT / 32);
-        const int rbeg = s + band * per;
-        const int rend = min(rbeg + per, H - s);
-        for (int lc = s + lane; lc < W - s; lc += 32) {
-            if (rbeg >= rend) break;
-            const int64_t gc = C0 + lc;
-            const bool col_fixed = gc <= 0 || gc >= N + 1;
-            const T *cp = cur + rbeg * W + lc;
-            T *np = nxt + rbeg * W + lc;
-            T top = cp[-W], mid = cp[0];
-            int64_t gr = R0 + rbeg;
-            for (int lr = rbeg; lr < rend; lr++, cp += W, np += W, gr++) {
-                const T down = cp[W];
-                T v = update<T, ORDER>(top, cp[-1], cp[1], down, mid, gr - 1);
-                if (col_fixed || gr <= 0 || gr >= M + 1) v = mid;
-                *np = v;
-                top = mid;
-                mid = down;
-            }
-        }
-        __syncthreads();
-        T *tmp = cur; cur = nxt; nxt = tmp;
-    }
-
-    for (int lr = tsweeps + band; lr < tsweeps + TH; lr += NT / 32) {
-        const int64_t r = R0 + lr;
-        if (r < 1 || r > M) continue;
-        T *drow = dst + r * ld;
-        for (int lc = tsweeps + lane; lc < tsweeps + TW; lc += 32) {
-            const int64_t c = C0 + lc;
-            if (c >= 1 && c <= N) drow[c] = cur[lr * W + lc];
+    const int lr0 = 1 + band * ROWS;
+    for (int lc = 1 + lane; lc <= TW; lc += 32) {
+        const int64_t c = C0 + lc;
+        if (c > N) break;
+        const T *cp = tile + lr0 * W + lc;
+        T top = cp[-W], mid = cp[0];
+        T *out = dst + (R0 + lr0) * ld + c;
+        for (int64_t r = R0 + lr0; r < R0 + lr0 + ROWS && r <= M; r++, cp += W, out += ld) {
+            const T down = cp[W];
+            *out = update<T, ORDER>(top, cp[-1], cp[1], down, mid, r - 1);
+            top = mid;
+            mid = down;
         }
     }
 }
@@ -254,8 +231,10 @@ __device__ __forceinline__ void rs_walk(const float *__restrict__ src, float *__
 
 // One warp per CTA, 16 of them resident per SM (128 registers), so that a
 // grid that does not fill the GPU spreads evenly.  A pass after the first is
-// launched as a programmatic dependent: its launch overlaps the pass before,
-// whose rows it waits for here.
+// launched as a programmatic dependent.  No pass triggers its dependent early
+// (1000 x 1500, 60 sweeps: 145 us with a trigger, 125 without the attribute,
+// 105 with it and the wait alone), so it starts when the last CTA of the pass
+// before has exited, and what is saved is the gap of a plain launch.
 template <int T, int ORDER>
 __global__ void __launch_bounds__(32, T > RS_T ? 12 : RS_WARPS) stencil_rs_kernel(const float *__restrict__ src,
                                                                   float *__restrict__ dst, int64_t M, int64_t N,
@@ -265,7 +244,9 @@ __global__ void __launch_bounds__(32, T > RS_T ? 12 : RS_WARPS) stencil_rs_kerne
     const int64_t c0 = 1 + sx * (RS_W - 2 * T) - T;   // padded column of the strip's first
     const int64_t r0 = 1 + sy * seg;                   // padded rows written: [r0, r1)
     const int64_t r1 = r0 + seg < M + 1 ? r0 + seg : M + 1;
-    // no fixed cell in the window and every load inside the grid
+    // every load inside the grid, and no fixed cell among those that the rows and columns written
+    // come from: a boundary column may be the window's outermost, whose sweeps only reach the strip's
+    // halo, which is not written
     const bool inside = c0 >= 0 && c0 + RS_W <= N + 2 && r0 - T - 1 >= 0 && r1 + T <= M + 2;
     if (inside) rs_walk<T, ORDER, false>(src, dst, M, N, c0, r0, r1);
     else rs_walk<T, ORDER, true>(src, dst, M, N, c0, r0, r1);
@@ -448,9 +429,10 @@ gb_status stencil9(int64_t M, int64_t N, E *A, E *B, int iters, const E *w_host,
 // k = 1 / 2 / 3 / 4; 146 in waves of four that other waves follow; the 1.2
 // are the row's loads and stores), a pass about 6000 cycles besides (launch,
 // first rows).  Long segments waste few halo rows, short ones fill the GPU:
-// 1000 x 1500, 60 sweeps, measures 105 us in segments of 12 rows, 116 in 24,
-// 120 in 16; 8192 x 8192, 48 sweeps, 1115 us in segments of 84, 1136 in 112,
-// 1153 in 64 (segments of 256 whatever the grid: 2311 and 2620 us).
+// 1000 x 1500, 60 sweeps, measures 112 us in segments of 12 rows (105 against
+// 116 in 24 and 120 in 16, before the loads behind the wait were made coherent);
+// 8192 x 8192, 48 sweeps, 1115 us in segments of 84, 1136 in 112, 1153 in 64
+// (segments of 256 whatever the grid: 2311 and 2620 us).
 struct RsPlan {
     int launches, seg;
 };
@@ -526,20 +508,15 @@ gb_status stencil(int64_t M, int64_t N, T *A, T *B, int iters, int order, void *
         }
         return ok();
     }
-    // FP64 is bound by the FP64 pipe, where recomputing halos only costs: one
-    // sweep per launch from shared-memory tiles (the streaming form measured
-    // slower there, 1.38 against 1.64 TB/s)
-    constexpr int TH = 32, TW = 64;
     dim3 grid((unsigned)ceil_div(N, TW), (unsigned)ceil_div(M, TH));
     GB_CHECK_ARG(grid.y <= 65535u, "stencil2d: M too large");
-    const size_t smem = 2 * (size_t)(TH + 2) * (TW + 2) * sizeof(double);
     for (int l = 0; l < iters; l++) {
         const double *src = (const double *)(l % 2 == 0 ? A : B);
         double *dst = (double *)(l % 2 == 0 ? B : A);
         switch (order) {
-            case 0: stencil_tb_kernel<double, 0><<<grid, NT, smem, st>>>(src, dst, M, N, 1, TH, TW); break;
-            case 1: stencil_tb_kernel<double, 1><<<grid, NT, smem, st>>>(src, dst, M, N, 1, TH, TW); break;
-            default: stencil_tb_kernel<double, 2><<<grid, NT, smem, st>>>(src, dst, M, N, 1, TH, TW); break;
+            case 0: stencil_tb_kernel<double, 0><<<grid, NT, 0, st>>>(src, dst, M, N); break;
+            case 1: stencil_tb_kernel<double, 1><<<grid, NT, 0, st>>>(src, dst, M, N); break;
+            default: stencil_tb_kernel<double, 2><<<grid, NT, 0, st>>>(src, dst, M, N); break;
         }
         GB_LAUNCH_CHECK("stencil_tb_kernel");
     }
