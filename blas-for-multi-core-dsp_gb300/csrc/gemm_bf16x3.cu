@@ -24,12 +24,15 @@
 //     absorbed here (a row-major or a transposed read, always a K-major
 //     write), so the GEMM kernel has one operand layout.
 //  3. gemm: persistent, one CTA per SM over 128 x 256 C tiles (128 x 128 or
-//     128 x 64 where those would leave SMs idle), K in blocks of 32 (one
-//     64-byte swizzle atom), a 4- to 8-stage TMA -> shared memory pipeline
-//     with mbarriers; warp 0 issues TMA, warp 1 issues tcgen05.mma (M=128,
-//     N=256, K=16, three products per K step into a TMEM accumulator of 256
-//     columns, two accumulators alternating), the epilogue warps read the
-//     finished accumulator with tcgen05.ld and write C with alpha/beta.
+//     128 x 64 where those would leave SMs idle), or a cluster of two over
+//     256 x 256; K in blocks of 32 or 64 (one 64- or 128-byte swizzle atom),
+//     a two- to four-stage TMA -> shared memory pipeline with mbarriers;
+//     warp 0 issues TMA, warp 1 (of a pair's first CTA) issues tcgen05.mma
+//     (K=16, the piece products of a K step into one TMEM accumulator, two
+//     accumulators alternating), the epilogue warps read the finished
+//     accumulator with tcgen05.ld and write C with alpha/beta.
+//  4. join: where even narrow tiles leave SMs idle, several CTAs share a
+//     tile's k-blocks and this kernel adds their sums.
 // Skinny products (min(M, N) <= 64) run BF16X3 in one fused kernel instead
 // (TMA of the FP32 tiles, converter warps, MMA).
 #include <cuda.h>

@@ -646,9 +646,10 @@ __global__ void __launch_bounds__(256) ozaki_join_kernel(const __grid_constant__
 // What bounds it is operand bytes into the SM's shared memory, about 64 a clock:
 // a k-block of 128 x 256 brings 48 KB for 1024 clocks of MMA at most.  Two CTAs on
 // one tile (cta_group::2) hold half of W each, 32 KB a k-block for the same work,
-// and six stages fit.  4096^3, s = 8: 4106 us one CTA, 3596 two; 8192^3 26.7 and
-// 25.5 ms, there 1.60 PFLOP/s under the power limit.  One CTA stays where tiles of
-// 256 rows would waste a wave.  The two FP32 accumulators take all 512 TMEM
+// and six stages fit.  4096^3, s = 8: 4106 us one CTA, 3596 two.  8192^3 runs at the
+// power limit and gains little or nothing: 26.7 and 25.5 ms in a loop, 28.25 and
+// 28.04 timed side by side, entries of U[-1, 1] (u 2^e: 22.8).  One CTA stays where
+// tiles of 256 rows would waste a wave.  The two FP32 accumulators take all 512 TMEM
 // columns, so the FP64 running sum of each diagonal flush lives in a per-CTA
 // scratch array in global memory (256 KB per CTA, L2-resident, interleaved so that
 // a warp's access to one pair of a lane's values is 512 contiguous bytes).  Warps:
@@ -1019,8 +1020,9 @@ static gb_status ozaki_one(const GemmArgs &g, int s) {
         return set_status(GB_ERR_UNSUPPORTED, "ozaki: operands too large");
     maxbits64_kernel<<<(unsigned)mblocks, 256, 0, g.stream>>>(ma);
     GB_LAUNCH_CHECK("ozaki line maxima");
-    // the slices and the GEMM are launched as programmatic dependents of the kernel before: their
-    // launch and set-up overlap it (captured launches keep plain stream order)
+    // the slices and the GEMM are launched as programmatic dependents of the kernel before: it
+    // triggers nothing early, so they start when its last CTA has exited, without the gap of a plain
+    // launch (captured launches keep plain stream order)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     GB_CUDA_TRY(cudaStreamIsCapturing(g.stream, &cap));
     cudaLaunchAttribute attrs[2];

@@ -638,9 +638,10 @@ gb_status make_plan(SkParams &p, Plan &pl, bool allow_tc = true) {
         // stages 5 to 29 per cent)
         const bool equal = p.want_splits <= 0 && !p.tx && ranges > 1 && pl.rtiles < 4 * sms &&
                            pl.rtiles * nst >= 24 * sms && 64 * pl.fold <= 6144;
-        // an accumulator's error grows with its range, about 6.4e-9 of the result a k: another split may
-        // change the ranges' mean length (weighted by themselves) by 1536 k, 1e-5, for a fuller last
-        // wave, no more
+        // results move with the ranges' length, by about 6.4e-9 of the result a k of an accumulator's
+        // range (shorter ones are the more exact): another split than the one into `ranges` may change
+        // the mean length (weighted by itself) by 1536 k for a fuller last wave, no more, so that a
+        // result stays within 1e-5 of the one that split gives
         int64_t want = p.want_splits > 0 ? p.want_splits : equal ? 1 : balanced_splits(pl.rtiles, nst, 8, (int)sms);
         if (p.want_splits <= 0 && !equal) {
             const double len = (double)ceil_div(nst, want), whole = floor(len / pl.fold), rem = len - whole * pl.fold;

@@ -891,8 +891,9 @@ gb_status launch_thin_oz(int64_t rows, int64_t K, const double *X, int64_t ldx, 
         GB_CUDA_TRY(cudaLaunchKernelEx(&wc, parts == 1 ? wexp_kernel<1, false> : cols == 1 ? wexp_kernel<1, true> : wexp_kernel<2, true>, W, ldw, tw, n, K, fcol));
         GB_LAUNCH_CHECK("wexp_kernel");
     }
-    // each further kernel is a programmatic dependent of the one before (captured ones keep plain
-    // stream order)
+    // each further kernel is a programmatic dependent of the one before, which triggers nothing
+    // early: it starts when that one's last CTA has exited, without the gap of a plain launch
+    // (captured ones keep plain stream order)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     GB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
     cudaLaunchAttribute pdl;

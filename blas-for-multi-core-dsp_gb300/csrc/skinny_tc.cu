@@ -26,12 +26,15 @@
 // tile's K leaves the last wave part empty and writes every tile `splits`
 // times: 20011 x 6007, n = 33: 126 us against 108).  With four tiles an SM and
 // more the tail costs nothing (HBM bound; 262144 x 4096: 678 us against 682 in
-// equal parts), with fewer than sixteen stages an SM the join costs more than
-// it gives (2000 x 1500, n = 40: 20.6 against 21.8): fixed split.  K-major X keeps a fixed split, summed by skinny_reduce_kernel, and
-// takes the tiles of one K range before the next, so that the CTAs at work read
-// neighbouring pieces of the same k lines (11499 rows, K = 48841: 499 us in equal
-// parts, 404 with the ranges of a tile one after the other, 367 so).  So does
-// a requested split count (gb_gemm_opts.split_k).
+// equal parts), with fewer than 24 stages an SM the join costs more than
+// it gives (2000 x 1500, n = 40: 20.6 against 21.8), as it does for tiles of a
+// single K range, and ranges above 6144 k are not cut anywhere (make_plan in
+// skinny.cu has the rule and both sides' times): fixed split.  K-major X keeps a
+// fixed split, summed by skinny_reduce_kernel, and takes the tiles of one K range
+// before the next, so that the CTAs at work read neighbouring pieces of the same
+// k lines (11499 rows, K = 48841: 499 us in equal parts, 404 with the ranges of a
+// tile one after the other, 367 so).  A requested split count
+// (gb_gemm_opts.split_k) is a fixed split too.
 // Shared-memory traffic per X value is the TMA write and one read (8 bytes).
 //
 // Row-major X whose leading dimension is not a multiple of 4 floats cannot be

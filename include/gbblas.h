@@ -101,7 +101,12 @@ gb_status gb_fill_f32(float *X, int64_t rows, int64_t cols, int64_t ld, uint64_t
 typedef enum gb_algo {
     GB_ALGO_AUTO = 0,     /* pick per shape and dtype                          */
     GB_ALGO_ORDERED = 1,  /* the reference's summation order, bit-exact         */
-    GB_ALGO_SIMT = 2,     /* plain FP32 FFMA / FP64 DFMA register tiles         */
+    GB_ALGO_SIMT = 2,     /* plain FP32 FFMA / FP64 DFMA register tiles.  FP32
+                             products of at most 2^27 multiply-adds, or K < 64,
+                             sum K in several parts by a plan that reads the SM
+                             count (their last bits depend on the GPU and on a
+                             server's SM share); larger ones keep one sum per
+                             output in k order                              */
     GB_ALGO_DMMA = 3,     /* FP64 tensor pipe (mma.sync m8n8k4 f64)             */
     GB_ALGO_BF16X3 = 4,   /* SGEMM as hi*hi+hi*lo+lo*hi BF16 on tcgen05, FP32 acc */
     GB_ALGO_OZAKI = 5,    /* DGEMM from exact integer slices on tensor cores    */
